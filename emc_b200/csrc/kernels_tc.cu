@@ -20,6 +20,7 @@
 
 #include "fixed.cuh"
 #include "tc.cuh"
+#include "tc_ptx.cuh"
 #include "voxel.h"
 
 namespace emc {
@@ -27,109 +28,7 @@ namespace {
 
 constexpr int BM = 128, BN = 256;
 constexpr int kTmemCols = 512;
-constexpr uint64_t kWaitLimitNs = 10ull * 1000ull * 1000ull * 1000ull;
 
-// ------------------------------------------------------------ PTX helpers --
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ uint64_t globaltimer() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm, int c0, int c1,
-                                            uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"((uint64_t)tm), "r"(c0), "r"(c1), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
-                                        uint32_t accum) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accum)
-      : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-        "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_wait() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-// Named barrier of the epilogue warps (n threads).
-__device__ __forceinline__ void epi_bar(int n = 128) {
-  asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory");
-}
-
-// Shared-memory matrix descriptor of a K-major operand whose rows are BK FP16
-// elements (BK = 64: 128-byte rows, 128B swizzle; BK = 32: 64-byte rows, 64B
-// swizzle, as TMA writes them); 8-row core groups 8 * row bytes apart (SBO);
-// LBO unused for swizzled K-major layouts; version 1 (sm_100).
-template <int BKT>
-__device__ __forceinline__ uint64_t sdesc(uint32_t addr) {
-  static_assert(BKT == 64 || BKT == 32, "row of 128 or 64 bytes");
-  uint64_t d = (uint64_t)((addr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)((8 * BKT * 2) >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)(BKT == 64 ? 2 : 4) << 61;
-  return d;
-}
-// Shared-memory descriptor of an MN-major B operand, 128B swizzle: blocks of
-// 64 N-elements (128-byte rows), one row per K index, rows 128 bytes apart so
-// 8-row core groups are 1024 bytes apart (SBO), the BN / 64 blocks BKT rows
-// of 128 bytes apart (LBO) -- the layout TMA writes for boxes of 64 x BKT.
-template <int BKT>
-__device__ __forceinline__ uint64_t sdesc_mn(uint32_t addr) {
-  uint64_t d = (uint64_t)((addr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)((BKT * 128) >> 4) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
 // Instruction descriptor, kind::f16: D = F32, A = B = F16, both K-major.
 constexpr uint32_t kIdesc = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(BN >> 3) << 17) |
                             ((uint32_t)(BM >> 4) << 24);
@@ -164,31 +63,6 @@ __device__ __forceinline__ bool gated_off(const Epi& e) {
     return e.a.gate_count && *e.a.gate_count <= (unsigned long long)e.a.gate_cap;
   else
     return false;
-}
-
-struct Ctl {
-  volatile int* abort;
-  TcStatus* st;
-};
-
-__device__ bool bounded_wait(uint32_t bar, uint32_t parity, const Ctl& c, int site,
-                             uint64_t limit_ns = kWaitLimitNs) {
-  if (mbar_test(bar, parity)) return true;
-  const uint64_t t0 = globaltimer();
-  for (uint32_t it = 1;; ++it) {
-    if (mbar_test(bar, parity)) return true;
-    if ((it & 31) == 0) {
-      if (*c.abort) return false;
-      if (globaltimer() - t0 > limit_ns) {
-        *c.abort = 1;
-        if (atomicCAS(&c.st->code, 0, TC_TIMEOUT) == 0) {
-          c.st->where = site;
-          c.st->block = blockIdx.x;
-        }
-        return false;
-      }
-    }
-  }
 }
 
 // One bounded wait, with a short limit, on an mbarrier that nothing completes:
@@ -995,51 +869,6 @@ cudaError_t run_gemm(const TmapSet<Epi::kSets>& maps, int64_t m_tiles, int64_t n
 // the MMAs; both CTAs' TMA loads complete on the leader's barriers; the
 // leader's commits release both CTAs' stages and accumulators; each CTA's
 // epilogue drains its own 128 TMEM lanes (its patterns) x 256 rotations.
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// Address of the same shared-memory object in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t peer_addr(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// TMA load into this CTA's shared memory completing on the pair leader's barrier.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* tm, int c0, int c1,
-                                                 uint32_t bar_cluster) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"((uint64_t)tm), "r"(c0), "r"(c1), "r"(bar_cluster)
-      : "memory");
-}
-__device__ __forceinline__ void mma_f16_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
-                                             uint32_t accum) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accum)
-      : "memory");
-}
-// Arrive on an mbarrier (this CTA's or the peer's, shared::cluster address)
-// once every MMA this thread issued before has completed.
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar_cluster) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   bar_cluster)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster)
-               : "memory");
-}
 
 // M = 256 (the pair), N = 256.
 constexpr uint32_t kIdescPair = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
@@ -2106,8 +1935,10 @@ bool tc_encode_2d(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t ro
   return tc_encode_2d_strided(tm, base, inner, rows, inner, box_rows, box_inner);
 }
 
-bool tc_encode_2d_strided(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t rows,
-                          uint64_t ld, uint32_t box_rows, uint32_t box_inner) {
+// A 2D tensor map with 128- or 64-byte swizzled box rows.
+static bool encode_2d(CUtensorMap* tm, CUtensorMapDataType type, uint32_t elem, const void* base,
+                      uint64_t inner, uint64_t rows, uint64_t ld, uint32_t box_rows,
+                      uint32_t box_inner) {
   typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -2123,15 +1954,27 @@ bool tc_encode_2d_strided(CUtensorMap* tm, const void* base, uint64_t inner, uin
     fn = (EncodeFn)p;
   }
   const cuuint64_t dims[2] = {inner, rows};
-  const cuuint64_t strides[1] = {ld * 2};
-  if (box_inner != 64 && box_inner != 32) return false;
-  if (ld < inner || (ld * 2) % 16 != 0) return false;
+  const cuuint64_t strides[1] = {ld * elem};
+  if (box_inner * elem != 128 && box_inner * elem != 64) return false;
+  if (ld < inner || (ld * elem) % 16 != 0) return false;
   const cuuint32_t box[2] = {box_inner, box_rows};
   const cuuint32_t estr[2] = {1, 1};
-  return fn(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box,
-            estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            box_inner == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+  return fn(tm, type, 2, const_cast<void*>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE,
+            box_inner * elem == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool tc_encode_2d_strided(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t rows,
+                          uint64_t ld, uint32_t box_rows, uint32_t box_inner) {
+  return encode_2d(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, inner, rows, ld, box_rows,
+                   box_inner);
+}
+
+bool tc_encode_2d_bytes(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t rows,
+                        uint64_t ld, uint32_t box_rows, uint32_t box_inner) {
+  return encode_2d(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, inner, rows, ld, box_rows,
+                   box_inner);
 }
 
 cudaError_t launch_maximize_tc(const CUtensorMap& tmK, const CUtensorMap& tmBhi,

@@ -32,6 +32,10 @@ cudaError_t launch_wait_probe(TcStatus* status, uint64_t limit_ns, cudaStream_t 
 bool tc_encode_2d_strided(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t rows,
                           uint64_t ld, uint32_t box_rows, uint32_t box_inner);
 
+// A matrix of bytes (kernels_i8.cu).
+bool tc_encode_2d_bytes(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t rows,
+                        uint64_t ld, uint32_t box_rows, uint32_t box_inner);
+
 // Maximize contraction: acc[p][r] = sum_j K[p][j] (B_hi[r][j] + B_lo[r][j]),
 // 128 patterns x 256 rotations per tile.  Epilogue writes Y[r][p] (LL for
 // poisson, the cross term C for gaussian) and per pattern and rotation tile
