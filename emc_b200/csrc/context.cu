@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../include/emc_b200.h"
+#include "i8.cuh"
 #include "kernels.cuh"
 #include "proposal.cuh"
 #include "tc.cuh"
@@ -190,9 +191,19 @@ struct emc_context {
   float* d_S = nullptr;   // [R][npa]
   float* d_LL = nullptr;  // [R][N] responsibilities (FP32)
   double* d_LL64 = nullptr;  // [R][N] log-likelihood (FP64) the softmax reads
-  double* d_den = nullptr;
   double* d_lse32 = nullptr;
-  double* d_plogp_part = nullptr;
+  double* d_plogp32 = nullptr;
+  double4* d_part64 = nullptr;  // [parts][N] online log-sum-exp partials
+  double* d_Tpart64 = nullptr;  // [blocks][R] row totals and maxima of the P sweep
+  float *d_Mpart = nullptr, *d_rowmax = nullptr;
+  // the contractions on the byte tensor cores (kernels_i8.cu): counts as bytes
+  // by pattern and by pixel, the digit planes of the other operand (slices,
+  // then responsibilities).  i8_planes 0: the counts are not small integers,
+  // or the memory is not there, and the CUDA-core contractions run
+  int i8_planes = 0;
+  int8_t *d_i8 = nullptr, *d_K8 = nullptr, *d_Kt8 = nullptr, *d_digits = nullptr;
+  float* d_unit = nullptr;
+  CUtensorMap tmK8[2], tmKt8[2], tmXp, tmXn;
   // mixed path
   int64_t Npad = 0, Ppad = 0, Rpad = 0, nrt = 0;
   __half *d_Kh = nullptr, *d_Kt = nullptr, *d_Bhi = nullptr, *d_Blo = nullptr;
@@ -332,10 +343,17 @@ struct emc_context {
   emc_status alloc(T** p, size_t count, bool zero = false) {
     void* q = nullptr;
     const size_t bytes = count * sizeof(T) ? count * sizeof(T) : 16;
+    // the byte operands are a faster route, not a need: they make room
+    if (mem_limit && mem_used + bytes > mem_limit) drop_i8();
     if (mem_limit && mem_used + bytes > mem_limit)
       return fail(EMC_ERR_OOM, "device memory limit of %zu bytes reached (%zu held, %zu requested)",
                   mem_limit, mem_used, bytes);
     cudaError_t e = cudaMalloc(&q, bytes);
+    if (e == cudaErrorMemoryAllocation && i8_planes) {
+      cudaGetLastError();
+      drop_i8();
+      e = cudaMalloc(&q, bytes);
+    }
     if (e != cudaSuccess) return cuda(e, "cudaMalloc");
     allocs.push_back(q);
     alloc_bytes.push_back(bytes);
@@ -355,6 +373,13 @@ struct emc_context {
         mem_used -= alloc_bytes[k];
         alloc_bytes[k] = 0;
       }
+  }
+  // Gives the byte operands back (cudaFree waits for the kernels reading
+  // them); the CUDA-core contractions take over.
+  void drop_i8() {
+    i8_planes = 0;
+    if (d_i8) release(d_i8);
+    d_i8 = nullptr;
   }
 };
 
@@ -477,6 +502,7 @@ int64_t emc_launch_count(const emc_context* ctx) { return ctx ? ctx->launches : 
 
 emc_status emc_set_memory_limit(emc_context* c, size_t bytes) {
   if (!c) return EMC_ERR_ARG;
+  if (bytes && bytes < c->mem_used) c->drop_i8();
   if (bytes && bytes < c->mem_used)
     return c->fail(EMC_ERR_ARG, "limit %zu is below the %zu bytes already held", bytes,
                    c->mem_used);
@@ -610,9 +636,17 @@ static emc_status alloc_work(emc_context* c) {
     // than the contraction's own error
     TRY(c->alloc(&c->d_LL64, R * N));
     TRY(c->alloc(&c->d_K, N * npa));
-    TRY(c->alloc(&c->d_den, ((R + 127) / 128) * N));
-    TRY(c->alloc(&c->d_plogp_part, (N + 31) / 32 + 1));
-    TRY(c->alloc(&c->d_lse32, N));
+    // the responsibility pass's scratch, one allocation
+    const int64_t chunk = resp_f32_chunk(R, N), nparts = (R + chunk - 1) / chunk;
+    const int64_t nb = resp_f32_blocks(N);
+    double* w = nullptr;
+    TRY(c->alloc(&w, 4 * nparts * N + nb * R + 2 * N + (nb * R + R + 1) / 2));
+    c->d_part64 = reinterpret_cast<double4*>(w);
+    c->d_Tpart64 = w + 4 * nparts * N;
+    c->d_plogp32 = c->d_Tpart64 + nb * R;
+    c->d_lse32 = c->d_plogp32 + N;
+    c->d_Mpart = reinterpret_cast<float*>(c->d_lse32 + N);
+    c->d_rowmax = c->d_Mpart + nb * R;
     return EMC_OK;
   }
   c->Npad = round_up(N, 128);
@@ -768,6 +802,47 @@ emc_status emc_set_patterns(emc_context* c, const float* counts) {
   return finish_patterns(c);
 }
 
+// The byte operands of an FP32 context whose largest count is `top` (every
+// count an integer): one digit plane up to 127, two above.  They are kept only
+// where they take less than half of the memory that is left, and the CUDA-core
+// contractions run without them.
+static void i8_prepare(emc_context* c, float top) {
+  const int64_t N = c->N, R = c->R, npa = c->npa;
+  const int planes = top <= (float)kI8MaxCount ? 1 : 2;
+  // 32-bit sums: 128 x the total of a row of counts
+  const double most = std::min((double)top, (double)kI8MaxCount) * (double)std::max(N, npa);
+  const int64_t ldK = round_up(npa, 16), ldT = round_up(N, 16);
+  auto pad = [](size_t n) { return (n + 255) / 256 * 256; };
+  const size_t digits = pad((size_t)kI8Digits * (size_t)R * (size_t)std::max(ldK, ldT));
+  const size_t k8 = pad((size_t)planes * (size_t)(N * ldK)), kt8 = pad((size_t)planes * (size_t)(npa * ldT));
+  const size_t bytes = k8 + kt8 + digits + sizeof(float) * (size_t)R;
+  const bool fits = top <= (float)kI8MaxCount2 && most <= kI8MaxTotal &&
+                    (double)R * kI8Digits < 2147483647.0 &&
+                    ((bytes <= ((size_t)64 << 20) && !c->mem_limit) || c->i8_planes == planes ||
+                     bytes <= avail_bytes(c, 0) / 2);
+  if (c->i8_planes == planes && fits) return;  // sized for these patterns already
+  c->drop_i8();
+  if (!fits) return;
+  const std::string err = c->err;
+  if (c->alloc(&c->d_i8, bytes) != EMC_OK) {
+    cudaGetLastError();
+    c->d_i8 = nullptr;
+    c->err = err;
+    return;
+  }
+  c->i8_planes = planes;
+  c->d_K8 = c->d_i8;
+  c->d_Kt8 = c->d_K8 + k8;
+  c->d_digits = c->d_Kt8 + kt8;
+  c->d_unit = reinterpret_cast<float*>(c->d_digits + digits);
+  bool ok = i8_encode(&c->tmXp, c->d_digits, npa, kI8Digits * R, ldK, false) &&
+            i8_encode(&c->tmXn, c->d_digits, N, kI8Digits * R, ldT, false);
+  for (int k = 0; k < planes && ok; ++k)
+    ok = i8_encode(&c->tmK8[k], c->d_K8 + (int64_t)k * N * ldK, npa, N, ldK, true) &&
+         i8_encode(&c->tmKt8[k], c->d_Kt8 + (int64_t)k * npa * ldT, N, npa, ldT, true);
+  if (!ok) c->drop_i8();
+}
+
 // Pattern statistics and the FP16 operands of the compact counts d_K.
 static emc_status finish_patterns(emc_context* c) {
   const int64_t N = c->N, npa = c->npa;
@@ -775,14 +850,19 @@ static emc_status finish_patterns(emc_context* c) {
   cudaError_t e = launch_pattern_stats(compact, nullptr, N, npa, npa, 1, c->d_patsq, c->st);
   if (e == cudaSuccess) e = launch_pattern_stats(compact, nullptr, N, npa, npa, 0, c->d_patsum, c->st);
   int bad = 0;
-  int* d_bad = reinterpret_cast<int*>(c->d_scratch);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_bad, 0, sizeof(int), c->st);
+  // mixed: [0] counts the path cannot take; FP32: largest count (bits),
+  // non-integers, invalid counts
+  unsigned int seen[3] = {0, 0, 0};
+  unsigned int* d_seen = reinterpret_cast<unsigned int*>(c->d_scratch);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d_seen, 0, sizeof(seen), c->st);
   if (e == cudaSuccess && c->mixed)
-    e = launch_pack_patterns(compact, N, npa, c->Npad, c->Ppad, c->d_Kh, c->d_Kt, d_bad, c->st);
+    e = launch_pack_patterns(compact, N, npa, c->Npad, c->Ppad, c->d_Kh, c->d_Kt,
+                             reinterpret_cast<int*>(d_seen), c->st);
   else if (e == cudaSuccess)
-    e = launch_count_invalid(compact, N * npa, d_bad, c->st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, c->st);
+    e = launch_count_range(compact, N * npa, (float)kI8MaxCount2, d_seen, c->st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(seen, d_seen, sizeof(seen), cudaMemcpyDeviceToHost, c->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
+  bad = (int)(c->mixed ? seen[0] : seen[2]);
   if (e != cudaSuccess) return c->cuda(e, "emc_set_patterns");
   c->have_pat = false;
   if (bad && c->mixed)
@@ -791,6 +871,16 @@ static emc_status finish_patterns(emc_context* c) {
                    bad);
   if (bad)
     return c->fail(EMC_ERR_RANGE, "%d counts are negative, NaN or infinite", bad);
+  if (!c->mixed && seen[1] == 0) {
+    float top;
+    std::memcpy(&top, &seen[0], sizeof(top));
+    i8_prepare(c, top);
+    if (c->i8_planes)
+      CK(c, launch_pack_counts_i8(compact, N, npa, c->i8_planes, round_up(npa, 16),
+                                  round_up(N, 16), c->d_K8, c->d_Kt8, c->st));
+  } else {
+    c->drop_i8();
+  }
   c->have_pat = true;
   c->csr.valid = false;
   c->csc.valid = false;
@@ -895,8 +985,9 @@ emc_status emc_expand(emc_context* c) {
   if (!c->mixed) {
     a.ld = c->npa;
     a.out = c->gauss ? EXP_F32 : EXP_LOG_F32;
-    a.stat = c->gauss ? STAT_NONE : STAT_SUM;
+    a.stat = c->gauss ? STAT_SUMSQ : STAT_SUM;
     a.out_f32 = c->d_S;
+    a.rowmax = c->d_rowmax;
   } else {
     a.ld = c->Ppad;
     a.out = EXP_F16_SPLIT;
@@ -1303,6 +1394,51 @@ static emc_status sparse_loglik(emc_context* c) {
   return EMC_OK;
 }
 
+// The FP32 contexts' log-likelihood on the byte tensor cores: the slices as
+// digit planes, then the contraction with the counts (twice when a count
+// exceeds 127).
+static emc_status i8_loglik(emc_context* c) {
+  CK(c, launch_quant_rows(c->d_S, nullptr, c->d_rowmax, c->R, c->npa, round_up(c->npa, 16),
+                          c->d_digits, c->d_unit, c->st));
+  I8LLArgs a{};
+  a.R = c->R;
+  a.N = c->N;
+  a.poisson = c->gauss ? 0 : 1;
+  a.unit = c->d_unit;
+  a.scaling = c->d_scaling_prev;
+  a.rowstat = c->d_rowstat;
+  a.patstat = c->d_patsq;
+  a.gauss_inv = gauss_inv(c);
+  a.LL = c->d_LL64;
+  for (int k = c->i8_planes - 1; k >= 0; --k) {
+    a.pass = c->i8_planes == 1 ? I8_ONLY : k ? I8_HIGH : I8_LOW;
+    a.mult = k ? 128.0 : 1.0;
+    CK(c, launch_i8_loglik(c->tmK8[k], c->tmXp, c->npa, a, c->d_status, c->num_sms, c->st));
+  }
+  c->launches += 1 + c->i8_planes;
+  return EMC_OK;
+}
+
+// The slice sums the same way: P / phi as digit planes (its row maxima come
+// from the responsibility sweep), contracted with the counts by pixel.
+static emc_status i8_slicesums(emc_context* c) {
+  CK(c, launch_quant_rows(c->d_LL, c->d_scaling, c->d_rowmax, c->R, c->N, round_up(c->N, 16),
+                          c->d_digits, c->d_unit, c->st));
+  I8UArgs a{};
+  a.R = c->R;
+  a.npa = c->npa;
+  a.unit = c->d_unit;
+  a.T = c->d_T;
+  a.U = c->d_S;  // the averaged slices replace the expanded ones (emc_atomic.cu:96)
+  for (int k = c->i8_planes - 1; k >= 0; --k) {
+    a.pass = c->i8_planes == 1 ? I8_ONLY : k ? I8_HIGH : I8_LOW;
+    a.mult = k ? 128.0 : 1.0;
+    CK(c, launch_i8_slices(c->tmKt8[k], c->tmXn, c->N, a, c->d_status, c->num_sms, c->st));
+  }
+  c->launches += 1 + c->i8_planes;
+  return EMC_OK;
+}
+
 // The slice sums U[r][j] = sum_p P_rp K_pj / phi_p / T_r as a gather over
 // each active pixel's non-zero counts: the counts' entries by pixel (built
 // once per pattern upload from a transposed copy of K), divided by the
@@ -1349,6 +1485,8 @@ emc_status emc_maximize(emc_context* c) {
                         cudaMemcpyDeviceToDevice, c->st));
   if (!c->mixed && c->tune.maximize_sparse) {
     TRY(sparse_loglik(c));
+  } else if (!c->mixed && c->i8_planes) {
+    TRY(i8_loglik(c));
   } else if (!c->mixed) {
     LLArgs l{};
     l.A = c->d_S;
@@ -1366,16 +1504,38 @@ emc_status emc_maximize(emc_context* c) {
     l.LL = c->d_LL;
     l.LL64 = c->d_LL64;
     CK(c, launch_ll_fp32(l, c->st));
+    c->launches += 1;
   }
   if (!c->mixed) {
     c->mark(2);
-    int nparts = 0;
-    CK(c, launch_softmax_from_f64(c->d_LL64, c->d_LL, R, N, c->d_plogp_part, &nparts,
-                                  c->d_lse32, c->st));
-    CK(c, launch_sum_f64(c->d_plogp_part, nparts, c->d_stats + 2, c->st));
-    CK(c, launch_sum_f64(c->d_lse32, N, c->d_stats + 3, c->st));
-    int64_t nden = 0;
-    if (c->gauss) {
+    RespF32Args a{};
+    a.R = R;
+    a.N = N;
+    a.poisson = c->gauss ? 0 : 1;
+    a.LL = c->d_LL64;
+    a.scaling = c->d_scaling_prev;
+    a.rowstat = c->d_rowstat;
+    a.patstat = c->d_patsq;
+    a.patsum = c->d_patsum;
+    a.gauss_inv = gauss_inv(c);
+    a.part = c->d_part64;
+    a.chunk = resp_f32_chunk(R, N);
+    a.nparts = (R + a.chunk - 1) / a.chunk;
+    a.lse = c->d_lse32;
+    a.plogp = c->d_plogp32;
+    // the gaussian scaling's sum P C comes from the log-likelihood (2 C / phi
+    // is one of its terms) where that is exact to FP64; the CUDA-core form
+    // sums (S - K / phi)^2 in FP32, which leaves C too few digits where phi is
+    // far off, so there the cross term is contracted by itself
+    const bool cross = c->gauss && !c->i8_planes;
+    a.new_scaling = cross ? nullptr : c->d_scaling;
+    a.P = c->d_LL;
+    a.Tpart = c->d_Tpart64;
+    a.Mpart = c->d_Mpart;
+    a.T = c->d_T;
+    a.rowmax = c->d_rowmax;
+    CK(c, launch_resp_f32(a, c->st));
+    if (cross) {
       CrossArgs x{};
       x.S = c->d_S;
       x.K = c->d_K;
@@ -1385,16 +1545,15 @@ emc_status emc_maximize(emc_context* c) {
       x.npa = c->npa;
       x.ldS = c->npa;
       x.ldK = c->npa;
-      x.den_part = c->d_den;
+      x.den_part = reinterpret_cast<double*>(c->d_part64);  // free again, and large enough
       CK(c, launch_scaling_cross(x, c->st));
-      nden = (R + 127) / 128;
-    } else {
-      CK(c, launch_scaling_rowweighted(c->d_LL, c->d_rowstat, R, N, c->d_den, &nden, c->st));
+      CK(c, launch_scaling_finish(c->d_patsq, x.den_part, (R + 127) / 128, N, c->d_scaling,
+                                  c->st));
+      c->launches += 2;
     }
-    CK(c, launch_scaling_finish(c->gauss ? c->d_patsq : c->d_patsum, c->d_den, nden, N,
-                                c->d_scaling, c->st));
-    CK(c, launch_row_sums(c->d_LL, R, N, c->d_T, c->st));
-    c->launches += 8;
+    CK(c, launch_sum_f64(c->d_plogp32, N, c->d_stats + 2, c->st));
+    CK(c, launch_sum_f64(c->d_lse32, N, c->d_stats + 3, c->st));
+    c->launches += 6;
   } else if (c->y_rows < R) {
     TRY(chunked_maximize(c));
   } else {
@@ -1434,6 +1593,8 @@ emc_status emc_compress_insert(emc_context* c) {
   if (!c->mixed) {
     if (c->tune.compress_sparse) {
       TRY(sparse_slicesums(c));
+    } else if (c->i8_planes) {
+      TRY(i8_slicesums(c));
     } else {
       CompressArgs a{};
       a.P = c->d_LL;
@@ -1447,6 +1608,7 @@ emc_status emc_compress_insert(emc_context* c) {
       a.ldU = c->npa;
       a.U = c->d_S;  // the averaged slices replace the expanded ones (emc_atomic.cu:96)
       CK(c, launch_compress_fp32(a, c->st));
+      c->launches += 1;
     }
     InsertArgs in{};
     in.U = c->d_S;
@@ -1467,7 +1629,7 @@ emc_status emc_compress_insert(emc_context* c) {
     in.weight = c->d_weight;
     in.acc64 = c->det ? c->d_acc64 : nullptr;
     CK(c, launch_insert(in, c->st));
-    c->launches += 2;
+    c->launches += 1;
   } else {
     CmpEpiArgs e = cmp_args(c);
     e.acc64 = c->det ? c->d_acc64 : nullptr;
@@ -2258,8 +2420,6 @@ static emc_status run_proposed(emc_context* c, const ProposedPlan& pl, Select se
   if (!c->ev_sel) CK(c, cudaEventCreateWithFlags(&c->ev_sel, cudaEventDisableTiming));
   CK(c, cudaEventRecord(c->ev_sel, c->st));
   TRY(emc_expand(c));
-  if (!c->mixed && c->gauss)  // the grouped gaussian LL uses the expanded form: sum_j S_rj^2
-    CK(c, launch_pattern_stats(c->d_S, nullptr, R, c->npa, c->npa, 1, c->d_rowstat, c->st));
   float* captured = nullptr;
   const int32_t n_aud = (int32_t)std::min<int64_t>(pl.audit, std::min<int64_t>(N, 128));
   if (n_aud > 0) TRY(run_audit(c, n_aud, m, &captured));
@@ -2576,7 +2736,7 @@ static emc_status run_proposed(emc_context* c, const ProposedPlan& pl, Select se
   CK(c, launch_sum_f64(c->d_lse_c, N, c->d_stats + 3, c->st));
   c->mark(5);
   // select, the grouped stages, normalise (4), two sums
-  c->launches += 1 + launches + 6 + ((!c->mixed && c->gauss) ? 1 : 0);
+  c->launches += 1 + launches + 6;
   c->stage = 0;
   TRY(check_status(c));
   double h[4];

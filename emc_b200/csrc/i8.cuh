@@ -1,0 +1,60 @@
+// FP32 contexts' contractions on the byte tensor cores (kernels_i8.cu): launch
+// interface.  X is quantised row by row into four digit planes D [4][R][ld]
+// (launch_quant_rows); the counts are bytes, in two base-128 planes when one
+// exceeds 127 (the contraction then runs twice, I8_HIGH then I8_LOW).
+#pragma once
+#include <cstdint>
+
+#include "tc.cuh"
+
+namespace emc {
+
+constexpr int kI8Digits = 4;
+constexpr int kI8MaxCount = 127;            // one plane
+constexpr int kI8MaxCount2 = 127 * 128 + 127;  // two
+// Elements of a row of X per unit of count: 32-bit sums hold 128 x the total
+// count of a row of the count operand.
+constexpr double kI8MaxTotal = 2147483647.0 / 128.0;
+
+enum I8Pass { I8_ONLY = 0, I8_HIGH = 1, I8_LOW = 2 };
+
+struct I8LLArgs {
+  int64_t R, N;
+  int poisson, pass;
+  double mult;             // 1, or 128 (I8_HIGH)
+  const float* unit;       // [R]
+  const float* scaling;    // [N]
+  const double* rowstat;   // [R] sum W or sum S^2
+  const double* patstat;   // [N] gaussian: sum K^2
+  double gauss_inv;
+  double* LL;              // [R][N]
+};
+struct I8UArgs {
+  int64_t R, npa;
+  int pass;
+  double mult;
+  const float* unit;       // [R]
+  const float* T;          // [R]
+  float* U;                // [R][npa]
+};
+
+// Tensor map of a byte operand: the counts (inner = contraction extent) or
+// the digit planes (rows = 4 R).  ld is a multiple of 16 bytes; bytes between
+// inner and ld are never read.
+bool i8_encode(CUtensorMap* tm, const void* base, int64_t inner, int64_t rows, int64_t ld,
+               bool counts);
+cudaError_t launch_i8_loglik(const CUtensorMap& tmK, const CUtensorMap& tmX, int64_t npa,
+                             const I8LLArgs& a, TcStatus* status, int num_sms, cudaStream_t st);
+cudaError_t launch_i8_slices(const CUtensorMap& tmKt, const CUtensorMap& tmX, int64_t N,
+                             const I8UArgs& a, TcStatus* status, int num_sms, cudaStream_t st);
+// rowmax [R]: the largest |X| of the row (after the division by div[column]).
+cudaError_t launch_quant_rows(const float* X, const float* div, const float* rowmax, int64_t R,
+                              int64_t cols, int64_t ld, int8_t* D, float* unit, cudaStream_t st);
+cudaError_t launch_pack_counts_i8(const float* K, int64_t N, int64_t npa, int planes, int64_t ldK,
+                                  int64_t ldT, int8_t* K8, int8_t* Kt8, cudaStream_t st);
+// out[0] = bits of the largest entry, out[1] = entries that are not integers
+// in [0, limit], out[2] = entries that are negative, NaN or infinite.
+cudaError_t launch_count_range(const float* x, int64_t n, float limit, unsigned int* out,
+                               cudaStream_t st);
+
+}  // namespace emc

@@ -26,6 +26,7 @@ struct ExpandArgs {
   __half* out_hi;
   __half* out_lo;
   double* rowstat;      // [R] or nullptr
+  float* rowmax;        // [R] largest magnitude of the row's output, or nullptr (FP32 outputs)
   // optional, nearest + EXP_F16_SPLIT: per-voxel table from launch_expand_table
   // ([side^3 + 1], the last entry for pixels that fall outside the grid)
   const uint2* tab;
@@ -109,13 +110,35 @@ cudaError_t launch_csr_fill(const float* K, int64_t N, int64_t npa, const int64_
 // Per-pattern softmax over r of X[r][p] (in place), FP32 arithmetic as the
 // reference; plogp_part[blockIdx] receives sum P log P partials (FP64) and
 // lse[p] (optional) the pattern's log-sum-exp.
-// The same per-pattern softmax from an FP64 log-likelihood L [R][N] into the
-// FP32 responsibilities P [R][N].
-cudaError_t launch_softmax_from_f64(const double* L, float* P, int64_t R, int64_t N,
-                                    double* plogp_part, int* nparts, double* lse,
-                                    cudaStream_t st);
 cudaError_t launch_softmax_fp32(float* X, int64_t R, int64_t N, double* plogp_part,
                                 int* nparts, double* lse, cudaStream_t st);
+// The responsibility pass of the FP32 contexts from an FP64 log-likelihood
+// LL [R][N]: per pattern lse, the new scaling and sum P log P (stats, over
+// `nparts` row chunks, then combine), then P [R][N] with each row's total T_r
+// and its largest P / phi (new phi).
+struct RespF32Args {
+  int64_t R, N;
+  int poisson;
+  const double* LL;
+  const float* scaling;    // [N] phi of the log-likelihood
+  const double* rowstat;   // [R] poisson: sum W; gaussian: sum S^2
+  const double* patstat;   // [N] gaussian: sum K^2
+  const double* patsum;    // [N] poisson: sum K
+  double gauss_inv;
+  double4* part;           // [nparts][N]
+  int64_t nparts, chunk;   // rows per chunk
+  double* lse;             // [N]
+  double* plogp;           // [N]
+  float* new_scaling;      // [N], or nullptr: left to the caller
+  float* P;                // [R][N]
+  double* Tpart;           // [resp_f32_blocks(N)][R]
+  float* Mpart;            // [resp_f32_blocks(N)][R]
+  float* T;                // [R]
+  float* rowmax;           // [R]
+};
+int64_t resp_f32_chunk(int64_t R, int64_t N);
+int64_t resp_f32_blocks(int64_t N);
+cudaError_t launch_resp_f32(const RespF32Args& a, cudaStream_t st);
 // sum of x log x over n floats into *out (FP64).
 cudaError_t launch_xlogx_sum(const float* x, int64_t n, double* out, double* scratch,
                              cudaStream_t st);
@@ -130,9 +153,6 @@ struct CrossArgs {
   double* den_part;      // [ceil(R/128)][N]
 };
 cudaError_t launch_scaling_cross(const CrossArgs& a, cudaStream_t st);
-// den[p] = sum_r P_rp w_r   (poisson scaling), deterministic two-level reduce.
-cudaError_t launch_scaling_rowweighted(const float* P, const double* w, int64_t R, int64_t N,
-                                       double* den_part, int64_t* nparts, cudaStream_t st);
 // phi_p = num_p / sum_k den_part[k][p] where both are positive, else unchanged.
 cudaError_t launch_scaling_finish(const double* num, const double* den_part, int64_t nparts,
                                   int64_t N, float* scaling, cudaStream_t st);
@@ -194,7 +214,5 @@ cudaError_t launch_model_max(const float* model, int64_t M, double* scratch, dou
                              cudaStream_t st);
 cudaError_t launch_fill(float* x, int64_t n, float v, cudaStream_t st);
 cudaError_t launch_sum_f64(const double* x, int64_t n, double* out, cudaStream_t st);
-// bad[0] += number of entries of x that are negative, NaN or infinite.
-cudaError_t launch_count_invalid(const float* x, int64_t n, int* bad, cudaStream_t st);
 
 }  // namespace emc

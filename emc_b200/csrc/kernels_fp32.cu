@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(kBlock) expand_kernel(const ExpandArgs a) {
   float m[9];
   emc_voxel::rotation_matrix(a.quat + 4 * r, m);
   double stat = 0.0;
+  float big = 0.0f;
   const int64_t step = (int64_t)blockDim.x * kExpandUnroll;
   for (int64_t i0 = threadIdx.x; i0 < a.ld; i0 += step) {
     float w[kExpandUnroll];
@@ -150,8 +151,11 @@ __global__ void __launch_bounds__(kBlock) expand_kernel(const ExpandArgs a) {
         const int64_t o = r * a.ld + i;
         if (OUT == EXP_F32) {
           a.out_f32[o] = w[u];
+          big = fmaxf(big, fabsf(w[u]));
         } else if (OUT == EXP_LOG_F32) {
-          a.out_f32[o] = real ? logf(fmaxf(w[u], a.floor_)) : 0.0f;
+          const float x = real ? logf(fmaxf(w[u], a.floor_)) : 0.0f;
+          a.out_f32[o] = x;
+          big = fmaxf(big, fabsf(x));
         } else {
           const float x = real ? (a.log_split ? logf(fmaxf(w[u], a.floor_)) : w[u]) : 0.0f;
           const __half hi = __float2half_rn(x);
@@ -164,6 +168,11 @@ __global__ void __launch_bounds__(kBlock) expand_kernel(const ExpandArgs a) {
   if (a.rowstat) {
     const double s = block_sum(stat, red);
     if (threadIdx.x == 0) a.rowstat[r] = s;
+  }
+  if (a.rowmax) {
+    __syncthreads();  // red is free again
+    const float mx = block_max(big, reinterpret_cast<float*>(red));
+    if (threadIdx.x == 0) a.rowmax[r] = mx;
   }
 }
 
@@ -353,21 +362,19 @@ struct OpCompress {
 };
 
 // ----------------------------------------------------------------- softmax --
-// 32 patterns per block (lane == pattern), 8 warps share the rotations.  The
-// log-likelihood is read from X (FP32, then overwritten by P in place) or, for
-// an FP64 log-likelihood, from X64 with P written to X.
-template <class T>
-__device__ __forceinline__ void softmax_body(const T* L, float* X, int64_t R, int64_t N,
-                                             double* plogp_part, double* lse) {
-  __shared__ T smax[8][32];
+// 32 patterns per block (lane == pattern), 8 warps share the rotations; X is
+// the FP32 log-likelihood, overwritten by P in place (the drop-in API).
+__global__ void __launch_bounds__(kBlock) softmax_kernel(float* X, int64_t R, int64_t N,
+                                                         double* plogp_part, double* lse) {
+  __shared__ float smax[8][32];
   __shared__ float ssum[8][32];
   __shared__ double sred[8][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t p = (int64_t)blockIdx.x * 32 + lane;
   const bool ok = p < N;
-  T mx = -FLT_MAX;
+  float mx = -FLT_MAX;
   if (ok)
-    for (int64_t r = w; r < R; r += 8) mx = L[r * N + p] > mx ? L[r * N + p] : mx;
+    for (int64_t r = w; r < R; r += 8) mx = X[r * N + p] > mx ? X[r * N + p] : mx;
   smax[w][lane] = mx;
   __syncthreads();
   mx = smax[0][lane];
@@ -375,7 +382,7 @@ __device__ __forceinline__ void softmax_body(const T* L, float* X, int64_t R, in
   float s = 0.0f;
   if (ok)
     for (int64_t r = w; r < R; r += 8) {
-      const float d = (float)(L[r * N + p] - mx);
+      const float d = X[r * N + p] - mx;
       if (d > -1.0e10f) s += expf(d);  // emc_cuda.cu:463-468
     }
   ssum[w][lane] = s;
@@ -387,7 +394,7 @@ __device__ __forceinline__ void softmax_body(const T* L, float* X, int64_t R, in
   double pl = 0.0;
   if (ok)
     for (int64_t r = w; r < R; r += 8) {
-      const float d = (float)(L[r * N + p] - mx);
+      const float d = X[r * N + p] - mx;
       const float P = d > -1.0e10f ? expf(d) * inv : 0.0f;
       X[r * N + p] = P;
       if (P > 0.0f) pl += (double)P * log((double)P);
@@ -402,15 +409,193 @@ __device__ __forceinline__ void softmax_body(const T* L, float* X, int64_t R, in
   }
 }
 
-__global__ void __launch_bounds__(kBlock) softmax_kernel(float* X, int64_t R, int64_t N,
-                                                         double* plogp_part, double* lse) {
-  softmax_body<float>(X, X, R, N, plogp_part, lse);
+// ------------------------------------ responsibilities of the FP32 contexts --
+// Two sweeps over the FP64 log-likelihood, both bound by its HBM traffic.  One
+// block walking every rotation of 32 patterns (63 blocks on 148 SMs at 2,000
+// patterns) took 3.6 ms at 2,000 x 25,680 and 4.1 ms at 10,000 x 25,680; with
+// the rotations split over blocks the two sweeps take 0.4 and 1.5 ms:
+//   stats    per (row chunk, pattern) the online log-sum-exp and the sums the
+//            scaling and sum P log P need, merged by resp_combine_kernel;
+//   resp     P = exp(LL - lse), its row totals and row maxima.
+// Exponentials are FP32 of FP64 differences; eight of them are summed in FP32
+// and folded into FP64.
+constexpr int kStatRows = 8;  // rows in flight per warp
+
+struct StatAcc {
+  double m, s, d, q;  // max; sum e, sum e X, sum e (LL - m), e = exp(LL - m)
+};
+__device__ __forceinline__ void stat_rescale(StatAcc& a, double m) {
+  if (m > a.m) {
+    const double f = a.m > -DBL_MAX ? exp(a.m - m) : 0.0;
+    a.q = f > 0.0 ? f * (a.q + (a.m - m) * a.s) : 0.0;
+    a.s *= f;
+    a.d *= f;
+    a.m = m;
+  }
+}
+__device__ __forceinline__ void stat_merge(StatAcc& a, const StatAcc& b) {
+  if (b.m <= -DBL_MAX) return;
+  stat_rescale(a, b.m);
+  const double f = exp(b.m - a.m);
+  a.q += f > 0.0 ? f * (b.q + (b.m - a.m) * b.s) : 0.0;
+  a.s += f * b.s;
+  a.d += f * b.d;
 }
 
-__global__ void __launch_bounds__(kBlock) softmax64_kernel(const double* L, float* X, int64_t R,
-                                                           int64_t N, double* plogp_part,
-                                                           double* lse) {
-  softmax_body<double>(L, X, R, N, plogp_part, lse);
+template <bool POISSON>
+__global__ void __launch_bounds__(256) resp_stats_kernel(const RespF32Args a) {
+  __shared__ double sh[8][32][4];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t cols = (a.N + 31) / 32, by = blockIdx.x / cols;
+  const int64_t p = (blockIdx.x - by * cols) * 32 + lane;
+  const bool ok = p < a.N;
+  const int64_t r0 = by * a.chunk;
+  const int64_t r1 = r0 + a.chunk < a.R ? r0 + a.chunk : a.R;
+  // gaussian: X = sum S K from LL = (2 X / phi - sum S^2 - sum K^2 / phi^2) inv
+  double half_phi = 0.0, k2 = 0.0, ginv = 0.0;
+  if (!POISSON && ok) {
+    const double phi = a.scaling[p];
+    half_phi = 0.5 * phi;
+    k2 = a.patstat[p] / (phi * phi);
+    ginv = 1.0 / a.gauss_inv;
+  }
+  StatAcc acc{-DBL_MAX, 0.0, 0.0, 0.0};
+  for (int64_t r = r0 + w * kStatRows; r < r1; r += 8 * kStatRows) {
+    double v[kStatRows];
+    double cm = -DBL_MAX;
+#pragma unroll
+    for (int k = 0; k < kStatRows; ++k)
+      v[k] = ok && r + k < r1 ? a.LL[(r + k) * a.N + p] : -DBL_MAX;
+#pragma unroll
+    for (int k = 0; k < kStatRows; ++k) cm = v[k] > cm ? v[k] : cm;
+    stat_rescale(acc, cm);
+    float s = 0.0f, d = 0.0f, q = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kStatRows; ++k) {
+      if (!(ok && r + k < r1)) continue;
+      const float dl = fmaxf((float)(v[k] - acc.m), -1.0e4f);
+      const float e = expf(dl);
+      const double rs = a.rowstat[r + k];
+      const float x = POISSON ? (float)rs : (float)(fma(v[k], ginv, rs + k2) * half_phi);
+      s += e;
+      d = fmaf(e, x, d);
+      q = fmaf(e, dl, q);
+    }
+    acc.s += (double)s;
+    acc.d += (double)d;
+    acc.q += (double)q;
+  }
+  sh[w][lane][0] = acc.m;
+  sh[w][lane][1] = acc.s;
+  sh[w][lane][2] = acc.d;
+  sh[w][lane][3] = acc.q;
+  __syncthreads();
+  if (w == 0 && ok) {
+    for (int k = 1; k < 8; ++k)
+      stat_merge(acc, StatAcc{sh[k][lane][0], sh[k][lane][1], sh[k][lane][2], sh[k][lane][3]});
+    a.part[by * a.N + p] = make_double4(acc.m, acc.s, acc.d, acc.q);
+  }
+}
+
+__global__ void __launch_bounds__(256) resp_combine_kernel(const RespF32Args a) {
+  __shared__ double sh[8][32][4];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t p = (int64_t)blockIdx.x * 32 + lane;
+  StatAcc acc{-DBL_MAX, 0.0, 0.0, 0.0};
+  if (p < a.N)
+    for (int64_t k = w; k < a.nparts; k += 8) {
+      const double4 v = a.part[k * a.N + p];
+      stat_merge(acc, StatAcc{v.x, v.y, v.z, v.w});
+    }
+  sh[w][lane][0] = acc.m;
+  sh[w][lane][1] = acc.s;
+  sh[w][lane][2] = acc.d;
+  sh[w][lane][3] = acc.q;
+  __syncthreads();
+  if (w != 0 || p >= a.N) return;
+  for (int k = 1; k < 8; ++k)
+    stat_merge(acc, StatAcc{sh[k][lane][0], sh[k][lane][1], sh[k][lane][2], sh[k][lane][3]});
+  const double ls = log(acc.s);
+  a.lse[p] = acc.m + ls;
+  a.plogp[p] = acc.q / acc.s - ls;  // sum P (LL - lse)
+  // emc_cuda.cu:226; a pattern without photons or weight keeps its scale
+  const double num = a.poisson ? a.patsum[p] : a.patstat[p], den = acc.d / acc.s;
+  if (a.new_scaling) a.new_scaling[p] = num > 0.0 && den > 0.0 ? (float)(num / den) : a.scaling[p];
+}
+
+constexpr int kRespRows = 32;
+
+// 256 patterns x 32 rows per block, a warp 32 patterns; 16 rows at a time are
+// reduced over the warp by halving exchanges (16 + 1 shuffles instead of 80).
+__global__ void __launch_bounds__(256) resp_kernel(const RespF32Args a) {
+  __shared__ double st[8][kRespRows];
+  __shared__ uint32_t sm[8][kRespRows];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t cols = (a.N + 255) / 256, by = blockIdx.x / cols, bx = blockIdx.x - by * cols;
+  const int64_t p = bx * 256 + threadIdx.x;
+  const bool ok = p < a.N;
+  const double lse = ok ? a.lse[p] : 0.0;
+  const float phi = ok ? (a.new_scaling ? a.new_scaling : a.scaling)[p] : 1.0f;
+  const int64_t r0 = by * kRespRows;
+#pragma unroll
+  for (int h = 0; h < kRespRows; h += 16) {
+    double v[16];
+    uint32_t b[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k)
+      v[k] = ok && r0 + h + k < a.R ? a.LL[(r0 + h + k) * a.N + p] : -DBL_MAX;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      float P = 0.0f;
+      if (ok && r0 + h + k < a.R) {
+        P = expf((float)(v[k] - lse));
+        a.P[(r0 + h + k) * a.N + p] = P;
+      }
+      v[k] = (double)P;
+      b[k] = __float_as_uint(P / phi);  // >= 0; a NaN stays the largest
+    }
+#pragma unroll
+    for (int o = 16, n = 8; n >= 1; o >>= 1, n >>= 1) {
+      const bool hi = lane & o;
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        const double keep = hi ? v[i + n] : v[i], send = hi ? v[i] : v[i + n];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        const uint32_t kb = hi ? b[i + n] : b[i], sb = hi ? b[i] : b[i + n];
+        b[i] = max(kb, __shfl_xor_sync(0xffffffffu, sb, o));
+      }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    b[0] = max(b[0], __shfl_xor_sync(0xffffffffu, b[0], 1));
+    if (!(lane & 1)) {
+      st[w][h + (lane >> 1)] = v[0];
+      sm[w][h + (lane >> 1)] = b[0];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < kRespRows && r0 + threadIdx.x < a.R) {
+    double t = 0.0;
+    uint32_t mx = 0;
+    for (int k = 0; k < 8; ++k) {
+      t += st[k][threadIdx.x];
+      mx = max(mx, sm[k][threadIdx.x]);
+    }
+    a.Tpart[bx * a.R + r0 + threadIdx.x] = t;
+    a.Mpart[bx * a.R + r0 + threadIdx.x] = __uint_as_float(mx);
+  }
+}
+
+__global__ void resp_rows_kernel(const RespF32Args a, int64_t nblk) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= a.R) return;
+  double t = 0.0;
+  uint32_t mx = 0;
+  for (int64_t b = 0; b < nblk; ++b) {
+    t += a.Tpart[b * a.R + r];
+    mx = max(mx, __float_as_uint(a.Mpart[b * a.R + r]));
+  }
+  a.T[r] = (float)t;
+  a.rowmax[r] = __uint_as_float(mx);
 }
 
 __global__ void xlogx_partial(const float* x, int64_t n, double* part) {
@@ -434,26 +619,6 @@ __global__ void sum_f64_kernel(const double* x, int64_t n, double* out) {
 }
 
 // --------------------------------------------------------------- scaling --
-// den_part[blockIdx.y][p] = sum_{r in chunk} P_rp w_r; lane == pattern.
-__global__ void __launch_bounds__(kBlock) rowweighted_kernel(const float* P, const double* wr,
-                                                             int64_t R, int64_t N, int64_t rchunk,
-                                                             double* part) {
-  __shared__ double red[8][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t p = (int64_t)blockIdx.x * 32 + lane;
-  const int64_t r0 = (int64_t)blockIdx.y * rchunk, r1 = min(R, r0 + rchunk);
-  double s = 0;
-  if (p < N)
-    for (int64_t r = r0 + w; r < r1; r += 8) s += (double)P[r * N + p] * wr[r];
-  red[w][lane] = s;
-  __syncthreads();
-  if (w == 0 && p < N) {
-    double t = 0;
-    for (int k = 0; k < 8; ++k) t += red[k][lane];
-    part[(int64_t)blockIdx.y * N + p] = t;
-  }
-}
-
 __global__ void scaling_finish_kernel(const double* num, const double* part, int64_t nparts,
                                       int64_t N, float* scaling) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -920,12 +1085,31 @@ cudaError_t launch_ll_fp32(const LLArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_softmax_from_f64(const double* L, float* P, int64_t R, int64_t N,
-                                    double* plogp_part, int* nparts, double* lse,
-                                    cudaStream_t st) {
-  const int64_t nb = (N + 31) / 32;
-  if (nparts) *nparts = (int)nb;
-  softmax64_kernel<<<(unsigned)nb, kBlock, 0, st>>>(L, P, R, N, plogp_part, lse);
+int64_t resp_f32_blocks(int64_t N) { return (N + 255) / 256; }
+
+// Rows per block of the stats sweep: at least 64 (eight per warp in flight),
+// more where the patterns alone fill the GPU several times.
+int64_t resp_f32_chunk(int64_t R, int64_t N) {
+  const int64_t cols = (N + 31) / 32, want = 8 * 148;  // blocks
+  int64_t parts = (want + cols - 1) / cols;
+  const int64_t most = (R + 63) / 64;
+  if (parts > most) parts = most;
+  int64_t chunk = (R + parts - 1) / parts;
+  if (chunk > 512) chunk = 512;  // the partials then also hold ceil(R / 128) doubles per pattern
+  return (chunk + 63) / 64 * 64;
+}
+
+cudaError_t launch_resp_f32(const RespF32Args& a, cudaStream_t st) {
+  const int64_t cols = (a.N + 31) / 32, nb = resp_f32_blocks(a.N);
+  const unsigned gs = (unsigned)(cols * a.nparts);
+  const unsigned gp = (unsigned)(nb * ((a.R + kRespRows - 1) / kRespRows));
+  if (a.poisson)
+    resp_stats_kernel<true><<<gs, 256, 0, st>>>(a);
+  else
+    resp_stats_kernel<false><<<gs, 256, 0, st>>>(a);
+  resp_combine_kernel<<<(unsigned)cols, 256, 0, st>>>(a);
+  resp_kernel<<<gp, 256, 0, st>>>(a);
+  resp_rows_kernel<<<(unsigned)((a.R + 255) / 256), 256, 0, st>>>(a, nb);
   return cudaGetLastError();
 }
 
@@ -950,16 +1134,6 @@ cudaError_t launch_scaling_cross(const CrossArgs& a, cudaStream_t st) {
   OpCross op;
   op.p = a;
   tile_kernel<<<grid, kBlock, 0, st>>>(op);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_scaling_rowweighted(const float* P, const double* w, int64_t R, int64_t N,
-                                       double* den_part, int64_t* nparts, cudaStream_t st) {
-  const int64_t rchunk = 1024;
-  const int64_t nc = (R + rchunk - 1) / rchunk;
-  *nparts = nc;
-  dim3 grid((unsigned)((N + 31) / 32), (unsigned)nc);
-  rowweighted_kernel<<<grid, kBlock, 0, st>>>(P, w, R, N, rchunk, den_part);
   return cudaGetLastError();
 }
 
@@ -1039,22 +1213,6 @@ cudaError_t launch_model_max(const float* model, int64_t M, double* scratch, dou
 cudaError_t launch_fill(float* x, int64_t n, float v, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   fill_kernel<<<grid_for(n), kBlock, 0, st>>>(x, n, v);
-  return cudaGetLastError();
-}
-
-__global__ void count_invalid_kernel(const float* x, int64_t n, int* bad) {
-  int nb = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const float v = x[i];
-    if (!(v >= 0.0f && v <= FLT_MAX)) nb++;  // negative, NaN or infinite
-  }
-  if (nb) atomicAdd(bad, nb);
-}
-
-cudaError_t launch_count_invalid(const float* x, int64_t n, int* bad, cudaStream_t st) {
-  if (n <= 0) return cudaSuccess;
-  count_invalid_kernel<<<grid_for(n), kBlock, 0, st>>>(x, n, bad);
   return cudaGetLastError();
 }
 

@@ -1,0 +1,509 @@
+// FP32 contractions of the context API on the tensor cores, exact by
+// construction: out[n][m] = sum_k A[m][k] X[n][k] with A small integers (photon
+// counts) and X FP32 (slices, log slices, responsibilities).
+//
+// Each row of X becomes a fixed-point integer per element, 30 bits and sign
+// relative to the row's largest magnitude (a power-of-two unit, so every
+// element within 2^-7 of it keeps all its FP32 bits), cut into four balanced
+// base-256 digits; the counts are signed bytes (0 .. 127, or base-128 digits
+// in two passes).  tcgen05.mma kind::i8 multiplies the bytes and accumulates
+// in 32-bit integers, one TMEM accumulator per digit, and the epilogue
+// recombines the four sums as one 64-bit integer: no rounding happens between
+// the quantisation and the final conversion to FP64.  The quantisation error
+// (2^-31 of the row maximum per element) is below the rounding of the FP32
+// partial sums it replaces.
+//
+// What bounds it: the tensor pipe; four byte digits cost the MMA time of two
+// FP16 operand halves.  Measured (10,000 patterns x 25,680 rotations x 4,044
+// pixels): 3.2 ms, 646 TFLOP/s of the contraction, where the register-tiled
+// CUDA-core form, held by its shared-memory loads and FP64 folds, takes 92 to
+// 255 ms; 2,000 x 25,680 x 16,272: 2.4 against 92 ms.  SM pairs (cta_group::2) compute 256 x 128 tiles: 128 columns,
+// since the four digit accumulators fill the 512 TMEM columns; TMEM then has
+// no second buffer, so sixteen epilogue warps first drain the accumulators
+// into registers (32 columns each, recombined to 64 bits as they come) and
+// release them, and convert and store behind the next tile's MMAs.
+#include <algorithm>
+#include <cfloat>
+#include <cstdint>
+
+#include "i8.cuh"
+#include "tc_ptx.cuh"
+
+namespace emc {
+namespace {
+
+constexpr int kTileM = 256, kTileN = 128;  // of an SM pair
+constexpr int kStepK = 128;                // bytes per shared-memory row and K-step
+constexpr int kStages = 4;
+constexpr int kDigits = kI8Digits;
+constexpr int kEpiWarps = 16;
+constexpr int kEpiThreads = 32 * kEpiWarps;
+constexpr int kWarpCols = kTileN / (kEpiWarps / 4);  // columns per epilogue warp
+constexpr uint32_t kABytes = 128 * kStepK;               // this CTA's 128 rows of A
+constexpr uint32_t kBBytes = (kTileN / 2) * kStepK;      // its half of one digit plane
+constexpr uint32_t kStageBytes = kABytes + kDigits * kBBytes;
+// kind::i8, D = S32, A = B = S8 (both K-major), N = 128, M = 256 over the pair
+constexpr uint32_t kIdescI8 = (2u << 4) | (1u << 7) | (1u << 10) |
+                              ((uint32_t)(kTileN >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+
+__device__ __forceinline__ void mma_i8_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t accum) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(kIdescI8), "r"(accum)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&v)[8]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7])
+      : "r"(taddr));
+}
+
+// Column constants of a tile in shared memory (two tiles' worth: the stores
+// of one tile run while the next one's constants arrive).
+struct ColConst {
+  double unit;  // value of one unit of the column's integer sum
+  double c;     // per-column term of the epilogue
+};
+
+// LL[n][m], n = rotation, m = pattern:
+//   poisson   C - phi sum W            gaussian  (2 C / phi - sum S^2 - sum K^2 / phi^2) inv
+struct EpiLL {
+  I8LLArgs a;
+  double c1, c0;
+  __device__ void column(int64_t n, ColConst& k) const {
+    const bool ok = n < a.R;
+    k.unit = ok ? (double)a.unit[n] * a.mult : 0.0;
+    k.c = ok ? (a.poisson ? a.rowstat[n] : a.rowstat[n] * a.gauss_inv) : 0.0;
+  }
+  __device__ void row(int64_t m) {
+    c1 = c0 = 0.0;
+    if (m >= a.N) return;
+    const double phi = a.scaling[m];
+    if (a.poisson) {
+      c1 = phi;
+    } else {
+      c1 = 2.0 * a.gauss_inv / phi;
+      c0 = -a.patstat[m] / (phi * phi) * a.gauss_inv;
+    }
+  }
+  __device__ void store(int64_t m, int64_t n, long long v, const ColConst& k) const {
+    if (m >= a.N || n >= a.R) return;
+    double* o = a.LL + n * a.N + m;
+    double x = (double)v * k.unit;
+    if (a.pass == I8_HIGH) {  // the base-128 digit of the counts: the bare sum
+      *o = x;
+      return;
+    }
+    if (a.pass == I8_LOW) x += *o;
+    *o = a.poisson ? fma(-c1, k.c, x) : fma(x, c1, c0 - k.c);
+  }
+};
+
+// U[n][m] = sum / T_n, n = rotation, m = active pixel (emc_atomic.cu:105-111)
+struct EpiU {
+  I8UArgs a;
+  __device__ void column(int64_t n, ColConst& k) const {
+    const bool ok = n < a.R;
+    const float T = ok ? a.T[n] : 1.0f;
+    k.unit = ok ? (double)a.unit[n] * a.mult / (T > 1e-30f ? (double)T : 1.0) : 0.0;
+    k.c = 0.0;
+  }
+  __device__ void row(int64_t) {}
+  __device__ void store(int64_t m, int64_t n, long long v, const ColConst& k) const {
+    if (m >= a.npa || n >= a.R) return;
+    float* o = a.U + n * a.npa + m;
+    double x = (double)v * k.unit;
+    if (a.pass == I8_LOW) x += (double)*o;
+    *o = (float)x;
+  }
+};
+
+template <class Epi>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + kEpiThreads, 1)
+    i8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                   const int64_t m_tiles, const int64_t n_tiles, const int64_t k_blocks,
+                   const int64_t plane_rows, const int raster, const Epi epi, TcStatus* status) {
+  extern __shared__ uint8_t dyn_smem[];
+  __shared__ __align__(8) uint64_t full_bar[kStages], empty_bar[kStages];
+  __shared__ __align__(8) uint64_t tfull_bar, tempty_bar, drain_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag, epi_abort;
+  __shared__ ColConst cols[2][kTileN];
+
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn_smem) + 1023) &
+                                             ~uintptr_t(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  const bool leader = rank == 0;
+  Ctl ctl{&abort_flag, status};
+  auto abort_pair = [&]() {  // the peer's waits end at their next check too
+    abort_flag = 1;
+    const uint32_t pa = peer_addr(smem_u32(&abort_flag), rank ^ 1u);
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(pa), "r"(1) : "memory");
+  };
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(smem_u32(&full_bar[s]), 1);
+      mbar_init(smem_u32(&empty_bar[s]), 1);
+    }
+    mbar_init(smem_u32(&tfull_bar), 1);
+    mbar_init(smem_u32(&tempty_bar), 2);  // one arrival per CTA's epilogue
+    mbar_init(smem_u32(&drain_bar), 1);
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&tmem_slot)),
+                 "r"(kDigits * kTileN)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+  const int64_t num_tiles = m_tiles * n_tiles;
+  const int64_t cid = blockIdx.x >> 1, ncl = gridDim.x >> 1;
+
+  // m fastest in bands of `raster` n tiles (as tc_pair_kernel)
+  auto tile_mn = [&](int64_t t, int64_t& m, int64_t& n) {
+    const int64_t span = (int64_t)raster * m_tiles, band = t / span, o0 = band * raster;
+    const int64_t g = n_tiles - o0 < raster ? n_tiles - o0 : raster;
+    const int64_t w = t - band * span;
+    n = o0 + w % g;
+    m = w / g;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // ------------------------------------------------ TMA producer (both CTAs)
+      int s = 0;
+      uint32_t ph = 0;
+      int64_t issued = 0;
+      bool ok = true;
+      for (int64_t t = cid; t < num_tiles && ok; t += ncl) {
+        int64_t mt, nt;
+        tile_mn(t, mt, nt);
+        const int ar = (int)(mt * kTileM + rank * 128);
+        const int br = (int)(nt * kTileN + rank * (kTileN / 2));
+        for (int64_t kb = 0; kb < k_blocks; ++kb) {
+          if (!bounded_wait(smem_u32(&empty_bar[s]), ph ^ 1, ctl, 11)) {
+            ok = false;
+            break;
+          }
+          const uint32_t fb = smem_u32(&full_bar[s]);
+          if (leader) mbar_expect_tx(fb, 2 * kStageBytes);  // both CTAs' bytes
+          const uint32_t fb_leader = peer_addr(fb, 0);
+          const uint32_t base = smem_u32(smem + (size_t)s * kStageBytes);
+          const int kc = (int)(kb * kStepK);
+          tma_load_2d_pair(base, &tmA, kc, ar, fb_leader);
+#pragma unroll
+          for (int q = 0; q < kDigits; ++q)
+            tma_load_2d_pair(base + kABytes + q * kBBytes, &tmB, kc, br + (int)(q * plane_rows),
+                             fb_leader);
+          ++issued;
+          if (++s == kStages) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+      }
+      if (!ok) {
+        abort_pair();
+        if (leader) {
+          // the last min(issued, stages) stages must land (both CTAs' bytes
+          // complete on these barriers) before the pair exits
+          const int64_t n = issued < kStages ? issued : kStages;
+          int ss = s;
+          uint32_t pp = ph;
+          for (int64_t i = 0; i < n; ++i) {
+            if (--ss < 0) {
+              ss = kStages - 1;
+              pp ^= 1;
+            }
+            const uint64_t t0 = globaltimer();
+            while (!mbar_test(smem_u32(&full_bar[ss]), pp) && globaltimer() - t0 < kWaitLimitNs) {
+            }
+          }
+        } else {
+          // the peer cannot observe its loads; give them time to land
+          const uint64_t t0 = globaltimer();
+          while (globaltimer() - t0 < 2000000ull) {
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && leader) {
+      // ------------------------------------------------ MMA issuer (leader)
+      int s = 0;
+      uint32_t ph = 0, i = 0;
+      bool ok = true;
+      for (int64_t t = cid; t < num_tiles && ok; t += ncl, ++i) {
+        if (!bounded_wait(smem_u32(&tempty_bar), (i & 1) ^ 1, ctl, 12)) {
+          abort_pair();
+          break;
+        }
+        tc_fence_after();
+        for (int64_t kb = 0; kb < k_blocks; ++kb) {
+          if (!bounded_wait(smem_u32(&full_bar[s]), ph, ctl, 13)) {
+            ok = false;
+            abort_pair();
+            break;
+          }
+          tc_fence_after();
+          const uint32_t base = smem_u32(smem + (size_t)s * kStageBytes);
+#pragma unroll
+          for (int k = 0; k < kStepK / 32; ++k)
+#pragma unroll
+            for (int q = 0; q < kDigits; ++q)
+              mma_i8_pair(tmem + q * kTileN, sdesc<64>(base + k * 32),
+                          sdesc<64>(base + kABytes + q * kBBytes + k * 32), (kb | k) != 0);
+          const uint32_t eb = smem_u32(&empty_bar[s]);
+          mma_commit_pair(peer_addr(eb, 0));
+          mma_commit_pair(peer_addr(eb, 1));
+          if (++s == kStages) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+        if (ok) {
+          const uint32_t tb = smem_u32(&tfull_bar);
+          mma_commit_pair(peer_addr(tb, 0));
+          mma_commit_pair(peer_addr(tb, 1));
+        }
+      }
+      mma_commit_pair(peer_addr(smem_u32(&drain_bar), 0));
+      const uint64_t t0 = globaltimer();
+      while (!mbar_test(smem_u32(&drain_bar), 0) && globaltimer() - t0 < kWaitLimitNs) {
+      }
+    }
+  } else {
+    // -------------------------------------------------- epilogue warps (both CTAs)
+    const int quarter = warp & 3;  // TMEM lane quarter
+    const int ep_tid = threadIdx.x - 64;
+    const int col0 = ((warp - 2) >> 2) * kWarpCols;
+    Epi e = epi;
+    uint32_t i = 0;
+    const uint32_t tempty_leader = peer_addr(smem_u32(&tempty_bar), 0);
+    for (int64_t t = cid; t < num_tiles; t += ncl, ++i) {
+      int64_t mt, nt;
+      tile_mn(t, mt, nt);
+      ColConst* cc = cols[i & 1];
+      if (ep_tid < kTileN) e.column(nt * kTileN + ep_tid, cc[ep_tid]);
+      const int64_t m = mt * kTileM + rank * 128 + quarter * 32 + lane;
+      e.row(m);
+      bounded_wait(smem_u32(&tfull_bar), i & 1, ctl, 14);
+      // the epilogue warps leave together
+      epi_bar(kEpiThreads);
+      if (ep_tid == 0) epi_abort = abort_flag;
+      epi_bar(kEpiThreads);
+      if (epi_abort) break;
+      tc_fence_after();
+      const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)col0;
+      long long sum[kWarpCols];
+#pragma unroll
+      for (int c = 0; c < kWarpCols; c += 8) {
+        int d[kDigits][8];
+#pragma unroll
+        for (int q = 0; q < kDigits; ++q) tmem_ld8(taddr + q * kTileN + c, d[q]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          sum[c + k] = (long long)d[0][k] + (long long)d[1][k] * 256 + (long long)d[2][k] * 65536 +
+                       (long long)d[3][k] * 16777216;
+      }
+      tc_fence_before();
+      epi_bar(kEpiThreads);  // the whole accumulator of this CTA has been read
+      if (ep_tid == 0) mbar_arrive_cluster(tempty_leader);
+      const int64_t n0 = nt * kTileN + col0;
+#pragma unroll
+      for (int c = 0; c < kWarpCols; ++c) e.store(m, n0 + c, sum[c], cc[col0 + c]);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();  // neither CTA leaves while the pair's MMAs or loads may touch it
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(kDigits * kTileN)
+                 : "memory");
+  }
+}
+
+template <class Epi>
+cudaError_t run_i8(const CUtensorMap& tmA, const CUtensorMap& tmB, int64_t m, int64_t n, int64_t k,
+                   const Epi& epi, TcStatus* status, int num_sms, cudaStream_t st) {
+  const size_t dyn = (size_t)kStages * kStageBytes + 1024;
+  auto kern = i8_pair_kernel<Epi>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+  if (e != cudaSuccess) return e;
+  const int64_t mt = (m + kTileM - 1) / kTileM, nt = (n + kTileN - 1) / kTileN;
+  const int64_t tiles = mt * nt, pairs = num_sms / 2;
+  if (tiles == 0 || pairs == 0) return cudaErrorInvalidValue;
+  kern<<<2 * (unsigned)(tiles < pairs ? tiles : pairs), 64 + kEpiThreads, dyn, st>>>(
+      tmA, tmB, mt, nt, (k + kStepK - 1) / kStepK, n, 1, epi, status);
+  return cudaGetLastError();
+}
+
+// ------------------------------------------------------------- operands --
+
+// Balanced base-256 digits of q (|q| <= 127 (2^24 + 2^16 + 2^8 + 1)), lowest
+// first, one byte each.
+__device__ __forceinline__ uint32_t digits_of(int q) {
+  uint32_t out = 0;
+#pragma unroll
+  for (int s = 0; s < kDigits; ++s) {
+    const int d = (int)(signed char)(q & 0xff);
+    out |= (uint32_t)(d & 0xff) << (8 * s);
+    q = (q - d) >> 8;
+  }
+  return out;
+}
+
+// One block per row of X [R][cols] (div: X = P / phi of the column): the
+// digit planes D [4][R][ld] and the row's unit 2^-k.  2^k puts the row's
+// largest magnitude below 2^31 and the top digit within a byte.
+__global__ void __launch_bounds__(256) quant_rows_kernel(const float* X, const float* div,
+                                                         const float* rowmax, int64_t R,
+                                                         int64_t cols, int64_t ld, int8_t* D,
+                                                         float* unit) {
+  const int64_t r = blockIdx.x;
+  const float mx = rowmax[r];
+  const int ex = (int)((__float_as_uint(mx) >> 23) & 0xff) - 127;
+  float up = 0.0f, one = 0.0f;  // a row of zeros (or denormals): all digits 0
+  if (ex == 128) {
+    one = __int_as_float(0x7fffffff);  // an infinite or NaN element: the row's sums are NaN
+  } else if (ex > -127) {
+    int k = 30 - ex;
+    if (k > 126) k = 126;
+    if (ldexpf(mx, k) > 2130706432.0f) --k;
+    up = ldexpf(1.0f, k);
+    one = ldexpf(1.0f, -k);
+  }
+  if (threadIdx.x == 0) unit[r] = one;
+  const float* x = X + r * cols;
+  for (int64_t j0 = 4 * (int64_t)threadIdx.x; j0 < cols; j0 += 4 * blockDim.x) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int64_t j = j0 + i;
+      float v = j < cols ? x[j] : 0.0f;
+      if (div && j < cols) v /= div[j];
+      w[i] = digits_of(__float2int_rn(v * up));
+    }
+#pragma unroll
+    for (int s = 0; s < kDigits; ++s) {
+      uint32_t b = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) b |= ((w[i] >> (8 * s)) & 0xffu) << (8 * i);
+      *reinterpret_cast<uint32_t*>(D + ((int64_t)s * R + r) * ld + j0) = b;
+    }
+  }
+}
+
+// Counts K [N][npa] as bytes by pattern (K8 [planes][N][ldK]) and by pixel
+// (Kt8 [planes][npa][ldT]), base-128 digits when planes == 2.
+__global__ void pack_counts_i8_kernel(const float* K, int64_t N, int64_t npa, int planes,
+                                      int64_t ldK, int64_t ldT, int8_t* K8, int8_t* Kt8) {
+  __shared__ int tile[32][33];
+  const int64_t jb = (npa + 31) / 32;
+  const int64_t j0 = blockIdx.x % jb * 32, p0 = blockIdx.x / jb * 32;
+  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
+  for (int i = ty; i < 32; i += 8) {
+    const int64_t p = p0 + i, j = j0 + tx;
+    const int k = (p < N && j < npa) ? (int)K[p * npa + j] : 0;
+    tile[i][tx] = k;
+    if (p < N && j < npa)
+      for (int s = 0; s < planes; ++s)
+        K8[((int64_t)s * N + p) * ldK + j] = (int8_t)((k >> (7 * s)) & 127);
+  }
+  __syncthreads();
+  for (int i = ty; i < 32; i += 8) {
+    const int64_t j = j0 + i, p = p0 + tx;
+    if (p < N && j < npa)
+      for (int s = 0; s < planes; ++s)
+        Kt8[((int64_t)s * npa + j) * ldT + p] = (int8_t)((tile[tx][i] >> (7 * s)) & 127);
+  }
+}
+
+// out[0] = bits of the largest entry, out[1] += entries that are not integers
+// in [0, limit], out[2] += entries that are negative, NaN or infinite.
+__global__ void count_range_kernel(const float* x, int64_t n, float limit, unsigned int* out) {
+  unsigned int mx = 0, odd = 0, bad = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const float v = x[i];
+    if (!(v >= 0.0f && v <= FLT_MAX)) {
+      ++bad;
+      continue;
+    }
+    if (!(v <= limit && v == floorf(v))) ++odd;
+    mx = max(mx, __float_as_uint(fabsf(v)));
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  odd = __reduce_add_sync(0xffffffffu, odd);
+  bad = __reduce_add_sync(0xffffffffu, bad);
+  if ((threadIdx.x & 31) == 0) {
+    if (mx) atomicMax(out, mx);
+    if (odd) atomicAdd(out + 1, odd);
+    if (bad) atomicAdd(out + 2, bad);
+  }
+}
+
+}  // namespace
+
+bool i8_encode(CUtensorMap* tm, const void* base, int64_t inner, int64_t rows, int64_t ld,
+               bool counts) {
+  return tc_encode_2d_bytes(tm, base, (uint64_t)inner, (uint64_t)rows, (uint64_t)ld,
+                            counts ? 128 : kTileN / 2, kStepK);
+}
+
+cudaError_t launch_i8_loglik(const CUtensorMap& tmK, const CUtensorMap& tmX, int64_t npa,
+                             const I8LLArgs& a, TcStatus* status, int num_sms, cudaStream_t st) {
+  EpiLL e;
+  e.a = a;
+  return run_i8(tmK, tmX, a.N, a.R, npa, e, status, num_sms, st);
+}
+
+cudaError_t launch_i8_slices(const CUtensorMap& tmKt, const CUtensorMap& tmX, int64_t N,
+                             const I8UArgs& a, TcStatus* status, int num_sms, cudaStream_t st) {
+  EpiU e;
+  e.a = a;
+  return run_i8(tmKt, tmX, a.npa, a.R, N, e, status, num_sms, st);
+}
+
+cudaError_t launch_quant_rows(const float* X, const float* div, const float* rowmax, int64_t R,
+                              int64_t cols, int64_t ld, int8_t* D, float* unit, cudaStream_t st) {
+  if (R <= 0) return cudaSuccess;
+  if (ld % 16 != 0 || ld < cols) return cudaErrorInvalidValue;
+  quant_rows_kernel<<<(unsigned)R, 256, 0, st>>>(X, div, rowmax, R, cols, ld, D, unit);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pack_counts_i8(const float* K, int64_t N, int64_t npa, int planes, int64_t ldK,
+                                  int64_t ldT, int8_t* K8, int8_t* Kt8, cudaStream_t st) {
+  const int64_t grid = ((npa + 31) / 32) * ((N + 31) / 32);
+  pack_counts_i8_kernel<<<(unsigned)grid, dim3(32, 8), 0, st>>>(K, N, npa, planes, ldK, ldT, K8, Kt8);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_count_range(const float* x, int64_t n, float limit, unsigned int* out,
+                               cudaStream_t st) {
+  const cudaError_t e = cudaMemsetAsync(out, 0, 3 * sizeof(unsigned int), st);
+  if (e != cudaSuccess || n <= 0) return e;
+  count_range_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 1184), 256, 0, st>>>(x, n,
+                                                                                        limit, out);
+  return cudaGetLastError();
+}
+
+}  // namespace emc
