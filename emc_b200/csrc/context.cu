@@ -1132,6 +1132,20 @@ static emc_status sort_scratch(emc_context* c, int64_t n) {
   return EMC_OK;
 }
 
+// The number of list entries up to which the compress from lists is faster
+// than the dense contraction.  An entry costs its pattern's photons as
+// shared-memory additions (measured 6.4e11 a second: 2.05e8 entries of 470
+// photons in 155 ms at 80^3 gaussian, whose posteriors stay broad); the dense
+// form costs the contraction (measured 6.5e14 flop a second with its
+// insertion) and the write of its operand (8 bytes per pair at 5 TB/s): 5 ms
+// there, so about 7e6 entries.
+static int64_t list_worth(const emc_context* c) {
+  const double pairs = (double)c->R * (double)c->N;
+  const double dense = 2.0 * pairs * (double)c->npa / 6.5e14 + 8.0 * pairs / 5e12;
+  const double photons = (double)c->csr.nnz / (double)c->N;
+  return (int64_t)std::min(dense * 6.4e11 / std::max(photons, 1.0), 9e15);
+}
+
 static emc_status mixed_resp_pass(emc_context* c, bool allow_lists = true) {
   const int64_t N = c->N;
   RespArgs a = resp_args(c);
@@ -1141,6 +1155,8 @@ static emc_status mixed_resp_pass(emc_context* c, bool allow_lists = true) {
     // entries P >= kListMinP are compacted during the row-sum sweep, the host
     // reads their count (one wait), a counting sort orders them by rotation
     TRY(list_buffers(c));
+    if (!c->csr.valid) TRY(build_rows(c, c->d_K, N, c->npa, c->csr, false));
+    const int64_t worth = std::max<int64_t>(list_worth(c), 64 * N);
     TRY(compact_capacity(c, std::max<int64_t>(64 * N, (int64_t)1 << 20)));
     CK(c, cudaMemsetAsync(c->d_lcount, 0, sizeof(unsigned long long), c->st));
     a.list_count = c->d_lcount;
@@ -1155,7 +1171,7 @@ static emc_status mixed_resp_pass(emc_context* c, bool allow_lists = true) {
                           c->st));
     CK(c, cudaStreamSynchronize(c->st));
     c->list_nnz = (int64_t)*hn;
-    if (c->list_nnz <= c->lcomp_cap) {
+    if (c->list_nnz <= std::min(worth, c->lcomp_cap)) {
       TRY(grow(c, &c->d_lpat, c->lcap, c->list_nnz + 1));
       int64_t cap = c->lcap_x;
       TRY(grow(c, &c->d_lx, cap, c->list_nnz + 1));
@@ -1178,9 +1194,9 @@ static emc_status mixed_resp_pass(emc_context* c, bool allow_lists = true) {
       c->launches += 6;  // combine, row sums, T, count, scan, fill
     } else {
       // more entries than the compaction holds: the dense operand this time,
-      // room for them next time
+      // room for them next time if they are worth it
       CK(c, launch_resp_write(a, c->st));
-      TRY(compact_capacity(c, c->list_nnz));
+      if (c->list_nnz <= worth) TRY(compact_capacity(c, c->list_nnz));
       c->launches += 3;
     }
   } else {
@@ -3245,15 +3261,16 @@ emc_status emc_batch_synchronize(emc_batch* b) {
   BCK(b, cudaStreamSynchronize(b->st));
   for (emc_context* c : b->ctx) BTRY(b, c, check_status(c));
   // a dataset whose compacted entries passed the capacity ran the dense
-  // compress (correct, slower): room for them from the next iteration on,
-  // and a recorded graph is recorded again with the new buffers
+  // compress: where lists of that length would be faster, room for them from
+  // the next iteration on, and a recorded graph is recorded again with the
+  // new buffers
   bool grew = false;
   for (size_t i = 0; i < b->ctx.size(); ++i) {
     emc_context* c = b->ctx[i];
     if (!b->lists[i]) continue;
     unsigned long long n = 0;
     BCK(b, cudaMemcpy(&n, c->d_lcount, sizeof(n), cudaMemcpyDeviceToHost));
-    if ((int64_t)n > c->lcomp_cap) {
+    if ((int64_t)n > c->lcomp_cap && (int64_t)n <= std::max(list_worth(c), 64 * c->N)) {
       BTRY(b, c, batch_lists_ready(c, (int64_t)n));
       grew = true;
     }
