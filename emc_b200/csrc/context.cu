@@ -166,6 +166,7 @@ struct emc_context {
   int32_t* d_rank = nullptr;  // mixed: ascending position of every compact pixel
   int32_t* d_ins = nullptr;
   float *d_cx = nullptr, *d_cy = nullptr, *d_cz = nullptr;
+  float4* d_pc = nullptr;  // the same packed: (cx, cy, cz, insert flag as 1 or 0)
   // rotations
   float *d_quat = nullptr, *d_rotw = nullptr;
   // patterns
@@ -755,6 +756,11 @@ emc_status emc_set_geometry(emc_context* c, const float* x, const float* y, cons
   CK(c, cudaMemcpyAsync(c->d_cx, cx.data(), 4 * c->npa, cudaMemcpyHostToDevice, c->st));
   CK(c, cudaMemcpyAsync(c->d_cy, cy.data(), 4 * c->npa, cudaMemcpyHostToDevice, c->st));
   CK(c, cudaMemcpyAsync(c->d_cz, cz.data(), 4 * c->npa, cudaMemcpyHostToDevice, c->st));
+  std::vector<float4> pc(c->npa);
+  for (int64_t j = 0; j < c->npa; ++j)
+    pc[j] = make_float4(cx[j], cy[j], cz[j], ins[j] == 1 ? 1.0f : 0.0f);
+  TRY(c->alloc(&c->d_pc, c->npa));
+  CK(c, cudaMemcpyAsync(c->d_pc, pc.data(), sizeof(float4) * c->npa, cudaMemcpyHostToDevice, c->st));
   if (!rank.empty()) {
     TRY(c->alloc(&c->d_rank, c->npa));
     CK(c, cudaMemcpyAsync(c->d_rank, rank.data(), 4 * c->npa, cudaMemcpyHostToDevice, c->st));
@@ -1049,6 +1055,7 @@ static CmpEpiArgs cmp_args(emc_context* c) {
   e.cy = c->d_cy;
   e.cz = c->d_cz;
   e.ins = c->d_ins;
+  e.pc = c->d_pc;
   e.acc = c->d_acc;
   return e;
 }

@@ -1798,14 +1798,24 @@ __global__ void sorted_place_kernel(const int2* rp, const float* Pv, int64_t n, 
 // pixels is accumulated in shared memory from the listed patterns' photon
 // lists (x times each non-zero count), then inserted exactly as the dense
 // contraction's epilogue does (EpiCmp).
-__global__ void __launch_bounds__(256) list_compress_kernel(const ListCmpArgs a) {
+//
+// The insertion bounds it (one reduction per pixel; the slice's shared memory
+// limits the blocks on an SM), and waiting for the pixel coordinates used to
+// bound the insertion: four loads per pixel, one pixel at a time, from L2.
+// They are one 16-byte load now, four pixels in flight per thread, in blocks
+// of 512 threads where the slice leaves room for few blocks.
+constexpr int kInsertUnroll = 4;
+template <int THREADS, int INTERP>
+__global__ void __launch_bounds__(THREADS, THREADS == 512 ? 3 : 6)
+    list_compress_kernel(const ListCmpArgs a) {
   extern __shared__ float Us[];  // [npa]
   const int64_t r = blockIdx.x;
   const CmpEpiArgs& e = a.e;
   if (a.gate_count && *a.gate_count > (unsigned long long)a.gate_cap) return;
   const float T = e.T[r];
   if (!((e.Tskip ? e.Tskip[r] : T) > 1e-10f) || !(T > 0.0f)) return;  // emc_atomic.cu:128
-  for (int64_t j = threadIdx.x; j < e.npa; j += blockDim.x) Us[j] = 0.0f;
+  const int npa = (int)e.npa;
+  for (int j = threadIdx.x; j < npa; j += THREADS) Us[j] = 0.0f;
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (a.ordered) {
@@ -1820,7 +1830,7 @@ __global__ void __launch_bounds__(256) list_compress_kernel(const ListCmpArgs a)
         __syncwarp();
       }
   } else {
-    for (int64_t q = a.rowoff[r] + w; q < a.rowoff[r + 1]; q += blockDim.x >> 5) {
+    for (int64_t q = a.rowoff[r] + w; q < a.rowoff[r + 1]; q += THREADS / 32) {
       const int64_t p = a.pat[q];
       const float x = a.xv[q];
       for (int64_t t = a.kptr[p] + lane; t < a.kptr[p + 1]; t += 32)
@@ -1831,21 +1841,30 @@ __global__ void __launch_bounds__(256) list_compress_kernel(const ListCmpArgs a)
   const float wT = e.rotw[r] * T;
   float m[9];
   emc_voxel::rotation_matrix(e.quat + 4 * r, m);
-  for (int64_t j = threadIdx.x; j < e.npa; j += blockDim.x) {
-    if (e.ins[j] != 1) continue;
-    float u[3];
-    emc_voxel::position(m, e.side, e.cx[j], e.cy[j], e.cz[j], u);
-    const float val = Us[j] * wT;
-    if (e.interp == 0) {
-      int64_t vox;
-      if (emc_voxel::nearest(u, e.side, 0, &vox)) insert_add(e, vox, val, wT);
-    } else {
+  for (int j0 = threadIdx.x; j0 < npa; j0 += kInsertUnroll * THREADS) {
+    float4 q[kInsertUnroll];
 #pragma unroll
-      for (int cc = 0; cc < 8; ++cc) {
-        int64_t vox;
-        float wc;
-        if (!emc_voxel::trilinear_corner(u, e.side, cc, &vox, &wc) || wc == 0.0f) continue;
-        insert_add(e, vox, wc * val, wc * wT);
+    for (int k = 0; k < kInsertUnroll; ++k) {
+      const int j = j0 + k * THREADS;
+      q[k] = j < npa ? __ldg(e.pc + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < kInsertUnroll; ++k) {
+      if (q[k].w == 0.0f) continue;
+      float u[3];
+      emc_voxel::position(m, e.side, q[k].x, q[k].y, q[k].z, u);
+      const float val = Us[j0 + k * THREADS] * wT;
+      if constexpr (INTERP == 0) {
+        int vox;
+        if (emc_voxel::nearest32(u, e.side, 0, &vox)) insert_add(e, vox, val, wT);
+      } else {
+#pragma unroll
+        for (int cc = 0; cc < 8; ++cc) {
+          int64_t vox;
+          float wc;
+          if (!emc_voxel::trilinear_corner(u, e.side, cc, &vox, &wc) || wc == 0.0f) continue;
+          insert_add(e, vox, wc * val, wc * wT);
+        }
       }
     }
   }
@@ -2306,13 +2325,22 @@ cudaError_t launch_cells_out(const double* acc, int64_t count, int take_log, flo
   return cudaGetLastError();
 }
 
+template <int THREADS, int INTERP>
+static cudaError_t run_list_compress(const ListCmpArgs& a, size_t smem, cudaStream_t st) {
+  auto kern = list_compress_kernel<THREADS, INTERP>;
+  cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  if (a.e.R > 0) kern<<<(unsigned)a.e.R, THREADS, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_list_compress(const ListCmpArgs& a, cudaStream_t st) {
   const size_t smem = sizeof(float) * (size_t)a.e.npa;
-  cudaError_t e = cudaFuncSetAttribute(list_compress_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  if (a.e.R > 0) list_compress_kernel<<<(unsigned)a.e.R, 256, smem, st>>>(a);
-  return cudaGetLastError();
+  const bool wide = smem > (32u << 10);  // six blocks or fewer fit an SM
+  if (a.e.interp == 0)
+    return wide ? run_list_compress<512, 0>(a, smem, st) : run_list_compress<256, 0>(a, smem, st);
+  return wide ? run_list_compress<512, 1>(a, smem, st) : run_list_compress<256, 1>(a, smem, st);
 }
 
 cudaError_t launch_resp_export(const RespArgs& a, float* P, cudaStream_t st) {

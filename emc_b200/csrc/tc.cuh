@@ -80,6 +80,7 @@ struct CmpEpiArgs {
   const float* cy;
   const float* cz;
   const int32_t* ins;      // [npa] insert flag (mask == 1)
+  const float4* pc;        // [npa] (cx, cy, cz, ins as 1 or 0)
   float2* acc;             // [side^3] interleaved (model, weight) accumulators
   unsigned long long* acc64;  // or, when set, fixed-point limbs [side^3][8] (fixed.cuh)
   // optional: the launch returns at once unless *gate_count > gate_cap (the

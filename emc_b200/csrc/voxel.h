@@ -83,6 +83,15 @@ EMC_HD bool nearest(const float* u, int side, int lower, int64_t* v) {
   return true;
 }
 
+// The same with a 32-bit index (side <= 1024, so side^3 <= 2^30).
+EMC_HD bool nearest32(const float* u, int side, int lower, int* v) {
+  const int kx = (int)roundf(u[0]), ky = (int)roundf(u[1]), kz = (int)roundf(u[2]);
+  if (kx < lower || kx >= side || ky < lower || ky >= side || kz < lower || kz >= side)
+    return false;
+  *v = (kz * side + ky) * side + kx;
+  return true;
+}
+
 // Corner c (0..7, bit 0 = x, 1 = y, 2 = z) of the trilinear stencil: its voxel
 // and weight, false when it lies outside the grid.  Callers unroll over c, so
 // no stencil array is kept.
