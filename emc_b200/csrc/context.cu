@@ -228,6 +228,7 @@ struct emc_context {
   unsigned long long* d_cand_key = nullptr;
   float4* d_part = nullptr;
   float2* d_acc = nullptr;  // interleaved (model, weight) accumulators
+  float2* d_acc_odd = nullptr;  // trilinear: the shifted pairs (insert.cuh), behind d_acc
   double *d_lse = nullptr, *d_plogp = nullptr;
   float* d_Tpart = nullptr;
   CUtensorMap tmKh, tmKt, tmBhi, tmBlo, tmPhi, tmPlo;
@@ -624,6 +625,20 @@ static emc_status set_y_rows(emc_context* c, int64_t rows) {
   return EMC_OK;
 }
 
+// The insertion accumulators.  Trilinear insertion takes a second, shifted
+// array in the same allocation where it is a small part of the memory left
+// (without it the pairs at odd voxels are two reductions).
+static emc_status alloc_acc(emc_context* c) {
+  const int64_t odd = round_up(c->M, 2) + c->M + 2;
+  if (c->cfg.interp == EMC_INTERP_TRILINEAR &&
+      sizeof(float2) * (size_t)odd <= avail_bytes(c, 0) / 8) {
+    TRY(c->alloc(&c->d_acc, odd, true));
+    c->d_acc_odd = c->d_acc + round_up(c->M, 2);
+    return EMC_OK;
+  }
+  return c->alloc(&c->d_acc, c->M, true);
+}
+
 static emc_status alloc_work(emc_context* c) {
   // called once geometry is known (npa fixes every pixel dimension)
   const int64_t R = c->R, N = c->N, npa = c->npa;
@@ -663,7 +678,7 @@ static emc_status alloc_work(emc_context* c) {
   if (c->tune.compress_pair) c->tune.compress_raster = 2;
   c->Rpad = round_up(R, 256);
   c->nrt = c->Rpad / 256;
-  TRY(c->alloc(&c->d_acc, c->M, true));
+  TRY(alloc_acc(c));
   // the nearest expansion's voxel table (here rather than at the first
   // expansion, so an iteration can be captured into a graph before any ran)
   if (c->cfg.interp == EMC_INTERP_NEAREST) TRY(c->alloc(&c->d_vtab, c->M + 1));
@@ -1039,6 +1054,17 @@ static MaxEpiArgs max_args(emc_context* c) {
   return e;
 }
 
+// The accumulators' starting state, and their sum after the insertion.
+static emc_status clear_acc(emc_context* c) {
+  const int64_t n = c->d_acc_odd ? round_up(c->M, 2) + c->M + 2 : c->M;
+  return c->cuda(cudaMemsetAsync(c->d_acc, 0, sizeof(float2) * n, c->st), "clear accumulators");
+}
+static emc_status merge_acc(emc_context* c) {
+  if (!c->d_acc_odd) return EMC_OK;
+  c->launches += 1;
+  return c->cuda(launch_merge_odd(c->d_acc, c->d_acc_odd, c->M, c->st), "merge accumulators");
+}
+
 // Epilogue arguments of the mixed compress contraction (insertion).
 static CmpEpiArgs cmp_args(emc_context* c) {
   CmpEpiArgs e{};
@@ -1056,7 +1082,7 @@ static CmpEpiArgs cmp_args(emc_context* c) {
   e.cz = c->d_cz;
   e.ins = c->d_ins;
   e.pc = c->d_pc;
-  e.acc = c->d_acc;
+  e.ins_acc = InsertAcc{c->d_acc, c->det ? nullptr : c->d_acc_odd, c->det ? c->d_acc64 : nullptr};
   return e;
 }
 
@@ -1611,7 +1637,7 @@ emc_status emc_compress_insert(emc_context* c) {
     CK(c, cudaMemsetAsync(c->d_model, 0, sizeof(float) * c->M, c->st));
     CK(c, cudaMemsetAsync(c->d_weight, 0, sizeof(float) * c->M, c->st));
   } else {
-    CK(c, cudaMemsetAsync(c->d_acc, 0, sizeof(float2) * c->M, c->st));
+    TRY(clear_acc(c));
   }
   if (!c->mixed) {
     if (c->tune.compress_sparse) {
@@ -1655,7 +1681,6 @@ emc_status emc_compress_insert(emc_context* c) {
     c->launches += 1;
   } else {
     CmpEpiArgs e = cmp_args(c);
-    e.acc64 = c->det ? c->d_acc64 : nullptr;
     if (c->list_mode) {
       // responsibility lists x the counts' photon lists (built once per upload)
       if (!c->csr.valid) TRY(build_rows(c, c->d_K, c->N, c->npa, c->csr, false));
@@ -1677,6 +1702,7 @@ emc_status emc_compress_insert(emc_context* c) {
                                c->d_status, c->num_sms, c->st, c->tune.compress_raster));
     }
     c->launches += 1;
+    if (!c->det) TRY(merge_acc(c));
   }
   if (c->det) {
     // the exact sums as the FP32 accumulators the normalisation (and a
@@ -2418,7 +2444,7 @@ static emc_status run_proposed(emc_context* c, const ProposedPlan& pl, Select se
     TRY(c->alloc(&c->d_best, N));
     TRY(c->alloc(&c->d_bestp, N));
   }
-  if (!c->d_acc) TRY(c->alloc(&c->d_acc, c->M));
+  if (!c->d_acc) TRY(alloc_acc(c));
   if (pairs > c->pairs_cap || c->cand_m != m) {
     int64_t cap = c->pairs_cap;
     TRY(grow(c, &c->d_cand, cap, pairs));
@@ -2707,7 +2733,7 @@ static emc_status run_proposed(emc_context* c, const ProposedPlan& pl, Select se
                                    c->st));
       if (!c->csr.valid) TRY(build_rows(c, c->d_K, c->N, c->npa, c->csr, false));
       c->mark(3);
-      CK(c, cudaMemsetAsync(c->d_acc, 0, sizeof(float2) * c->M, c->st));
+      TRY(clear_acc(c));
       ListCmpArgs la{};
       la.rowoff = c->d_lrowoff;
       la.pat = c->d_lpat;
@@ -2718,11 +2744,12 @@ static emc_status run_proposed(emc_context* c, const ProposedPlan& pl, Select se
       la.e = cmp_args(c);
       la.e.Tskip = nullptr;  // the proposed iteration's own T_r
       CK(c, launch_list_compress(la, c->st));
+      TRY(merge_acc(c));
       launches = 7;  // row build, contraction, softmax, count + scan, fill, compress
     } else {
     CK(c, launch_p_split(g, c->d_cell, R, c->d_T, c->a_ld, c->d_Ahi, c->d_Alo, c->st));
     c->mark(3);
-    CK(c, cudaMemsetAsync(c->d_acc, 0, sizeof(float2) * c->M, c->st));
+    TRY(clear_acc(c));
     GCmpEpiArgs ce{};
     ce.tiles = c->d_gct;
     ce.mcnt = c->d_mcnt;
@@ -2746,7 +2773,7 @@ static emc_status run_proposed(emc_context* c, const ProposedPlan& pl, Select se
     CK(c, launch_group_maximize(g, (int64_t)mt.size(), c->st));
     c->mark(2);
     c->mark(3);
-    CK(c, cudaMemsetAsync(c->d_acc, 0, sizeof(float2) * c->M, c->st));
+    TRY(clear_acc(c));
     CK(c, launch_group_compress(g, (int64_t)ct.size(), c->st));
     launches = 3;  // contraction, softmax, contraction
   }
@@ -2920,7 +2947,7 @@ static emc_status batch_resp(emc_batch* b, int i) {
                          b->st));
   c->resp_source = 1;
   c->stage = 2;
-  BCK(b, cudaMemsetAsync(c->d_acc, 0, sizeof(float2) * c->M, b->st));
+  BTRY(b, c, clear_acc(c));
   return EMC_OK;
 }
 
@@ -3143,6 +3170,7 @@ emc_status emc_batch_iterate(emc_batch* b) {
     if (s == EMC_OK) s = batch_resp(b, i);
     if (s == EMC_OK) s = batch_own_compress(b, i);
     if (s != EMC_OK) return s;
+    BTRY(b, c, merge_acc(c));
     c->stage = 3;
     BTRY(b, c, emc_normalize(c));
   }
@@ -3204,6 +3232,7 @@ emc_status emc_batch_iterate(emc_batch* b) {
   for (int i = 0; i < n; ++i) {
     if (b->alone[i]) continue;
     emc_context* c = b->ctx[i];
+    BTRY(b, c, merge_acc(c));
     c->stage = 3;
     BTRY(b, c, emc_normalize(c));
   }

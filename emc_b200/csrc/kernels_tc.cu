@@ -18,7 +18,7 @@
 #include <cstdint>
 #include <type_traits>
 
-#include "fixed.cuh"
+#include "insert.cuh"
 #include "tc.cuh"
 #include "tc_ptx.cuh"
 #include "voxel.h"
@@ -483,26 +483,15 @@ struct EpiMaxT {
 };
 using EpiMax = EpiMaxT<4>;
 
-// (model, weight) += (x, y) at one voxel as a single vector reduction.
-__device__ __forceinline__ void red_add_v2(float2* p, float x, float y) {
-  asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(x), "f"(y) : "memory");
-}
-// The same into the context's accumulators: FP32, or the order-independent
-// fixed-point limbs of the deterministic mode.
-__device__ __forceinline__ void insert_add(const CmpEpiArgs& e, int64_t vox, float x, float y) {
-  if (e.acc64) {
-    add_fixed(e.acc64 + 8 * vox, x);
-    add_fixed(e.acc64 + 8 * vox + 4, y);
-  } else {
-    red_add_v2(e.acc + vox, x, y);
-  }
-}
-
 // compress: row = rotation, column = active pixel; inserts into model/weight.
+// Sixteen epilogue warps (four per TMEM lane quarter, a quarter of the columns
+// each) keep the insertions in flight: with four, the insertion outlasted the
+// contraction (trilinear, 2,000 patterns x 36,540 rotations at 96^3: 21.6 ms
+// with four, 9.2 ms with sixteen).
 struct EpiCmp {
   static constexpr bool kListed = false;
   static constexpr int kSets = 1;
-  static constexpr int kEpiWarps = 4;
+  static constexpr int kEpiWarps = 16;
   static constexpr int kSmemBytes = BN * 16;
   CmpEpiArgs a;
   int64_t j0;
@@ -513,13 +502,13 @@ struct EpiCmp {
   __device__ void tile_begin(int64_t mt, int64_t nt, int tid, uint8_t* smem) {
     float4* cs = reinterpret_cast<float4*>(smem);
     j0 = nt * BN;
-    epi_bar();
-    for (int c = tid; c < BN; c += 128) {
+    epi_bar(32 * kEpiWarps);
+    for (int c = tid; c < BN; c += 32 * kEpiWarps) {
       const int64_t j = j0 + c;
       cs[c] = j < a.npa ? make_float4(a.cx[j], a.cy[j], a.cz[j], a.ins[j] == 1 ? 1.0f : 0.0f)
                         : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    epi_bar();
+    epi_bar(32 * kEpiWarps);
     (void)mt;
   }
   __device__ void row_begin(int64_t r) {
@@ -549,9 +538,7 @@ struct EpiCmp {
         if (q.w == 0.0f) continue;
         float u[3];
         emc_voxel::position(m, a.side, q.x, q.y, q.z, u);
-        int64_t vox;
-        if (!emc_voxel::nearest(u, a.side, 0, &vox)) continue;
-        insert_add(a, vox, __uint_as_float(v[k]) * wU, wT);
+        insert_nearest(a.ins_acc, u, a.side, __uint_as_float(v[k]) * wU, wT);
       }
     } else {
 #pragma unroll
@@ -560,14 +547,7 @@ struct EpiCmp {
         if (q.w == 0.0f) continue;
         float u[3];
         emc_voxel::position(m, a.side, q.x, q.y, q.z, u);
-        const float val = __uint_as_float(v[k]) * wU;
-#pragma unroll
-        for (int cc = 0; cc < 8; ++cc) {
-          int64_t vox;
-          float wc;
-          if (!emc_voxel::trilinear_corner(u, a.side, cc, &vox, &wc) || wc == 0.0f) continue;
-          insert_add(a, vox, wc * val, wc * wT);
-        }
+        insert_trilinear(a.ins_acc, u, a.side, __uint_as_float(v[k]) * wU, wT);
       }
     }
   }
@@ -772,7 +752,7 @@ struct EpiBatchMax {
 struct EpiBatchCmp {
   static constexpr bool kListed = true;
   static constexpr int kSets = kMaxBatch;
-  static constexpr int kEpiWarps = 4;
+  static constexpr int kEpiWarps = EpiCmp::kEpiWarps;
   static constexpr int kSmemBytes = EpiCmp::kSmemBytes;
   BatchCmpArgs a;
   EpiCmp inner;
@@ -820,7 +800,7 @@ struct EpiBatchMaxPair {
 struct EpiBatchCmpPair {
   static constexpr bool kListed = true;
   static constexpr int kSets = kMaxBatch;
-  static constexpr int kEpiWarps = 4;
+  static constexpr int kEpiWarps = EpiCmp::kEpiWarps;
   static constexpr int kSmemBytes = EpiCmp::kSmemBytes;
   BatchCmpArgs a;
   EpiCmp inner;
@@ -1101,10 +1081,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * Epi::kEpiW
     }
   } else {
     // -------------------------------------------------- epilogue warps (both CTAs)
-    // TMEM lane quarter = warp % 4; with 8 epilogue warps two share a quarter
-    // and take one half of the columns each
+    // TMEM lane quarter = warp % 4; with 8 or 16 epilogue warps, 2 or 4 share
+    // a quarter and split the columns
     constexpr int EW = Epi::kEpiWarps;
-    static_assert(EW == 4 || EW == 8, "4 or 8 epilogue warps");
+    static_assert(EW == 4 || EW == 8 || EW == 16, "4, 8 or 16 epilogue warps");
     constexpr int COLS = BN / (EW / 4);
     const int quarter = warp & 3;
     const int ep_tid = threadIdx.x - 64;
@@ -1806,7 +1786,7 @@ __global__ void sorted_place_kernel(const int2* rp, const float* Pv, int64_t n, 
 // of 512 threads where the slice leaves room for few blocks.
 constexpr int kInsertUnroll = 4;
 template <int THREADS, int INTERP>
-__global__ void __launch_bounds__(THREADS, THREADS == 512 ? 3 : 6)
+__global__ void __launch_bounds__(THREADS, INTERP == 0 ? (THREADS == 512 ? 3 : 6) : (THREADS == 512 ? 2 : 4))
     list_compress_kernel(const ListCmpArgs a) {
   extern __shared__ float Us[];  // [npa]
   const int64_t r = blockIdx.x;
@@ -1854,19 +1834,22 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 3 : 6)
       float u[3];
       emc_voxel::position(m, e.side, q[k].x, q[k].y, q[k].z, u);
       const float val = Us[j0 + k * THREADS] * wT;
-      if constexpr (INTERP == 0) {
-        int vox;
-        if (emc_voxel::nearest32(u, e.side, 0, &vox)) insert_add(e, vox, val, wT);
-      } else {
-#pragma unroll
-        for (int cc = 0; cc < 8; ++cc) {
-          int64_t vox;
-          float wc;
-          if (!emc_voxel::trilinear_corner(u, e.side, cc, &vox, &wc) || wc == 0.0f) continue;
-          insert_add(e, vox, wc * val, wc * wT);
-        }
-      }
+      if constexpr (INTERP == 0)
+        insert_nearest(e.ins_acc, u, e.side, val, wT);
+      else
+        insert_trilinear(e.ins_acc, u, e.side, val, wT);
     }
+  }
+}
+
+__global__ void merge_odd_kernel(float2* acc, const float2* odd, int64_t M) {
+  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < M;
+       v += (int64_t)gridDim.x * blockDim.x) {
+    float2 a = acc[v];
+    const float2 b = odd[v + 1];
+    a.x += b.x;
+    a.y += b.y;
+    acc[v] = a;
   }
 }
 
@@ -2341,6 +2324,11 @@ cudaError_t launch_list_compress(const ListCmpArgs& a, cudaStream_t st) {
   if (a.e.interp == 0)
     return wide ? run_list_compress<512, 0>(a, smem, st) : run_list_compress<256, 0>(a, smem, st);
   return wide ? run_list_compress<512, 1>(a, smem, st) : run_list_compress<256, 1>(a, smem, st);
+}
+
+cudaError_t launch_merge_odd(float2* acc, const float2* odd, int64_t M, cudaStream_t st) {
+  merge_odd_kernel<<<(unsigned)std::min<int64_t>((M + 255) / 256, 1184), 256, 0, st>>>(acc, odd, M);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_resp_export(const RespArgs& a, float* P, cudaStream_t st) {

@@ -65,6 +65,17 @@ cudaError_t launch_maximize_pair_tc(const CUtensorMap& tmK, const CUtensorMap& t
                                     int64_t Kpad, const MaxEpiArgs& e, TcStatus* status,
                                     int num_sms, cudaStream_t st, int raster);
 
+// Where an insertion adds: FP32 pairs (acc), or the fixed-point limbs of the
+// deterministic mode (acc64).  odd (trilinear, optional): a second array of
+// pairs, shifted by one voxel (odd[v + 1] belongs to voxel v), so that the
+// pairs of voxels (v, v + 1) are 16-byte aligned there for odd v as they are
+// in acc for even v; launch_merge_odd adds it to acc.
+struct InsertAcc {
+  float2* acc;
+  float2* odd;
+  unsigned long long* acc64;
+};
+
 // Compress contraction: acc[r][j] = sum_p (P'_hi + P'_lo)[r][p] Kt[j][p] with
 // P' = c0 P / (T_r phi_p), i.e. the averaged slice U_r / T_r; 128 rotations x
 // 256 pixels per tile, inserted in the epilogue.
@@ -81,13 +92,14 @@ struct CmpEpiArgs {
   const float* cz;
   const int32_t* ins;      // [npa] insert flag (mask == 1)
   const float4* pc;        // [npa] (cx, cy, cz, ins as 1 or 0)
-  float2* acc;             // [side^3] interleaved (model, weight) accumulators
-  unsigned long long* acc64;  // or, when set, fixed-point limbs [side^3][8] (fixed.cuh)
+  InsertAcc ins_acc;       // [side^3] interleaved (model, weight) accumulators (insert.cuh)
   // optional: the launch returns at once unless *gate_count > gate_cap (the
   // dense form as the fallback of responsibility lists that overflowed)
   const unsigned long long* gate_count;
   int64_t gate_cap;
 };
+// acc[v] += odd[v + 1] (InsertAcc::odd, after the insertion).
+cudaError_t launch_merge_odd(float2* acc, const float2* odd, int64_t M, cudaStream_t st);
 // raster: rotation tiles per band of the tile order.
 cudaError_t launch_compress_tc(const CUtensorMap& tmPhi, const CUtensorMap& tmPlo,
                                const CUtensorMap& tmKt, int64_t Rpad, int64_t Ppad,
