@@ -1137,7 +1137,7 @@ static emc_status list_buffers(emc_context* c) {
   if (!c->d_lcount) {
     const int64_t R = c->R;
     TRY(c->alloc(&c->d_lcount, 1));
-    TRY(c->alloc(&c->d_lrowtot, R));
+    TRY(c->alloc(&c->d_lrowtot, R + 1));
     TRY(c->alloc(&c->d_lrowoff, R + 1));
     TRY(c->alloc(&c->d_lcursor, R));
   }
@@ -1224,7 +1224,7 @@ static emc_status mixed_resp_pass(emc_context* c, bool allow_lists = true) {
                                        c->d_lrowoff, c->d_lpat, c->d_lx, c->st));
       }
       c->list_mode = true;
-      c->launches += 6;  // combine, row sums, T, count, scan, fill
+      c->launches += 6;  // combine, row sums, T, count, room, fill
     } else {
       // more entries than the compaction holds: the dense operand this time,
       // room for them next time if they are worth it
@@ -1236,9 +1236,8 @@ static emc_status mixed_resp_pass(emc_context* c, bool allow_lists = true) {
     CK(c, launch_resp_pass(a, c->st));
     c->launches += 3;  // combine, 2 sweeps
   }
-  CK(c, launch_sum_f64(c->d_plogp, N, c->d_stats + 2, c->st));
-  CK(c, launch_sum_f64(c->d_lse, N, c->d_stats + 3, c->st));
-  c->launches += 2;
+  CK(c, launch_sum2_f64(c->d_plogp, c->d_lse, N, c->d_stats + 2, c->st));
+  c->launches += 1;
   return EMC_OK;
 }
 
@@ -1264,9 +1263,8 @@ static emc_status gated_list_pass(emc_context* c) {
   a.gate_count = c->d_lcount;
   a.gate_cap = c->lcomp_cap;
   CK(c, launch_resp_write(a, c->st));
-  CK(c, launch_sum_f64(c->d_plogp, c->N, c->d_stats + 2, c->st));
-  CK(c, launch_sum_f64(c->d_lse, c->N, c->d_stats + 3, c->st));
-  c->launches += 9;  // combine, row sums, T, count, scan, fill, write, 2 sums
+  CK(c, launch_sum2_f64(c->d_plogp, c->d_lse, c->N, c->d_stats + 2, c->st));
+  c->launches += 8;  // combine, row sums, T, count, room, fill, write, sums
   return EMC_OK;
 }
 
@@ -1376,9 +1374,8 @@ static emc_status chunked_maximize(emc_context* c) {
                                       c->d_lx, c->st));
   }
   c->list_mode = true;
-  CK(c, launch_sum_f64(c->d_plogp, N, c->d_stats + 2, c->st));
-  CK(c, launch_sum_f64(c->d_lse, N, c->d_stats + 3, c->st));
-  c->launches += 7;  // finish, T, count, scan, fill, 2 sums
+  CK(c, launch_sum2_f64(c->d_plogp, c->d_lse, N, c->d_stats + 2, c->st));
+  c->launches += 6;  // finish, T, count, room, fill, sums
   return EMC_OK;
 }
 
@@ -1600,9 +1597,8 @@ emc_status emc_maximize(emc_context* c) {
                                   c->st));
       c->launches += 2;
     }
-    CK(c, launch_sum_f64(c->d_plogp32, N, c->d_stats + 2, c->st));
-    CK(c, launch_sum_f64(c->d_lse32, N, c->d_stats + 3, c->st));
-    c->launches += 6;
+    CK(c, launch_sum2_f64(c->d_plogp32, c->d_lse32, N, c->d_stats + 2, c->st));
+    c->launches += 5;
   } else if (c->y_rows < R) {
     TRY(chunked_maximize(c));
   } else {
@@ -1685,7 +1681,8 @@ emc_status emc_compress_insert(emc_context* c) {
       // responsibility lists x the counts' photon lists (built once per upload)
       if (!c->csr.valid) TRY(build_rows(c, c->d_K, c->N, c->npa, c->csr, false));
       ListCmpArgs la{};
-      la.rowoff = c->d_lrowoff;
+      la.rowbeg = c->d_lrowoff;
+      la.rowend = c->det ? c->d_lrowoff + 1 : c->d_lcursor;  // sorted lists lie end to end
       la.pat = c->d_lpat;
       la.xv = c->d_lx;
       la.kptr = c->csr.ptr;
@@ -1729,7 +1726,7 @@ emc_status emc_normalize(emc_context* c) {
   else
     CK(c, launch_normalize_acc(c->d_acc, c->d_model, c->d_weight, c->M, c->d_scratch,
                                c->d_stats, c->st));
-  c->launches += 4;
+  c->launches += 2;
   c->mark(5);
   c->stage = 0;
   return EMC_OK;
@@ -2717,7 +2714,7 @@ static emc_status run_proposed(emc_context* c, const ProposedPlan& pl, Select se
     CK(c, launch_group_softmax(g, c->st));
     if (lists) {
       if (!c->d_lrowoff) {
-        TRY(c->alloc(&c->d_lrowtot, R));
+        TRY(c->alloc(&c->d_lrowtot, R + 1));
         TRY(c->alloc(&c->d_lrowoff, R + 1));
       }
       if (!c->d_lcursor) TRY(c->alloc(&c->d_lcursor, R));
@@ -2728,14 +2725,14 @@ static emc_status run_proposed(emc_context* c, const ProposedPlan& pl, Select se
       TRY(grow(c, &c->d_lx, cap, evals + 1));
       c->lcap_x = cap;
       CK(c, launch_group_list_count(g, kListRel, c->d_lrowtot, c->st));
-      CK(c, launch_list_rowscan(c->d_lrowtot, R, c->d_lrowoff, c->st));
-      CK(c, launch_group_list_fill(g, kListRel, c->d_lcursor, c->d_lrowoff, c->d_lpat, c->d_lx,
-                                   c->st));
+      CK(c, launch_list_alloc(c->d_lrowtot, R, c->d_lrowoff, c->d_lcursor, c->st));
+      CK(c, launch_group_list_fill(g, kListRel, c->d_lcursor, c->d_lpat, c->d_lx, c->st));
       if (!c->csr.valid) TRY(build_rows(c, c->d_K, c->N, c->npa, c->csr, false));
       c->mark(3);
       TRY(clear_acc(c));
       ListCmpArgs la{};
-      la.rowoff = c->d_lrowoff;
+      la.rowbeg = c->d_lrowoff;
+      la.rowend = c->d_lcursor;
       la.pat = c->d_lpat;
       la.xv = c->d_lx;
       la.kptr = c->csr.ptr;
@@ -2782,11 +2779,10 @@ static emc_status run_proposed(emc_context* c, const ProposedPlan& pl, Select se
   c->mark(4);
   CK(c, launch_normalize_acc(c->d_acc, c->d_model, c->d_weight, c->M, c->d_scratch, c->d_stats,
                              c->st));
-  CK(c, launch_sum_f64(c->d_plogp_c, N, c->d_stats + 2, c->st));
-  CK(c, launch_sum_f64(c->d_lse_c, N, c->d_stats + 3, c->st));
+  CK(c, launch_sum2_f64(c->d_plogp_c, c->d_lse_c, N, c->d_stats + 2, c->st));
   c->mark(5);
-  // select, the grouped stages, normalise (4), two sums
-  c->launches += 1 + launches + 6;
+  // select, the grouped stages, normalise (2), the sums
+  c->launches += 1 + launches + 3;
   c->stage = 0;
   TRY(check_status(c));
   double h[4];
@@ -2960,7 +2956,8 @@ static emc_status batch_own_compress(emc_batch* b, int i) {
   if (b->lists[i]) {
     if (!c->csr.valid) BTRY(b, c, build_rows(c, c->d_K, c->N, c->npa, c->csr, false));
     ListCmpArgs la{};
-    la.rowoff = c->d_lrowoff;
+    la.rowbeg = c->d_lrowoff;
+    la.rowend = c->d_lcursor;
     la.pat = c->d_lpat;
     la.xv = c->d_lx;
     la.kptr = c->csr.ptr;

@@ -213,6 +213,9 @@ cudaError_t launch_normalize_acc(const float2* acc, float* model, float* weight,
 cudaError_t launch_model_max(const float* model, int64_t M, double* scratch, double* out,
                              cudaStream_t st);
 cudaError_t launch_fill(float* x, int64_t n, float v, cudaStream_t st);
+// out[0], out[1] = the sums of a and of b.
+cudaError_t launch_sum2_f64(const double* a, const double* b, int64_t n, double* out,
+                            cudaStream_t st);
 cudaError_t launch_sum_f64(const double* x, int64_t n, double* out, cudaStream_t st);
 
 }  // namespace emc

@@ -610,6 +610,17 @@ __global__ void xlogx_partial(const float* x, int64_t n, double* part) {
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
+// out[0] = sum of a, out[1] = sum of b: one block each.
+__global__ void __launch_bounds__(1024) sum2_f64_kernel(const double* a, const double* b,
+                                                        int64_t n, double* out) {
+  __shared__ double red[32];
+  const double* x = blockIdx.x ? b : a;
+  double s = 0;
+  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += x[i];
+  s = block_sum(s, red);
+  if (threadIdx.x == 0) out[blockIdx.x] = s;
+}
+
 __global__ void sum_f64_kernel(const double* x, int64_t n, double* out) {
   __shared__ double red[32];
   double s = 0;
@@ -739,9 +750,11 @@ __global__ void fixed_to_pairs_kernel(const unsigned long long* acc64, int64_t M
   }
 }
 
+// Both divisions also zero the counter the scaling after them finishes with.
 __global__ void divide_kernel(float* model, const float* weight, int64_t M, int fp64,
-                              double* part) {
+                              double* part, unsigned int* done) {
   __shared__ double red[32];
+  if (blockIdx.x == 0 && threadIdx.x == 0) *done = 0;
   double s = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < M;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -760,8 +773,9 @@ __global__ void divide_kernel(float* model, const float* weight, int64_t M, int 
 
 // Mixed path: model/weight from the interleaved accumulators (FP64 division).
 __global__ void divide_acc_kernel(const float2* acc, float* model, float* weight, int64_t M,
-                                  double* part) {
+                                  double* part, unsigned int* done) {
   __shared__ double red[32];
+  if (blockIdx.x == 0 && threadIdx.x == 0) *done = 0;
   double s = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < M;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -775,10 +789,21 @@ __global__ void divide_acc_kernel(const float2* acc, float* model, float* weight
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-__global__ void scale_max_kernel(float* model, int64_t M, const double* sum, int fp64,
-                                 double* stats, double* part) {
-  __shared__ float red[32];
-  const double mean = *sum / (double)M;
+// model /= mean, its maximum to stats[1].  Every block sums the `nsum` partial
+// sums of the division itself (the same order, so the same mean), and the last
+// block to finish reduces the maxima, so no one-block kernel runs between the
+// two sweeps or after them.  done[0] is 0 on entry and on exit.
+__global__ void scale_max_kernel(float* model, int64_t M, const double* sums, int nsum, int fp64,
+                                 double* stats, float* maxima, unsigned int* done) {
+  __shared__ double red[32];
+  __shared__ double total;
+  __shared__ bool last;
+  double s = 0.0;
+  for (int i = threadIdx.x; i < nsum; i += blockDim.x) s += sums[i];
+  s = block_sum(s, red);
+  if (threadIdx.x == 0) total = s;
+  __syncthreads();
+  const double mean = total / (double)M;
   const float f = (float)(1.0 / mean);
   float mx = 0.0f;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < M;
@@ -788,10 +813,23 @@ __global__ void scale_max_kernel(float* model, int64_t M, const double* sum, int
     model[i] = v;
     mx = fmaxf(mx, v);
   }
-  mx = block_max(mx, red);
+  mx = block_max(mx, reinterpret_cast<float*>(red));
   if (threadIdx.x == 0) {
-    part[blockIdx.x] = mx;
+    maxima[blockIdx.x] = mx;
     if (blockIdx.x == 0) stats[0] = mean;
+    __threadfence();
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  mx = 0.0f;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x)
+    mx = fmaxf(mx, *reinterpret_cast<volatile float*>(maxima + i));
+  mx = block_max(mx, reinterpret_cast<float*>(red));
+  if (threadIdx.x == 0) {
+    stats[1] = mx;
+    *done = 0;
   }
 }
 
@@ -1175,14 +1213,24 @@ cudaError_t launch_insert(const InsertArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// Scratch of a normalisation (kReduceBlocks + kReduceBlocks / 2 + 1 doubles):
+// partial sums, block maxima, the counter of finished blocks.
+static void scale_after_division(float* model, int64_t M, int g, int fp64, double* scratch,
+                                 double* stats, cudaStream_t st) {
+  float* maxima = reinterpret_cast<float*>(scratch + kReduceBlocks);
+  unsigned int* done = reinterpret_cast<unsigned int*>(maxima + kReduceBlocks);
+  scale_max_kernel<<<g, kBlock, 0, st>>>(model, M, scratch, g, fp64, stats, maxima, done);
+}
+static unsigned int* done_counter(double* scratch) {
+  return reinterpret_cast<unsigned int*>(scratch + kReduceBlocks) + kReduceBlocks;
+}
+
 cudaError_t launch_normalize_model(float* model, const float* weight, int64_t M, int fp64,
                                    double* scratch, double* stats, cudaStream_t st) {
-  // scratch: kReduceBlocks + 2 doubles; stats[0] = mean, stats[1] = max
+  // stats[0] = mean, stats[1] = max
   const int g = grid_for(M);
-  divide_kernel<<<g, kBlock, 0, st>>>(model, weight, M, fp64, scratch);
-  sum_f64_kernel<<<1, kBlock, 0, st>>>(scratch, g, scratch + kReduceBlocks);
-  scale_max_kernel<<<g, kBlock, 0, st>>>(model, M, scratch + kReduceBlocks, fp64, stats, scratch);
-  max_f64_kernel<<<1, kBlock, 0, st>>>(scratch, g, stats + 1);
+  divide_kernel<<<g, kBlock, 0, st>>>(model, weight, M, fp64, scratch, done_counter(scratch));
+  scale_after_division(model, M, g, fp64, scratch, stats, st);
   return cudaGetLastError();
 }
 
@@ -1195,10 +1243,8 @@ cudaError_t launch_fixed_to_pairs(const unsigned long long* acc64, int64_t M, fl
 cudaError_t launch_normalize_acc(const float2* acc, float* model, float* weight, int64_t M,
                                  double* scratch, double* stats, cudaStream_t st) {
   const int g = grid_for(M);
-  divide_acc_kernel<<<g, kBlock, 0, st>>>(acc, model, weight, M, scratch);
-  sum_f64_kernel<<<1, kBlock, 0, st>>>(scratch, g, scratch + kReduceBlocks);
-  scale_max_kernel<<<g, kBlock, 0, st>>>(model, M, scratch + kReduceBlocks, 1, stats, scratch);
-  max_f64_kernel<<<1, kBlock, 0, st>>>(scratch, g, stats + 1);
+  divide_acc_kernel<<<g, kBlock, 0, st>>>(acc, model, weight, M, scratch, done_counter(scratch));
+  scale_after_division(model, M, g, 1, scratch, stats, st);
   return cudaGetLastError();
 }
 
@@ -1213,6 +1259,12 @@ cudaError_t launch_model_max(const float* model, int64_t M, double* scratch, dou
 cudaError_t launch_fill(float* x, int64_t n, float v, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   fill_kernel<<<grid_for(n), kBlock, 0, st>>>(x, n, v);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_sum2_f64(const double* a, const double* b, int64_t n, double* out,
+                            cudaStream_t st) {
+  sum2_f64_kernel<<<2, 1024, 0, st>>>(a, b, n, out);
   return cudaGetLastError();
 }
 

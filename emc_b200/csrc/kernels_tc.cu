@@ -1162,28 +1162,46 @@ cudaError_t run_pair(const TmapSet<Epi::kSets>& maps, int64_t m_tiles, int64_t n
 //   lse = M + log sum_k s_k e^(m_k - M)
 //   D   = sum_k d_k e^(m_k - lse)                       (= sum_r P_rp X_rp)
 //   sum_r P log P = sum_k e^(m_k - lse) (q_k + (m_k - lse) s_k)
-__global__ void combine_kernel(const RespArgs a) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= a.N) return;
+// 32 patterns per block, its 8 warps share the partials: one thread per pattern
+// left most SMs idle (338 partials at 20,000 patterns: 0.57 ms on 79 blocks).
+// The sums are taken relative to M, so one pass follows the maximum:
+//   D = D' / S,  sum P log P = Q' / S - log S   (D', Q' and S relative to M)
+__global__ void __launch_bounds__(256) combine_kernel(const RespArgs a) {
+  __shared__ float sm[8][32];
+  __shared__ double ss[3][8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t p = (int64_t)blockIdx.x * 32 + lane;
+  const bool ok = p < a.N;
   float M = -FLT_MAX;
-  for (int64_t k = 0; k < a.nparts; ++k) M = fmaxf(M, a.part[k * a.N + p].x);
-  double S = 0.0;
-  for (int64_t k = 0; k < a.nparts; ++k) {
-    const float4 v = a.part[k * a.N + p];
-    if (v.y > 0.0f) S += (double)v.y * exp((double)v.x - (double)M);
+  if (ok)
+    for (int64_t k = w; k < a.nparts; k += 8) M = fmaxf(M, a.part[k * a.N + p].x);
+  sm[w][lane] = M;
+  __syncthreads();
+  for (int k = 0; k < 8; ++k) M = fmaxf(M, sm[k][lane]);
+  double S = 0.0, D = 0.0, Q = 0.0;
+  if (ok)
+    for (int64_t k = w; k < a.nparts; k += 8) {
+      const float4 v = a.part[k * a.N + p];
+      if (!(v.y > 0.0f)) continue;
+      const double dm = (double)v.x - (double)M, f = exp(dm);
+      S += (double)v.y * f;
+      D += (double)v.z * f;
+      Q += f * ((double)v.w + dm * (double)v.y);
+    }
+  ss[0][w][lane] = S;
+  ss[1][w][lane] = D;
+  ss[2][w][lane] = Q;
+  __syncthreads();
+  if (w != 0 || !ok) return;
+  for (int k = 1; k < 8; ++k) {
+    S += ss[0][k][lane];
+    D += ss[1][k][lane];
+    Q += ss[2][k][lane];
   }
-  const double lse = (double)M + log(S);
-  double D = 0.0, Q = 0.0;
-  for (int64_t k = 0; k < a.nparts; ++k) {
-    const float4 v = a.part[k * a.N + p];
-    if (!(v.y > 0.0f)) continue;
-    const double dm = (double)v.x - lse;
-    const double f = exp(dm);
-    D += (double)v.z * f;
-    Q += f * ((double)v.w + dm * (double)v.y);
-  }
-  a.lse[p] = lse;
-  a.plogp[p] = Q;
+  const double ls = log(S);
+  D /= S;
+  a.lse[p] = (double)M + ls;
+  a.plogp[p] = Q / S - ls;
   // emc_cuda.cu:226 for gaussian; poisson MLE sum K / sum_r P_rp sum W_r
   const double num = a.poisson ? a.patsum[p] : a.patstat[p];
   float phi = a.scaling[p];
@@ -1256,21 +1274,30 @@ __device__ __forceinline__ void load_consts(const RespArgs& a, int64_t p0, PatCo
 // every entry that does not underflow, and the one rounding left is the
 // one the FP64 difference gets when it is rounded to FP32.
 template <bool POISSON>
-__device__ __forceinline__ void probs_from(const PatConst<POISSON>& k, float4 y, double rs,
-                                           float (&P)[4]) {
+__device__ __forceinline__ void log_probs(const PatConst<POISSON>& k, float4 y, double rs,
+                                          float (&d)[4]) {
   const float yy[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    float d;
     if constexpr (POISSON)
-      d = __fsub_rn(__fsub_rn(yy[i], k.lse_hi[i]), k.lse_lo[i]);
+      d[i] = __fsub_rn(__fsub_rn(yy[i], k.lse_hi[i]), k.lse_lo[i]);
     else
-      d = (float)(fma((double)yy[i], k.c1[i], k.c0[i] - rs) - k.lse[i]);
-    P[i] = k.ok[i] ? expf(d) : 0.0f;
+      d[i] = (float)(fma((double)yy[i], k.c1[i], k.c0[i] - rs) - k.lse[i]);
   }
+}
+template <bool POISSON>
+__device__ __forceinline__ void probs_from(const PatConst<POISSON>& k, float4 y, double rs,
+                                           float (&P)[4]) {
+  log_probs<POISSON>(k, y, rs, P);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) P[i] = k.ok[i] ? expf(P[i]) : 0.0f;
 }
 
 // Sweep A: Tpart[pattern block][r] = sum over the block's patterns of P_rp.
+// Once the posteriors are sharp, most of P is zero in FP32: where no element
+// of a warp's four rows x 128 patterns reaches kExpZero, they are left at the
+// comparison (no exponential, no reduction, no compaction).
+constexpr float kExpZero = -105.0f;  // expf is zero below (the smallest float is e^-103.3)
 template <bool POISSON>
 __global__ void __launch_bounds__(kSweepThreads, 4) rowsum_kernel(const RespArgs a) {
   __shared__ float red[kSweepThreads / 32][kSweepRows];
@@ -1313,14 +1340,29 @@ __global__ void __launch_bounds__(kSweepThreads, 4) rowsum_kernel(const RespArgs
       y[u] = (r < a.R && any) ? *reinterpret_cast<const float4*>(a.Y + r * a.ldY + p0)
                               : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    bool live = false;
+    float d[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t r = r0 + i0 + u;
+      const bool in = r < a.R && any;
+      const double rs = POISSON || !in ? 0.0 : a.rowstat[r] * a.gauss_inv;
+      log_probs<POISSON>(k, y[u], rs, d[u]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) live |= in && !(d[u][j] < kExpZero);
+    }
+    if (!__any_sync(0xffffffffu, live)) {
+      if (lane < 4) red[w][i0 + lane] = 0.0f;
+      continue;
+    }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int64_t r = r0 + i0 + u;
       t[u] = 0.0f;
       float P[4] = {0.f, 0.f, 0.f, 0.f};
       if (r < a.R && any) {
-        const double rs = POISSON ? 0.0 : a.rowstat[r] * a.gauss_inv;
-        probs_from<POISSON>(k, y[u], rs, P);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) P[j] = k.ok[j] ? expf(d[u][j]) : 0.0f;
         t[u] = (P[0] + P[1]) + (P[2] + P[3]);
       }
       if (a.list_count) {
@@ -1350,12 +1392,19 @@ __global__ void __launch_bounds__(kSweepThreads, 4) rowsum_kernel(const RespArgs
         }
       }
     }
+    // four row sums by halving exchanges: lane 8 u ends with row u's
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int o = 16, n = 2; n >= 1; o >>= 1, n >>= 1) {
+      const bool hi = lane & o;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t[u] += __shfl_xor_sync(0xffffffffu, t[u], o);
-      if (lane == 0) red[w][i0 + u] = t[u];
+      for (int i = 0; i < n; ++i) {
+        const float keep = hi ? t[i + n] : t[i], send = hi ? t[i] : t[i + n];
+        t[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
     }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) t[0] += __shfl_xor_sync(0xffffffffu, t[0], o);
+    if ((lane & 7) == 0) red[w][i0 + (lane >> 3)] = t[0];
   }
   if (a.list_count && nb > 0) flush();
   __syncthreads();
@@ -1537,23 +1586,48 @@ __global__ void __launch_bounds__(1024) scan_apply_kernel(const int64_t* in, int
 
 // T_r from the row-sum partials (FP64 sum in pattern-block order, as
 // write_kernel forms it).
-__global__ void finish_T_kernel(const float* Tpart, int64_t nblk, int64_t R, float* T) {
+// rowtot (optional, [R + 1]): zeroed for the lists' counts.
+__global__ void finish_T_kernel(const float* Tpart, int64_t nblk, int64_t R, float* T,
+                                int64_t* rowtot) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (rowtot && r <= R) rowtot[r] = 0;
   if (r >= R) return;
   double t = 0.0;
   for (int64_t b = 0; b < nblk; ++b) t += Tpart[b * R + r];
   T[r] = (float)t;
 }
 
+// Room for every rotation's list: beg[r] (and the fill's cursor[r]) from one
+// counter, a warp's rotations at a time.  The lists need not lie in rotation
+// order, so no scan over the rotations is needed (a block scanning 86,520
+// counts took 0.1 ms).
+__global__ void list_alloc_kernel(const int64_t* rowtot, int64_t R, unsigned long long* total,
+                                  int64_t* beg, int64_t* cursor) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const long long n = r < R ? rowtot[r] : 0;
+  long long inc = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  unsigned long long base = 0;
+  if (lane == 31) base = atomicAdd(total, (unsigned long long)inc);
+  base = __shfl_sync(0xffffffffu, base, 31);
+  if (r < R) beg[r] = cursor[r] = (int64_t)base + inc - n;
+}
+
 // Counting sort of the compacted entries by rotation: STEP 0 counts per
-// rotation, STEP 1 writes (pattern, x) at rowoff[r] + cursor.
+// rotation, STEP 1 writes (pattern, x) at the rotation's cursor, which ends at
+// the end of its list.
 // Entries below rel_min T_r are dropped: each moves its rotation's slice sum
 // by less than rel_min.
 template <int STEP>
 __global__ void compact_sort_kernel(const int2* rp, const float* Pv, int64_t n, const float* T,
                                     const float* new_scaling, float rel_min,
-                                    unsigned long long* cnt, const int64_t* rowoff, int32_t* pat,
-                                    float* xv, const unsigned long long* n_dev) {
+                                    unsigned long long* cnt, int32_t* pat, float* xv,
+                                    const unsigned long long* n_dev) {
   if (n_dev) {  // the count on the device; above the capacity n the lists stay empty
     const unsigned long long c = *n_dev;
     if (c > (unsigned long long)n) return;
@@ -1567,7 +1641,7 @@ __global__ void compact_sort_kernel(const int2* rp, const float* Pv, int64_t n, 
     if (STEP == 0) {
       atomicAdd(cnt + v.x, 1ull);
     } else {
-      const int64_t pos = rowoff[v.x] + (int64_t)atomicAdd(cnt + v.x, 1ull);
+      const int64_t pos = (int64_t)atomicAdd(cnt + v.x, 1ull);
       pat[pos] = v.y;
       xv[pos] = P / Tr / new_scaling[v.y];
     }
@@ -1802,7 +1876,7 @@ __global__ void __launch_bounds__(THREADS, INTERP == 0 ? (THREADS == 512 ? 3 : 6
     // the listed patterns in list order by one warp: a pattern's photons lie
     // on distinct pixels, so each pixel sums its terms in that order
     if (w == 0)
-      for (int64_t q = a.rowoff[r]; q < a.rowoff[r + 1]; ++q) {
+      for (int64_t q = a.rowbeg[r]; q < a.rowend[r]; ++q) {
         const int64_t p = a.pat[q];
         const float x = a.xv[q];
         for (int64_t t = a.kptr[p] + lane; t < a.kptr[p + 1]; t += 32)
@@ -1810,7 +1884,7 @@ __global__ void __launch_bounds__(THREADS, INTERP == 0 ? (THREADS == 512 ? 3 : 6
         __syncwarp();
       }
   } else {
-    for (int64_t q = a.rowoff[r] + w; q < a.rowoff[r + 1]; q += THREADS / 32) {
+    for (int64_t q = a.rowbeg[r] + w; q < a.rowend[r]; q += THREADS / 32) {
       const int64_t p = a.pat[q];
       const float x = a.xv[q];
       for (int64_t t = a.kptr[p] + lane; t < a.kptr[p + 1]; t += 32)
@@ -2092,7 +2166,7 @@ cudaError_t launch_batch_compress_tc(const TmapSet<kMaxBatch>& maps, int64_t n_t
 }
 
 cudaError_t launch_resp_rowsums(RespArgs& a, cudaStream_t st) {
-  combine_kernel<<<(unsigned)((a.N + 255) / 256), 256, 0, st>>>(a);
+  combine_kernel<<<(unsigned)((a.N + 31) / 32), 256, 0, st>>>(a);
   const int64_t nblk = (a.N + kSweepPatterns - 1) / kSweepPatterns;
   const int64_t rblk = (a.R + kSweepRows - 1) / kSweepRows;
   if (a.poisson)
@@ -2122,28 +2196,27 @@ cudaError_t launch_resp_pass(RespArgs& a, cudaStream_t st) {
 
 int64_t resp_list_blocks(int64_t N) { return (N + kSweepPatterns - 1) / kSweepPatterns; }
 
-cudaError_t launch_list_rowscan(const int64_t* rowtot, int64_t R, int64_t* rowoff,
-                                cudaStream_t st) {
-  list_rowscan_kernel<<<1, 1024, 0, st>>>(rowtot, R, rowoff);
+cudaError_t launch_list_alloc(int64_t* rowtot, int64_t R, int64_t* beg, int64_t* cursor,
+                              cudaStream_t st) {
+  list_alloc_kernel<<<(unsigned)((R + 255) / 256), 256, 0, st>>>(
+      rowtot, R, reinterpret_cast<unsigned long long*>(rowtot + R), beg, cursor);
   return cudaGetLastError();
 }
 
 cudaError_t launch_list_from_compact(RespArgs& a, int64_t n, float rel_min, int64_t* rowtot,
-                                     int64_t* cursor, int64_t* rowoff, int32_t* pat, float* xv,
+                                     int64_t* cursor, int64_t* rowbeg, int32_t* pat, float* xv,
                                      cudaStream_t st, const unsigned long long* n_dev) {
   const int64_t nblk = resp_list_blocks(a.N);
-  finish_T_kernel<<<(unsigned)((a.R + 255) / 256), 256, 0, st>>>(a.Tpart, nblk, a.R, a.T);
-  cudaError_t e = cudaMemsetAsync(rowtot, 0, sizeof(int64_t) * a.R, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(cursor, 0, sizeof(int64_t) * a.R, st);
-  if (e != cudaSuccess) return e;
+  finish_T_kernel<<<(unsigned)(a.R / 256 + 1), 256, 0, st>>>(a.Tpart, nblk, a.R, a.T, rowtot);
   const unsigned g = (unsigned)std::min<int64_t>((n + 255) / 256 + 1, 4096);
   compact_sort_kernel<0><<<g, 256, 0, st>>>(a.list_rp, a.list_P, n, a.T, a.new_scaling, rel_min,
                                             reinterpret_cast<unsigned long long*>(rowtot),
-                                            nullptr, nullptr, nullptr, n_dev);
-  list_rowscan_kernel<<<1, 1024, 0, st>>>(rowtot, a.R, rowoff);
+                                            nullptr, nullptr, n_dev);
+  cudaError_t e = launch_list_alloc(rowtot, a.R, rowbeg, cursor, st);
+  if (e != cudaSuccess) return e;
   compact_sort_kernel<1><<<g, 256, 0, st>>>(a.list_rp, a.list_P, n, a.T, a.new_scaling, rel_min,
-                                            reinterpret_cast<unsigned long long*>(cursor), rowoff,
-                                            pat, xv, n_dev);
+                                            reinterpret_cast<unsigned long long*>(cursor), pat, xv,
+                                            n_dev);
   return cudaGetLastError();
 }
 
@@ -2161,20 +2234,20 @@ cudaError_t launch_cand_probs(const RespArgs& a, int64_t n, float* Pv, double* T
 
 cudaError_t launch_list_from_candidates(RespArgs& a, int64_t n, float rel_min, float* Pv,
                                         double* T64, int64_t* rowtot, int64_t* cursor,
-                                        int64_t* rowoff, int32_t* pat, float* xv, cudaStream_t st) {
+                                        int64_t* rowbeg, int32_t* pat, float* xv, cudaStream_t st) {
   cudaError_t e = launch_cand_probs(a, n, Pv, T64, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(rowtot, 0, sizeof(int64_t) * a.R, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(cursor, 0, sizeof(int64_t) * a.R, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(rowtot, 0, sizeof(int64_t) * (a.R + 1), st);
   if (e != cudaSuccess) return e;
   const unsigned g = grid_for(n);
   T_from64_kernel<<<(unsigned)((a.R + 255) / 256), 256, 0, st>>>(T64, a.R, a.T);
   compact_sort_kernel<0><<<g, 256, 0, st>>>(a.list_rp, Pv, n, a.T, a.new_scaling, rel_min,
                                             reinterpret_cast<unsigned long long*>(rowtot),
-                                            nullptr, nullptr, nullptr, nullptr);
-  list_rowscan_kernel<<<1, 1024, 0, st>>>(rowtot, a.R, rowoff);
+                                            nullptr, nullptr, nullptr);
+  e = launch_list_alloc(rowtot, a.R, rowbeg, cursor, st);
+  if (e != cudaSuccess) return e;
   compact_sort_kernel<1><<<g, 256, 0, st>>>(a.list_rp, Pv, n, a.T, a.new_scaling, rel_min,
-                                            reinterpret_cast<unsigned long long*>(cursor), rowoff,
-                                            pat, xv, nullptr);
+                                            reinterpret_cast<unsigned long long*>(cursor), pat, xv,
+                                            nullptr);
   return cudaGetLastError();
 }
 
@@ -2265,7 +2338,8 @@ cudaError_t launch_list_from_sorted(const int2* rp, const float* Pv, int64_t n, 
 }
 
 cudaError_t launch_finish_T(const float* Tpart, int64_t N, int64_t R, float* T, cudaStream_t st) {
-  finish_T_kernel<<<(unsigned)((R + 255) / 256), 256, 0, st>>>(Tpart, resp_list_blocks(N), R, T);
+  finish_T_kernel<<<(unsigned)((R + 255) / 256), 256, 0, st>>>(Tpart, resp_list_blocks(N), R, T,
+                                                              nullptr);
   return cudaGetLastError();
 }
 

@@ -483,7 +483,7 @@ __global__ void group_softmax_kernel(const GroupArgs g) {
 // warp per pattern.
 template <int FILL>
 __global__ void group_list_kernel(const GroupArgs g, float theta, unsigned long long* cnt,
-                                  const int64_t* rowoff, int32_t* pat, float* xv) {
+                                  int32_t* pat, float* xv) {
   const int64_t p = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (p >= g.N) return;
@@ -508,7 +508,7 @@ __global__ void group_list_kernel(const GroupArgs g, float theta, unsigned long 
       if (FILL == 0) {
         atomicAdd(cnt + r, 1ull);
       } else {
-        const int64_t pos = rowoff[r] + (int64_t)atomicAdd(cnt + r, 1ull);
+        const int64_t pos = (int64_t)atomicAdd(cnt + r, 1ull);
         pat[pos] = (int32_t)p;
         xv[pos] = x;
       }
@@ -731,20 +731,17 @@ cudaError_t launch_audit(const AuditArgs& a, int64_t n_audit, cudaStream_t st) {
 
 cudaError_t launch_group_list_count(const GroupArgs& g, float theta, int64_t* cnt,
                                     cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(int64_t) * g.R, st);
+  cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(int64_t) * (g.R + 1), st);
   if (e != cudaSuccess) return e;
   group_list_kernel<0><<<(unsigned)((g.N + 7) / 8), 256, 0, st>>>(
-      g, theta, reinterpret_cast<unsigned long long*>(cnt), nullptr, nullptr, nullptr);
+      g, theta, reinterpret_cast<unsigned long long*>(cnt), nullptr, nullptr);
   return cudaGetLastError();
 }
 
-cudaError_t launch_group_list_fill(const GroupArgs& g, float theta, int64_t* cursor,
-                                   const int64_t* rowoff, int32_t* pat, float* xv,
-                                   cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(cursor, 0, sizeof(int64_t) * g.R, st);
-  if (e != cudaSuccess) return e;
+cudaError_t launch_group_list_fill(const GroupArgs& g, float theta, int64_t* cursor, int32_t* pat,
+                                   float* xv, cudaStream_t st) {
   group_list_kernel<1><<<(unsigned)((g.N + 7) / 8), 256, 0, st>>>(
-      g, theta, reinterpret_cast<unsigned long long*>(cursor), rowoff, pat, xv);
+      g, theta, reinterpret_cast<unsigned long long*>(cursor), pat, xv);
   return cudaGetLastError();
 }
 

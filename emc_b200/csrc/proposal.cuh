@@ -146,13 +146,13 @@ struct AuditArgs {
 };
 cudaError_t launch_audit(const AuditArgs& a, int64_t n_audit, cudaStream_t st);
 // Responsibility lists of a proposed iteration (after the grouped softmax):
-// count[r] of the patterns with P >= theta T_r, then the entries
-// (pattern, value) at rowoff[r] (cursor [R] scratch); for launch_list_compress.
+// cnt[r] of the patterns with P >= theta T_r (cnt [R + 1]), room for them
+// (launch_list_alloc), then the entries (pattern, value) at cursor[r], which
+// ends at the end of the list; for launch_list_compress.
 cudaError_t launch_group_list_count(const GroupArgs& g, float theta, int64_t* cnt,
                                     cudaStream_t st);
-cudaError_t launch_group_list_fill(const GroupArgs& g, float theta, int64_t* cursor,
-                                   const int64_t* rowoff, int32_t* pat, float* xv,
-                                   cudaStream_t st);
+cudaError_t launch_group_list_fill(const GroupArgs& g, float theta, int64_t* cursor, int32_t* pat,
+                                   float* xv, cudaStream_t st);
 // FP32 responsibilities [R][N] of the last proposed iteration (zero outside
 // each pattern's candidate cells).
 cudaError_t launch_proposed_resp(const GroupArgs& g, float* P, cudaStream_t st);

@@ -256,17 +256,19 @@ cudaError_t launch_resp_write(RespArgs& a, cudaStream_t st);
 // launch_resp_rowsums with RespArgs.list_* set compacts the entries, then
 // launch_list_from_compact sorts them by rotation.
 int64_t resp_list_blocks(int64_t N);
-// rowoff[0..R] = exclusive prefix sums of rowtot (rowoff[R] = total).
-cudaError_t launch_list_rowscan(const int64_t* rowtot, int64_t R, int64_t* rowoff,
-                                cudaStream_t st);
+// Room for the lists from their counts rowtot [R] (rowtot[R]: scratch, zeroed
+// by the caller): beg[r] and cursor[r], in no particular order of rotations.
+cudaError_t launch_list_alloc(int64_t* rowtot, int64_t R, int64_t* beg, int64_t* cursor,
+                              cudaStream_t st);
 // From the entries compacted by launch_resp_rowsums (n of them): T_r, then
 // the lists sorted by rotation with x = P / (T_r phi_new), keeping entries
-// with P >= rel_min T_r (rowtot, cursor: [R] scratch; rowoff [R+1]).  Order
-// within a row is not fixed.  With n_dev the count is read on the device (n
+// with P >= rel_min T_r: rotation r's list is rowbeg[r] .. cursor[r] - 1
+// (rowtot [R + 1] scratch).  Neither the order of the lists nor that within one
+// is fixed.  With n_dev the count is read on the device (n
 // is then the capacity; a count above it leaves every list empty), so no host
 // wait is needed, as in a captured graph.
 cudaError_t launch_list_from_compact(RespArgs& a, int64_t n, float rel_min, int64_t* rowtot,
-                                     int64_t* cursor, int64_t* rowoff, int32_t* pat, float* xv,
+                                     int64_t* cursor, int64_t* rowbeg, int32_t* pat, float* xv,
                                      cudaStream_t st,
                                      const unsigned long long* n_dev = nullptr);
 // After a maximize over rotation chunks (launch_resp_rowsums per chunk with
@@ -279,7 +281,7 @@ cudaError_t launch_cand_probs(const RespArgs& a, int64_t n, float* Pv, double* T
                               cudaStream_t st);
 cudaError_t launch_list_from_candidates(RespArgs& a, int64_t n, float rel_min, float* Pv,
                                         double* T64, int64_t* rowtot, int64_t* cursor,
-                                        int64_t* rowoff, int32_t* pat, float* xv, cudaStream_t st);
+                                        int64_t* rowbeg, int32_t* pat, float* xv, cudaStream_t st);
 // Deterministic list order: the n entries (rp, v) sorted by (rotation,
 // pattern) in place (stable radix sort; rp2, v2 [n] and hist
 // [sort_hist_size(n)] scratch; N, R bound the fields) ...
@@ -324,7 +326,7 @@ cudaError_t launch_cells_out(const double* acc, int64_t count, int take_log, flo
 // in shared memory (npa floats) and inserts it as the contraction's epilogue
 // does (e.inv_c0 unused).
 struct ListCmpArgs {
-  const int64_t* rowoff;
+  const int64_t *rowbeg, *rowend;  // [R] rotation r's list is rowbeg[r] .. rowend[r] - 1
   const int32_t* pat;
   const float* xv;
   const int64_t* kptr;
