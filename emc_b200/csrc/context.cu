@@ -667,9 +667,16 @@ static emc_status alloc_work(emc_context* c) {
   }
   c->Npad = round_up(N, 128);
   c->Ppad = round_up(npa, 256);
-  // the two-SM maximize pays where the pixel extent is long (measured: 18%
-  // faster at 16,384 padded pixels, 8% slower at 4,096); emc_autotune decides
-  c->tune.maximize_pair = c->Ppad >= 8192 ? 1 : 0;
+  // the two-SM maximize: measured 1.15-1.25 times as fast per tile from 16^2
+  // to 128^2 pixels, so it is taken unless its larger tiles leave its last wave
+  // that much emptier (300 patterns x 10,860 rotations at 48^2: 86 pair tiles
+  // on 74 pairs, 0.067 ms, against 129 tiles on 148 SMs, 0.048 ms);
+  // emc_autotune re-measures
+  const int64_t nrt = round_up(R, 256) / 256;
+  auto waves = [&](int64_t tiles, int64_t units) { return (tiles + units - 1) / units; };
+  const int64_t w2 = waves((c->Npad + 255) / 256 * nrt, std::max(1, c->num_sms / 2));
+  const int64_t w1 = waves(c->Npad / 128 * nrt, c->num_sms);
+  c->tune.maximize_pair = 5 * w2 <= 6 * w1 ? 1 : 0;
   // the compress on pairs: 5% faster at 128^3 / 50k patterns (raster 2)
   c->tune.compress_pair = (c->Ppad >= 8192 && c->Npad >= 8192) ? 1 : 0;
   // the compress from responsibility lists (a handful of non-zero entries
@@ -2571,8 +2578,12 @@ static emc_status run_proposed(emc_context* c, const ProposedPlan& pl, Select se
   std::vector<int4> mt, ct;
   int64_t n_gmt = 0, n_gct = 0;
   TileDesc *gmt = nullptr, *gct = nullptr;
-  // the grouped maximize on SM pairs (256-slot tiles) where the dense one is
-  const bool gpair_form = tc && c->tune.maximize_pair;
+  // the grouped maximize on SM pairs (256-slot tiles) where the dense one is,
+  // unless the cells are nearly empty (measured: 70 to 250 slots a cell 1.2-1.3
+  // times as fast as one SM with 128-slot tiles, 12 slots a cell 0.8 times)
+  int64_t busy = 0;
+  for (int32_t k = 0; k < n_cells; ++k) busy += gcnt[k] > 0;
+  const bool gpair_form = tc && c->tune.maximize_pair && npairs >= 32 * busy;
   const int32_t gm_rows = gpair_form ? 256 : 128;
   if (tc) {
     const int64_t ptiles = (c->npa + 255) / 256;
