@@ -9,6 +9,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <functional>
+#include <queue>
 #include <string>
 #include <vector>
 
@@ -2905,6 +2907,11 @@ struct emc_batch {
   std::vector<int64_t> per_iter;  // each dataset's launches in one captured iteration
   MaxEpiArgs* d_max = nullptr;  // per-dataset epilogue arguments (fixed per context)
   CmpEpiArgs* d_cmp = nullptr;
+  // one stream per dataset for the stages between the shared launches, and the
+  // events that fork them from the batch's stream and join them to it
+  std::vector<cudaStream_t> sub;
+  std::vector<cudaEvent_t> joined;
+  cudaEvent_t forked = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   std::string err;
@@ -2930,6 +2937,59 @@ struct emc_batch {
     if (_s != EMC_OK) return (b)->fail(_s, (c)->err); \
   } while (0)
 
+// Reorders a tile list (costliest first) for persistent CTAs (or pairs) that
+// take entries i, i + units, ...: each tile goes to the least loaded unit that
+// has an entry left.  Round robin gave the units with the costliest tiles the
+// costliest of the next round too (six datasets of 48 to 128 pixels: 436
+// k-blocks on the longest unit, of a mean of 280).
+static void spread_tiles(std::vector<TileDesc>& t, int64_t units) {
+  const int64_t n = (int64_t)t.size();
+  if (units < 1 || n <= units) return;
+  constexpr int64_t kTileCost = 4;  // of a tile besides its k-blocks (epilogue, pipeline fill)
+  typedef std::pair<int64_t, int64_t> Unit;  // load, index
+  std::priority_queue<Unit, std::vector<Unit>, std::greater<Unit>> q;
+  for (int64_t u = 0; u < units; ++u) q.push({0, u});
+  std::vector<int64_t> used(units, 0);
+  std::vector<TileDesc> out(n);
+  for (const TileDesc& d : t) {
+    const Unit x = q.top();
+    q.pop();
+    const int64_t u = x.second;
+    out[used[u]++ * units + u] = d;
+    // entries of unit u: u, u + units, ... below n
+    if (used[u] * units + u < n) q.push({x.first + d.k_blocks + kTileCost, u});
+  }
+  t.swap(out);
+}
+
+// Runs f(i) for every dataset that `take` selects, each on a stream of its own
+// between a fork from the batch's stream and a join to it: the stages between
+// the shared launches are many small kernels per dataset, which leave most of
+// the GPU idle one after the other (six datasets of 500 patterns x 3,240
+// rotations: 1.92 ms per iteration in sequence, 1.45 ms forked and with the
+// tiles spread as above).
+template <class Take, class F>
+static emc_status each_dataset(emc_batch* b, Take take, F f) {
+  std::vector<int> set;
+  for (int i = 0; i < (int)b->ctx.size(); ++i)
+    if (take(i)) set.push_back(i);
+  if (set.size() == 1) return f(set[0]);
+  BCK(b, cudaEventRecord(b->forked, b->st));
+  emc_status first = EMC_OK;
+  for (int i : set) {
+    // every fork is joined, also after an error: a capture ends only then
+    emc_context* c = b->ctx[i];
+    BCK(b, cudaStreamWaitEvent(b->sub[i], b->forked, 0));
+    c->st = b->sub[i];
+    const emc_status s = first == EMC_OK ? f(i) : EMC_OK;
+    c->st = b->st;
+    if (s != EMC_OK) first = s;
+    BCK(b, cudaEventRecord(b->joined[i], b->sub[i]));
+    BCK(b, cudaStreamWaitEvent(b->st, b->joined[i], 0));
+  }
+  return first;
+}
+
 // Dataset i's stages of a batched iteration that are not shared launches.
 // The maximize contraction of a dataset with its own launches.
 static emc_status batch_own_maximize(emc_batch* b, int i) {
@@ -2937,10 +2997,10 @@ static emc_status batch_own_maximize(emc_batch* b, int i) {
   const MaxEpiArgs e = max_args(c);
   if (c->tune.maximize_pair)
     BCK(b, launch_maximize_pair_tc(c->tmKh64, c->tmBhi64, c->tmBlo64, c->Npad, c->Rpad, c->Ppad, e,
-                                   c->d_status, c->num_sms, b->st, c->tune.maximize_raster));
+                                   c->d_status, c->num_sms, c->st, c->tune.maximize_raster));
   else
     BCK(b, launch_maximize_tc(c->tmKh, c->tmBhi, c->tmBlo, c->Npad, c->Rpad, c->Ppad, e,
-                              c->d_status, c->num_sms, b->st, c->tune.maximize_raster));
+                              c->d_status, c->num_sms, c->st, c->tune.maximize_raster));
   c->launches += 1;
   return EMC_OK;
 }
@@ -2951,7 +3011,7 @@ static emc_status batch_resp(emc_batch* b, int i) {
   emc_context* c = b->ctx[i];
   BTRY(b, c, b->lists[i] ? gated_list_pass(c) : mixed_resp_pass(c, false));
   BCK(b, cudaMemcpyAsync(c->d_Tskip, c->d_T, sizeof(float) * c->R, cudaMemcpyDeviceToDevice,
-                         b->st));
+                         c->st));
   c->resp_source = 1;
   c->stage = 2;
   BTRY(b, c, clear_acc(c));
@@ -2977,17 +3037,17 @@ static emc_status batch_own_compress(emc_batch* b, int i) {
     la.e = e;
     la.gate_count = c->d_lcount;
     la.gate_cap = c->lcomp_cap;
-    BCK(b, launch_list_compress(la, b->st));
+    BCK(b, launch_list_compress(la, c->st));
     e.gate_count = c->d_lcount;
     e.gate_cap = c->lcomp_cap;
     c->launches += 1;
   }
   if (c->tune.compress_pair)
     BCK(b, launch_compress_pair_tc(c->tmPhi, c->tmPlo, c->tmKt128, c->Rpad, c->Ppad, c->Npad, e,
-                                   c->d_status, c->num_sms, b->st, c->tune.compress_raster));
+                                   c->d_status, c->num_sms, c->st, c->tune.compress_raster));
   else
     BCK(b, launch_compress_tc(c->tmPhi, c->tmPlo, c->tmKt, c->Rpad, c->Ppad, c->Npad, e,
-                              c->d_status, c->num_sms, b->st, c->tune.compress_raster));
+                              c->d_status, c->num_sms, c->st, c->tune.compress_raster));
   c->launches += 1;
   return EMC_OK;
 }
@@ -2997,6 +3057,11 @@ extern "C" {
 emc_status emc_batch_destroy(emc_batch* b) {
   if (!b) return EMC_OK;
   if (b->st) cudaStreamSynchronize(b->st);
+  for (cudaStream_t q : b->sub)
+    if (q) cudaStreamDestroy(q);
+  for (cudaEvent_t q : b->joined)
+    if (q) cudaEventDestroy(q);
+  if (b->forked) cudaEventDestroy(b->forked);
   for (size_t i = 0; i < b->ctx.size(); ++i) {
     b->ctx[i]->st = b->own[i];
     b->ctx[i]->batched = false;
@@ -3031,6 +3096,16 @@ emc_status emc_batch_create(emc_context* const* ctxs, int32_t n, emc_batch** out
   emc_batch* b = new emc_batch();
   if (cudaSetDevice(dev) != cudaSuccess ||
       cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking) != cudaSuccess) {
+    emc_batch_destroy(b);
+    return EMC_ERR_CUDA;
+  }
+  b->sub.assign(n, nullptr);
+  b->joined.assign(n, nullptr);
+  bool ok = cudaEventCreateWithFlags(&b->forked, cudaEventDisableTiming) == cudaSuccess;
+  for (int32_t i = 0; i < n && ok; ++i)
+    ok = cudaStreamCreateWithFlags(&b->sub[i], cudaStreamNonBlocking) == cudaSuccess &&
+         cudaEventCreateWithFlags(&b->joined[i], cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) {
     emc_batch_destroy(b);
     return EMC_ERR_CUDA;
   }
@@ -3108,6 +3183,7 @@ emc_status emc_batch_create(emc_context* const* ctxs, int32_t n, emc_batch** out
                               (int32_t)(c->Ppad / kMaximizeBK), (int32_t)nt, (int32_t)m, i});
       });
   }
+  spread_tiles(mt, b->pair ? ctxs[0]->num_sms / 2 : ctxs[0]->num_sms);
   std::stable_sort(order.begin(), order.end(),
                    [&](int32_t x, int32_t y) { return ctxs[x]->Npad > ctxs[y]->Npad; });
   double cwork_pair = 0.0;
@@ -3194,13 +3270,15 @@ emc_status emc_batch_iterate(emc_batch* b) {
   me.set = b->d_max;
   ce.tiles = b->d_ct;
   ce.set = b->d_cmp;
-  for (int i = 0; i < n; ++i) {
-    if (b->alone[i]) continue;
+  auto shared = [&](int i) { return !b->alone[i]; };
+  emc_status s = each_dataset(b, shared, [&](int i) -> emc_status {
     emc_context* c = b->ctx[i];
     BTRY(b, c, emc_expand(c));
     BCK(b, cudaMemcpyAsync(c->d_scaling_prev, c->d_scaling, sizeof(float) * c->N,
-                           cudaMemcpyDeviceToDevice, b->st));
-  }
+                           cudaMemcpyDeviceToDevice, c->st));
+    return EMC_OK;
+  });
+  if (s != EMC_OK) return s;
   for (int i = 0; i < kMaxBatch; ++i) {
     const emc_context* c = b->ctx[i < n && !b->alone[i] ? i : first];
     maps.a0[i] = b->pair ? c->tmKh64 : c->tmKh;
@@ -3213,38 +3291,37 @@ emc_status emc_batch_iterate(emc_batch* b) {
   else
     BCK(b, launch_batch_maximize_tc(maps, b->n_mt, me, c0->d_status, c0->num_sms, b->st));
   c0->launches += 1;
-  for (int i = 0; i < n; ++i) {
-    if (b->alone[i]) continue;
-    const emc_status s = batch_resp(b, i);
-    if (s != EMC_OK) return s;
-  }
-  if (b->n_ct) {
-    for (int i = 0; i < kMaxBatch; ++i) {
-      const emc_context* c = b->ctx[i < n && !b->alone[i] ? i : first];
-      maps.a0[i] = c->tmPhi;
-      maps.a1[i] = c->tmPlo;
-      maps.b0[i] = b->cmp_pair ? c->tmKt128 : c->tmKt;
-      maps.b1[i] = maps.b0[i];
-    }
-    if (b->cmp_pair)
-      BCK(b, launch_batch_compress_pair_tc(maps, b->n_ct, ce, c0->d_status, c0->num_sms, b->st));
-    else
-      BCK(b, launch_batch_compress_tc(maps, b->n_ct, ce, c0->d_status, c0->num_sms, b->st));
-    c0->launches += 1;
-  }
-  for (int i = 0; i < n; ++i) {
-    if (b->alone[i] || !b->lists[i]) continue;
-    const emc_status s = batch_own_compress(b, i);
-    if (s != EMC_OK) return s;
-  }
-  for (int i = 0; i < n; ++i) {
-    if (b->alone[i]) continue;
+  auto finish = [&](int i) -> emc_status {
     emc_context* c = b->ctx[i];
     BTRY(b, c, merge_acc(c));
     c->stage = 3;
     BTRY(b, c, emc_normalize(c));
+    return EMC_OK;
+  };
+  // a dataset with lists goes through to its new model on its own; the others
+  // meet in the batched compress
+  s = each_dataset(b, shared, [&](int i) -> emc_status {
+    emc_status r = batch_resp(b, i);
+    if (r == EMC_OK && b->lists[i]) {
+      r = batch_own_compress(b, i);
+      if (r == EMC_OK) r = finish(i);
+    }
+    return r;
+  });
+  if (s != EMC_OK || !b->n_ct) return s;
+  for (int i = 0; i < kMaxBatch; ++i) {
+    const emc_context* c = b->ctx[i < n && !b->alone[i] ? i : first];
+    maps.a0[i] = c->tmPhi;
+    maps.a1[i] = c->tmPlo;
+    maps.b0[i] = b->cmp_pair ? c->tmKt128 : c->tmKt;
+    maps.b1[i] = maps.b0[i];
   }
-  return EMC_OK;
+  if (b->cmp_pair)
+    BCK(b, launch_batch_compress_pair_tc(maps, b->n_ct, ce, c0->d_status, c0->num_sms, b->st));
+  else
+    BCK(b, launch_batch_compress_tc(maps, b->n_ct, ce, c0->d_status, c0->num_sms, b->st));
+  c0->launches += 1;
+  return each_dataset(b, [&](int i) { return shared(i) && !b->lists[i]; }, finish);
 }
 
 emc_status emc_batch_capture(emc_batch* b) {
