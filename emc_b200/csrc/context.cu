@@ -273,7 +273,12 @@ struct emc_context {
   int32_t* d_lpat = nullptr;
   float* d_lx = nullptr;
   int64_t lcap = 0, lcap_x = 0, list_nnz = 0;
-  bool list_mode = false;  // this iteration's compress reads the lists
+  // this iteration's compress: the dense operand, the lists, or both gated on
+  // the count of compacted entries (lists up to list_gate of them)
+  enum { CMP_DENSE, CMP_LISTS, CMP_GATED } cmp_mode = CMP_DENSE;
+  int64_t list_gate = 0;
+  cudaEvent_t ev_count = nullptr;  // that count has reached hpin[8]
+  bool count_pending = false;
   GroupArgs last_group{};     // arguments of the last grouped iteration (responsibility export)
   // dense audit of sampled patterns in a proposed iteration
   int64_t* d_aud_pat = nullptr;
@@ -312,9 +317,34 @@ struct emc_context {
     cudaEventRecord(ev[cur][i], st);
   }
 
+  // One iteration as a CUDA graph (iterate_graph): what it was captured for,
+  // and how often in a row iterations have found the same.
+  struct GraphKey {
+    emc_tuning tune;
+    cudaStream_t st;
+    int64_t version, y_rows, gate;
+    int32_t planes, csr, csc;
+    bool operator==(const GraphKey& o) const {
+      return std::memcmp(&tune, &o.tune, sizeof(tune)) == 0 && st == o.st &&
+             version == o.version && y_rows == o.y_rows && gate == o.gate &&
+             planes == o.planes && csr == o.csr && csc == o.csc;
+    }
+  };
+  GraphKey graph_key{};
+  int graph_seen = 0;
+  bool graph_off = false;   // a capture failed: iterations stay eager
+  bool capturing = false;
+  cudaGraphExec_t graph_exec = nullptr;
+  int64_t graph_launches = 0;
+  int64_t version = 0;      // allocations and releases so far
+  // uploads from the caller's memory that may still be in flight
+  cudaEvent_t ev_upload = nullptr;
+  bool upload_pending = false;
+
   // pinned host staging of the proposed iteration, reused between calls
-  void* hpin[8] = {nullptr};
-  size_t hcap[8] = {0};
+  // [8]: the count of compacted entries (ev_count); [9], [10]: read_back
+  void* hpin[11] = {nullptr};
+  size_t hcap[11] = {0};
   template <class T>
   T* pinned(int slot, size_t n) {
     const size_t bytes = n * sizeof(T) + 16;
@@ -359,6 +389,7 @@ struct emc_context {
       e = cudaMalloc(&q, bytes);
     }
     if (e != cudaSuccess) return cuda(e, "cudaMalloc");
+    ++version;
     allocs.push_back(q);
     alloc_bytes.push_back(bytes);
     mem_used += bytes;
@@ -370,6 +401,7 @@ struct emc_context {
     return EMC_OK;
   }
   void release(void* p) {
+    ++version;
     for (size_t k = 0; k < allocs.size(); ++k)
       if (allocs[k] == p) {
         cudaFree(allocs[k]);
@@ -495,6 +527,9 @@ emc_status emc_destroy(emc_context* ctx) {
   for (void* h : ctx->hpin)
     if (h) cudaFreeHost(h);
   if (ctx->ev_sel) cudaEventDestroy(ctx->ev_sel);
+  if (ctx->ev_count) cudaEventDestroy(ctx->ev_count);
+  if (ctx->ev_upload) cudaEventDestroy(ctx->ev_upload);
+  if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
   if (ctx->ev_audit) cudaEventDestroy(ctx->ev_audit);
   if (ctx->st) cudaStreamDestroy(ctx->st);
   delete ctx;
@@ -795,6 +830,8 @@ emc_status emc_set_geometry(emc_context* c, const float* x, const float* y, cons
   return EMC_OK;
 }
 
+static emc_status upload_enqueued(emc_context* c);
+
 emc_status emc_set_rotations(emc_context* c, const float* q, const float* w) {
   if (!c || !q || !w) return EMC_ERR_ARG;
   if (count_bad(q, 4 * c->R, false) || count_bad(w, c->R, true))
@@ -802,7 +839,23 @@ emc_status emc_set_rotations(emc_context* c, const float* q, const float* w) {
   CK(c, cudaMemcpyAsync(c->d_quat, q, sizeof(float) * 4 * c->R, cudaMemcpyHostToDevice, c->st));
   CK(c, cudaMemcpyAsync(c->d_rotw, w, sizeof(float) * c->R, cudaMemcpyHostToDevice, c->st));
   c->have_rot = true;
+  return upload_enqueued(c);
+}
+
+// Uploads of models, scalings and rotations are enqueued, and their source may
+// be pinned memory that the copy reads later.  An iteration of a mixed context
+// returns only once they have been read, as it always has.
+static emc_status upload_enqueued(emc_context* c) {
+  if (!c->mixed) return EMC_OK;
+  if (!c->ev_upload) CK(c, cudaEventCreateWithFlags(&c->ev_upload, cudaEventDisableTiming));
+  CK(c, cudaEventRecord(c->ev_upload, c->st));
+  c->upload_pending = true;
   return EMC_OK;
+}
+static emc_status uploads_read(emc_context* c) {
+  if (!c->upload_pending || c->capturing) return EMC_OK;
+  c->upload_pending = false;
+  return c->cuda(cudaEventSynchronize(c->ev_upload), "uploads");
 }
 
 static emc_status finish_patterns(emc_context* c);
@@ -977,7 +1030,7 @@ emc_status emc_set_model(emc_context* c, const float* model) {
   CK(c, cudaMemcpyAsync(c->d_model, model, sizeof(float) * c->M, cudaMemcpyHostToDevice, c->st));
   c->have_model = true;
   c->stage = 0;
-  return EMC_OK;
+  return upload_enqueued(c);
 }
 
 emc_status emc_set_scaling(emc_context* c, const float* scaling) {
@@ -987,7 +1040,7 @@ emc_status emc_set_scaling(emc_context* c, const float* scaling) {
       return c->fail(EMC_ERR_RANGE, "scaling of pattern %lld is not a finite positive number",
                      (long long)p);
   CK(c, cudaMemcpyAsync(c->d_scaling, scaling, sizeof(float) * c->N, cudaMemcpyHostToDevice, c->st));
-  return EMC_OK;
+  return upload_enqueued(c);
 }
 
 static double gauss_inv(const emc_context* c) {
@@ -1188,78 +1241,15 @@ static int64_t list_worth(const emc_context* c) {
   return (int64_t)std::min(dense * 6.4e11 / std::max(photons, 1.0), 9e15);
 }
 
-static emc_status mixed_resp_pass(emc_context* c, bool allow_lists = true) {
+// The deterministic lists: the host reads the entries' count (one wait), since
+// the sort's launches depend on it.
+static emc_status det_resp_pass(emc_context* c) {
   const int64_t N = c->N;
   RespArgs a = resp_args(c);
-  c->list_mode = false;
-  if (allow_lists && c->tune.compress_sparse && c->npa <= kListMaxPixels) {
-    // the compress operand as per-rotation lists of its non-zero entries:
-    // entries P >= kListMinP are compacted during the row-sum sweep, the host
-    // reads their count (one wait), a counting sort orders them by rotation
-    TRY(list_buffers(c));
-    if (!c->csr.valid) TRY(build_rows(c, c->d_K, N, c->npa, c->csr, false));
-    const int64_t worth = std::max<int64_t>(list_worth(c), 64 * N);
-    TRY(compact_capacity(c, std::max<int64_t>(64 * N, (int64_t)1 << 20)));
-    CK(c, cudaMemsetAsync(c->d_lcount, 0, sizeof(unsigned long long), c->st));
-    a.list_count = c->d_lcount;
-    a.list_cap = c->lcomp_cap;
-    a.list_rp = c->d_lcomp_rp;
-    a.list_P = c->d_lcomp_P;
-    a.list_min = kListMinP;
-    CK(c, launch_resp_rowsums(a, c->st));
-    unsigned long long* hn = c->pinned<unsigned long long>(7, 1);
-    if (!hn) return c->fail(EMC_ERR_OOM, "pinned host staging");
-    CK(c, cudaMemcpyAsync(hn, c->d_lcount, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                          c->st));
-    CK(c, cudaStreamSynchronize(c->st));
-    c->list_nnz = (int64_t)*hn;
-    if (c->list_nnz <= std::min(worth, c->lcomp_cap)) {
-      TRY(grow(c, &c->d_lpat, c->lcap, c->list_nnz + 1));
-      int64_t cap = c->lcap_x;
-      TRY(grow(c, &c->d_lx, cap, c->list_nnz + 1));
-      c->lcap_x = cap;
-      if (c->det) {
-        // the entries in (rotation, pattern) order, so the lists do not
-        // depend on the order the sweep appended them
-        TRY(sort_scratch(c, c->list_nnz));
-        CK(c, launch_finish_T(c->d_Tpart, N, c->R, c->d_T, c->st));
-        CK(c, launch_sort_entries(c->d_lcomp_rp, c->d_lcomp_P, c->list_nnz, N, c->R,
-                                  c->d_sort_rp, c->d_sort_v, c->d_sort_hist, c->st));
-        CK(c, launch_list_from_sorted(c->d_lcomp_rp, c->d_lcomp_P, c->list_nnz, c->R, c->d_T,
-                                      c->d_scaling, kListRel, c->d_lrowtot, c->d_lrowoff,
-                                      c->d_sort_flag, c->d_lpat, c->d_lx, c->st));
-      } else {
-        CK(c, launch_list_from_compact(a, c->list_nnz, kListRel, c->d_lrowtot, c->d_lcursor,
-                                       c->d_lrowoff, c->d_lpat, c->d_lx, c->st));
-      }
-      c->list_mode = true;
-      c->launches += 6;  // combine, row sums, T, count, room, fill
-    } else {
-      // more entries than the compaction holds: the dense operand this time,
-      // room for them next time if they are worth it
-      CK(c, launch_resp_write(a, c->st));
-      if (c->list_nnz <= worth) TRY(compact_capacity(c, c->list_nnz));
-      c->launches += 3;
-    }
-  } else {
-    CK(c, launch_resp_pass(a, c->st));
-    c->launches += 3;  // combine, 2 sweeps
-  }
-  CK(c, launch_sum2_f64(c->d_plogp, c->d_lse, N, c->d_stats + 2, c->st));
-  c->launches += 1;
-  return EMC_OK;
-}
-
-// The responsibility pass of a batched dataset with lists, in a form a CUDA
-// graph can hold: the count of compacted entries stays on the device, the
-// lists are built from it when it fits the compaction's capacity, and the
-// dense compress operand is written only when it does not (write_kernel
-// gated on the count), so the compress then runs from the lists or, gated
-// the other way, as the dense contraction.  No host wait and no allocation:
-// batch_lists_ready sized every buffer when the batch was made.
-static emc_status gated_list_pass(emc_context* c) {
-  RespArgs a = resp_args(c);
-  c->list_mode = false;
+  TRY(list_buffers(c));
+  if (!c->csr.valid) TRY(build_rows(c, c->d_K, N, c->npa, c->csr, false));
+  const int64_t worth = std::max<int64_t>(list_worth(c), 64 * N);
+  TRY(compact_capacity(c, std::max<int64_t>(64 * N, (int64_t)1 << 20)));
   CK(c, cudaMemsetAsync(c->d_lcount, 0, sizeof(unsigned long long), c->st));
   a.list_count = c->d_lcount;
   a.list_cap = c->lcomp_cap;
@@ -1267,10 +1257,113 @@ static emc_status gated_list_pass(emc_context* c) {
   a.list_P = c->d_lcomp_P;
   a.list_min = kListMinP;
   CK(c, launch_resp_rowsums(a, c->st));
-  CK(c, launch_list_from_compact(a, c->lcomp_cap, kListRel, c->d_lrowtot, c->d_lcursor,
+  unsigned long long* hn = c->pinned<unsigned long long>(7, 1);
+  if (!hn) return c->fail(EMC_ERR_OOM, "pinned host staging");
+  c->count_pending = false;
+  CK(c, cudaMemcpyAsync(hn, c->d_lcount, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                        c->st));
+  CK(c, cudaStreamSynchronize(c->st));
+  c->list_nnz = (int64_t)*hn;
+  if (c->list_nnz <= std::min(worth, c->lcomp_cap)) {
+    TRY(grow(c, &c->d_lpat, c->lcap, c->list_nnz + 1));
+    int64_t cap = c->lcap_x;
+    TRY(grow(c, &c->d_lx, cap, c->list_nnz + 1));
+    c->lcap_x = cap;
+    // the entries in (rotation, pattern) order, so the lists do not depend on
+    // the order the sweep appended them
+    TRY(sort_scratch(c, c->list_nnz));
+    CK(c, launch_finish_T(c->d_Tpart, N, c->R, c->d_T, c->st));
+    CK(c, launch_sort_entries(c->d_lcomp_rp, c->d_lcomp_P, c->list_nnz, N, c->R, c->d_sort_rp,
+                              c->d_sort_v, c->d_sort_hist, c->st));
+    CK(c, launch_list_from_sorted(c->d_lcomp_rp, c->d_lcomp_P, c->list_nnz, c->R, c->d_T,
+                                  c->d_scaling, kListRel, c->d_lrowtot, c->d_lrowoff,
+                                  c->d_sort_flag, c->d_lpat, c->d_lx, c->st));
+    c->cmp_mode = emc_context::CMP_LISTS;
+    c->launches += 6;  // combine, row sums, T, sort, count, place
+  } else {
+    // more entries than the compaction holds: the dense operand this time,
+    // room for them next time if they are worth it
+    CK(c, launch_resp_write(a, c->st));
+    if (c->list_nnz <= worth) TRY(compact_capacity(c, c->list_nnz));
+    c->launches += 3;
+  }
+  CK(c, launch_sum2_f64(c->d_plogp, c->d_lse, N, c->d_stats + 2, c->st));
+  c->launches += 1;
+  return EMC_OK;
+}
+
+static emc_status gated_list_pass(emc_context* c);
+static emc_status batch_lists_ready(emc_context* c, int64_t entries);
+
+static bool uses_lists(const emc_context* c) {
+  return c->mixed && c->tune.compress_sparse && c->npa <= kListMaxPixels;
+}
+
+// The entries' count stays on the device and gates the lists and the dense
+// operand, so the host does not wait in the middle of an iteration.  Before a
+// pass it reads the count of an earlier one, if that has arrived, and makes
+// room for that many entries where lists of that length would be the faster
+// form; after a pass it has the count copied back.
+static emc_status list_room(emc_context* c) {
+  int64_t want = std::max<int64_t>({64 * c->N, (int64_t)1 << 20, c->lcomp_cap});
+  if (c->count_pending && cudaEventQuery(c->ev_count) == cudaSuccess) {
+    c->count_pending = false;
+    c->list_nnz = (int64_t)*c->pinned<unsigned long long>(8, 1);
+    if (c->csr.valid && c->list_nnz <= std::max<int64_t>(list_worth(c), 64 * c->N))
+      want = std::max(want, c->list_nnz);
+  }
+  return batch_lists_ready(c, want);
+}
+static emc_status list_count_back(emc_context* c) {
+  if (c->count_pending) return EMC_OK;
+  unsigned long long* hn = c->pinned<unsigned long long>(8, 1);
+  if (!hn) return c->fail(EMC_ERR_OOM, "pinned host staging");
+  if (!c->ev_count) CK(c, cudaEventCreateWithFlags(&c->ev_count, cudaEventDisableTiming));
+  CK(c, cudaMemcpyAsync(hn, c->d_lcount, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                        c->st));
+  CK(c, cudaEventRecord(c->ev_count, c->st));
+  c->count_pending = true;
+  return EMC_OK;
+}
+
+static emc_status mixed_resp_pass(emc_context* c, bool allow_lists = true) {
+  c->cmp_mode = emc_context::CMP_DENSE;
+  if (allow_lists && uses_lists(c)) {
+    // the compress operand as per-rotation lists of its non-zero entries
+    if (c->det) return det_resp_pass(c);
+    if (!c->capturing) TRY(list_room(c));
+    TRY(gated_list_pass(c));
+    c->cmp_mode = emc_context::CMP_GATED;
+    return c->capturing ? EMC_OK : list_count_back(c);
+  }
+  RespArgs a = resp_args(c);
+  CK(c, launch_resp_pass(a, c->st));
+  CK(c, launch_sum2_f64(c->d_plogp, c->d_lse, c->N, c->d_stats + 2, c->st));
+  c->launches += 4;  // combine, 2 sweeps, sums
+  return EMC_OK;
+}
+
+// The responsibility pass with lists, in a form a CUDA graph can hold: the
+// count of compacted entries stays on the device, the lists are built from it
+// when it is within list_gate (what the buffers hold, and what is worth it),
+// and the dense compress operand is written only when it is not (write_kernel
+// gated on the count), so the compress then runs from the lists or, gated the
+// other way, as the dense contraction.  No host wait and no allocation:
+// batch_lists_ready sized every buffer.
+static emc_status gated_list_pass(emc_context* c) {
+  RespArgs a = resp_args(c);
+  c->list_gate = std::min(std::max<int64_t>(list_worth(c), 64 * c->N), c->lcomp_cap);
+  CK(c, cudaMemsetAsync(c->d_lcount, 0, sizeof(unsigned long long), c->st));
+  a.list_count = c->d_lcount;
+  a.list_cap = c->lcomp_cap;
+  a.list_rp = c->d_lcomp_rp;
+  a.list_P = c->d_lcomp_P;
+  a.list_min = kListMinP;
+  CK(c, launch_resp_rowsums(a, c->st));
+  CK(c, launch_list_from_compact(a, c->list_gate, kListRel, c->d_lrowtot, c->d_lcursor,
                                  c->d_lrowoff, c->d_lpat, c->d_lx, c->st, c->d_lcount));
   a.gate_count = c->d_lcount;
-  a.gate_cap = c->lcomp_cap;
+  a.gate_cap = c->list_gate;
   CK(c, launch_resp_write(a, c->st));
   CK(c, launch_sum2_f64(c->d_plogp, c->d_lse, c->N, c->d_stats + 2, c->st));
   c->launches += 8;  // combine, row sums, T, count, room, fill, write, sums
@@ -1382,7 +1475,7 @@ static emc_status chunked_maximize(emc_context* c) {
                                       c->d_lrowtot, c->d_lcursor, c->d_lrowoff, c->d_lpat,
                                       c->d_lx, c->st));
   }
-  c->list_mode = true;
+  c->cmp_mode = emc_context::CMP_LISTS;
   CK(c, launch_sum2_f64(c->d_plogp, c->d_lse, N, c->d_stats + 2, c->st));
   c->launches += 6;  // finish, T, count, room, fill, sums
   return EMC_OK;
@@ -1628,7 +1721,7 @@ emc_status emc_maximize(emc_context* c) {
   c->mark(3);
   c->resp_source = c->mixed && c->y_rows < R ? 3 : 1;
   c->stage = 2;
-  return EMC_OK;
+  return uploads_read(c);
 }
 
 emc_status emc_compress_insert(emc_context* c) {
@@ -1686,7 +1779,8 @@ emc_status emc_compress_insert(emc_context* c) {
     c->launches += 1;
   } else {
     CmpEpiArgs e = cmp_args(c);
-    if (c->list_mode) {
+    const bool gated = c->cmp_mode == emc_context::CMP_GATED;
+    if (c->cmp_mode != emc_context::CMP_DENSE) {
       // responsibility lists x the counts' photon lists (built once per upload)
       if (!c->csr.valid) TRY(build_rows(c, c->d_K, c->N, c->npa, c->csr, false));
       ListCmpArgs la{};
@@ -1699,15 +1793,22 @@ emc_status emc_compress_insert(emc_context* c) {
       la.kval = c->csr.val;
       la.e = e;
       la.ordered = c->det ? 1 : 0;
+      la.gate_count = gated ? c->d_lcount : nullptr;
+      la.gate_cap = c->list_gate;
       CK(c, launch_list_compress(la, c->st));
-    } else if (c->tune.compress_pair) {
-      CK(c, launch_compress_pair_tc(c->tmPhi, c->tmPlo, c->tmKt128, c->Rpad, c->Ppad, c->Npad, e,
-                                    c->d_status, c->num_sms, c->st, c->tune.compress_raster));
-    } else {
-      CK(c, launch_compress_tc(c->tmPhi, c->tmPlo, c->tmKt, c->Rpad, c->Ppad, c->Npad, e,
-                               c->d_status, c->num_sms, c->st, c->tune.compress_raster));
+      c->launches += 1;
     }
-    c->launches += 1;
+    if (c->cmp_mode != emc_context::CMP_LISTS) {
+      e.gate_count = gated ? c->d_lcount : nullptr;
+      e.gate_cap = c->list_gate;
+      if (c->tune.compress_pair)
+        CK(c, launch_compress_pair_tc(c->tmPhi, c->tmPlo, c->tmKt128, c->Rpad, c->Ppad, c->Npad, e,
+                                      c->d_status, c->num_sms, c->st, c->tune.compress_raster));
+      else
+        CK(c, launch_compress_tc(c->tmPhi, c->tmPlo, c->tmKt, c->Rpad, c->Ppad, c->Npad, e,
+                                 c->d_status, c->num_sms, c->st, c->tune.compress_raster));
+      c->launches += 1;
+    }
     if (!c->det) TRY(merge_acc(c));
   }
   if (c->det) {
@@ -1746,18 +1847,34 @@ emc_status emc_compress(emc_context* c) {
   return emc_normalize(c);
 }
 
-static emc_status check_status(emc_context* c) {
-  TcStatus h{};
-  CK(c, cudaMemcpyAsync(&h, c->d_status, sizeof(h), cudaMemcpyDeviceToHost, c->st));
+// What a waited-for call reads back: the status word of the device-side waits
+// and, with stats, the statistics and T_r, in pinned memory behind one wait.
+struct HostBack {
+  TcStatus status;
+  double stats[4];
+};
+static emc_status read_back(emc_context* c, HostBack** out, float** T) {
+  HostBack* h = c->pinned<HostBack>(9, 1);
+  float* t = T ? c->pinned<float>(10, c->R) : nullptr;
+  if (!h || (T && !t)) return c->fail(EMC_ERR_OOM, "pinned host staging");
+  CK(c, cudaMemcpyAsync(&h->status, c->d_status, sizeof(TcStatus), cudaMemcpyDeviceToHost, c->st));
+  if (T) {
+    CK(c, cudaMemcpyAsync(h->stats, c->d_stats, sizeof(h->stats), cudaMemcpyDeviceToHost, c->st));
+    CK(c, cudaMemcpyAsync(t, c->d_T, sizeof(float) * c->R, cudaMemcpyDeviceToHost, c->st));
+    *T = t;
+  }
   CK(c, cudaStreamSynchronize(c->st));
-  if (h.code != 0) {
+  if (out) *out = h;
+  if (h->status.code != 0) {
+    const TcStatus s = h->status;
     cudaMemsetAsync(c->d_status, 0, sizeof(TcStatus), c->st);
     cudaStreamSynchronize(c->st);
-    return c->fail(EMC_ERR_TIMEOUT, "tensor-core kernel wait %d timed out in block %d", h.where,
-                   h.block);
+    return c->fail(EMC_ERR_TIMEOUT, "tensor-core kernel wait %d timed out in block %d", s.where,
+                   s.block);
   }
   return EMC_OK;
 }
+static emc_status check_status(emc_context* c) { return read_back(c, nullptr, nullptr); }
 
 emc_status emc_synchronize(emc_context* c) {
   if (!c) return EMC_ERR_ARG;
@@ -1772,21 +1889,102 @@ emc_status emc_wait_probe(emc_context* c, uint32_t limit_us) {
   return check_status(c);
 }
 
-emc_status emc_iterate(emc_context* c, emc_iter_stats* stats) {
+static emc_status iterate_stages(emc_context* c) {
   TRY(emc_expand(c));
   TRY(emc_maximize(c));
-  TRY(emc_compress(c));
+  return emc_compress(c);
+}
+
+// One iteration through a CUDA graph of its launches.  Small problems are
+// bound by them (16^3, 64 patterns x 420 rotations: @G0 us launched one by
+// one, @G1 us as a graph).  The graph is captured at the third iteration in a
+// row that finds the same buffers and tuning, so a context that iterates once
+// or twice never pays for it, and it holds the same launches: nothing in it
+// depends on values.  Rotation chunks, the deterministic sort, profiling,
+// batches and a caller's own capture keep the separate launches.
+static emc_context::GraphKey graph_key(const emc_context* c) {
+  emc_context::GraphKey k{};
+  k.tune = c->tune;
+  k.st = c->st;
+  k.version = c->version;
+  k.y_rows = c->y_rows;
+  k.planes = c->i8_planes;
+  k.csr = c->csr.valid;
+  k.csc = c->csc.valid;
+  if (uses_lists(c) && c->csr.valid)
+    k.gate = std::min(std::max<int64_t>(list_worth(c), 64 * c->N), c->lcomp_cap);
+  return k;
+}
+
+static emc_status iterate_graph(emc_context* c, bool* done) {
+  *done = false;
+  if (c->graph_off || c->prof || c->batched || c->det || (c->mixed && c->y_rows < c->R) ||
+      c->stage != 0 || !c->have_geom || !c->have_rot || !c->have_pat || !c->have_model)
+    return EMC_OK;
+  cudaStreamCaptureStatus busy = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->st, &busy) != cudaSuccess || busy != cudaStreamCaptureStatusNone)
+    return EMC_OK;
+  if (c->graph_seen > 0 && uses_lists(c)) TRY(list_room(c));
+  const emc_context::GraphKey k = graph_key(c);
+  if (!(c->graph_seen > 0 && k == c->graph_key)) {
+    if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
+    c->graph_exec = nullptr;
+    c->graph_seen = 0;
+  }
+  if (!c->graph_exec) {
+    if (c->graph_seen < 2) return EMC_OK;
+    const int64_t l0 = c->launches;
+    const std::string err = c->err;
+    c->capturing = true;
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+      const emc_status s = iterate_stages(c);
+      e = cudaStreamEndCapture(c->st, &g);
+      if (e == cudaSuccess && s != EMC_OK) e = cudaErrorUnknown;
+    }
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&c->graph_exec, g, 0);
+    if (g) cudaGraphDestroy(g);
+    c->capturing = false;
+    c->stage = 0;
+    c->graph_launches = c->launches - l0;
+    c->launches = l0;
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      c->graph_exec = nullptr;
+      c->graph_off = true;
+      c->err = err;
+      return EMC_OK;
+    }
+  }
+  CK(c, cudaGraphLaunch(c->graph_exec, c->st));
+  c->launches += c->graph_launches;
+  c->resp_source = 1;
+  if (uses_lists(c)) TRY(list_count_back(c));
+  *done = true;
+  return uploads_read(c);
+}
+
+emc_status emc_iterate(emc_context* c, emc_iter_stats* stats) {
+  if (!c) return EMC_ERR_ARG;
+  bool done = false;
+  TRY(iterate_graph(c, &done));
+  if (!done) {
+    TRY(iterate_stages(c));
+    // the same buffers and tuning as the iteration before?
+    const emc_context::GraphKey k = graph_key(c);
+    c->graph_seen = c->graph_seen > 0 && k == c->graph_key ? c->graph_seen + 1 : 1;
+    c->graph_key = k;
+  }
   if (stats) {
-    TRY(check_status(c));
-    double h[4] = {0, 0, 0, 0};
-    CK(c, cudaMemcpy(h, c->d_stats, sizeof(h), cudaMemcpyDeviceToHost));
+    HostBack* h = nullptr;
+    float* t = nullptr;
+    TRY(read_back(c, &h, &t));
     double T = 0;
-    std::vector<float> t(c->R);
-    CK(c, cudaMemcpy(t.data(), c->d_T, sizeof(float) * c->R, cudaMemcpyDeviceToHost));
-    for (float v : t) T += v;
-    stats->model_max = h[1];
-    stats->sum_plogp = h[2];
-    stats->total_loglik = h[3];
+    for (int64_t r = 0; r < c->R; ++r) T += t[r];
+    stats->model_max = h->stats[1];
+    stats->sum_plogp = h->stats[2];
+    stats->total_loglik = h->stats[3];
     stats->total_resp = T;
   }
   return EMC_OK;
@@ -3036,10 +3234,10 @@ static emc_status batch_own_compress(emc_batch* b, int i) {
     la.kval = c->csr.val;
     la.e = e;
     la.gate_count = c->d_lcount;
-    la.gate_cap = c->lcomp_cap;
+    la.gate_cap = c->list_gate;
     BCK(b, launch_list_compress(la, c->st));
     e.gate_count = c->d_lcount;
-    e.gate_cap = c->lcomp_cap;
+    e.gate_cap = c->list_gate;
     c->launches += 1;
   }
   if (c->tune.compress_pair)
