@@ -230,7 +230,9 @@ struct emc_context {
   unsigned long long* d_cand_key = nullptr;
   float4* d_part = nullptr;
   float2* d_acc = nullptr;  // interleaved (model, weight) accumulators
-  float2* d_acc_odd = nullptr;  // trilinear: the shifted pairs (insert.cuh), behind d_acc
+  float2* d_acc_odd = nullptr;  // trilinear: the shifted pairs (InsertAcc), behind d_acc
+  int64_t acc_stride = 0;       // pairs from one copy of both to the next
+  int acc_copies = 1;
   double *d_lse = nullptr, *d_plogp = nullptr;
   float* d_Tpart = nullptr;
   CUtensorMap tmKh, tmKt, tmBhi, tmBlo, tmPhi, tmPlo;
@@ -662,18 +664,27 @@ static emc_status set_y_rows(emc_context* c, int64_t rows) {
   return EMC_OK;
 }
 
-// The insertion accumulators.  Trilinear insertion takes a second, shifted
-// array in the same allocation where it is a small part of the memory left
-// (without it the pairs at odd voxels are two reductions).
-static emc_status alloc_acc(emc_context* c) {
-  const int64_t odd = round_up(c->M, 2) + c->M + 2;
-  if (c->cfg.interp == EMC_INTERP_TRILINEAR &&
-      sizeof(float2) * (size_t)odd <= avail_bytes(c, 0) / 8) {
-    TRY(c->alloc(&c->d_acc, odd, true));
-    c->d_acc_odd = c->d_acc + round_up(c->M, 2);
-    return EMC_OK;
-  }
-  return c->alloc(&c->d_acc, c->M, true);
+// The insertion accumulators: for an FP32 context copies of up to 16 MB in all
+// (they stay in L2; measured 10-15% off the compress of 1,000 patterns x 3,240
+// rotations with an unmasked centre, and a shorter FP32 sum per voxel; a mixed
+// context would need a pass of its own to merge them and gained nothing), each
+// with the shifted array of trilinear pairs behind it, where they are a small
+// part of the memory left; otherwise one array of pairs, or, for an FP32
+// context's dense iterations (needed = false), none: they then add to its model
+// and weight arrays.
+static emc_status alloc_acc(emc_context* c, bool needed) {
+  const bool tri = c->cfg.interp == EMC_INTERP_TRILINEAR;
+  const int64_t one = round_up(c->M, 2), stride = tri ? 2 * one + 2 : one;
+  int copies = 1;
+  while (!c->mixed && copies < 8 && (int64_t)sizeof(float2) * stride * copies * 2 <= (16 << 20)) copies *= 2;
+  const size_t bytes = sizeof(float2) * (size_t)(stride * copies);
+  const bool room = bytes <= avail_bytes(c, 0) / 8;
+  if (!room && !needed) return EMC_OK;
+  c->acc_copies = room ? copies : 1;
+  c->acc_stride = room ? stride : c->M;
+  TRY(c->alloc(&c->d_acc, c->acc_stride * c->acc_copies, true));
+  if (room && tri) c->d_acc_odd = c->d_acc + one;
+  return EMC_OK;
 }
 
 static emc_status alloc_work(emc_context* c) {
@@ -689,6 +700,7 @@ static emc_status alloc_work(emc_context* c) {
     // than the contraction's own error
     TRY(c->alloc(&c->d_LL64, R * N));
     TRY(c->alloc(&c->d_K, N * npa));
+    TRY(alloc_acc(c, false));
     // the responsibility pass's scratch, one allocation
     const int64_t chunk = resp_f32_chunk(R, N), nparts = (R + chunk - 1) / chunk;
     const int64_t nb = resp_f32_blocks(N);
@@ -722,7 +734,7 @@ static emc_status alloc_work(emc_context* c) {
   if (c->tune.compress_pair) c->tune.compress_raster = 2;
   c->Rpad = round_up(R, 256);
   c->nrt = c->Rpad / 256;
-  TRY(alloc_acc(c));
+  TRY(alloc_acc(c, true));
   // the nearest expansion's voxel table (here rather than at the first
   // expansion, so an iteration can be captured into a graph before any ran)
   if (c->cfg.interp == EMC_INTERP_NEAREST) TRY(c->alloc(&c->d_vtab, c->M + 1));
@@ -1118,13 +1130,18 @@ static MaxEpiArgs max_args(emc_context* c) {
 
 // The accumulators' starting state, and their sum after the insertion.
 static emc_status clear_acc(emc_context* c) {
-  const int64_t n = c->d_acc_odd ? round_up(c->M, 2) + c->M + 2 : c->M;
-  return c->cuda(cudaMemsetAsync(c->d_acc, 0, sizeof(float2) * n, c->st), "clear accumulators");
+  return c->cuda(cudaMemsetAsync(c->d_acc, 0, sizeof(float2) * c->acc_stride * c->acc_copies,
+                                 c->st), "clear accumulators");
+}
+static InsertAcc insert_acc(const emc_context* c) {
+  if (c->det) return InsertAcc{c->d_acc, nullptr, c->d_acc64, 0, 1};
+  return InsertAcc{c->d_acc, c->d_acc_odd, nullptr, c->acc_stride, c->acc_copies};
 }
 static emc_status merge_acc(emc_context* c) {
-  if (!c->d_acc_odd) return EMC_OK;
+  if (c->mixed && !c->d_acc_odd && c->acc_copies == 1) return EMC_OK;
   c->launches += 1;
-  return c->cuda(launch_merge_odd(c->d_acc, c->d_acc_odd, c->M, c->st), "merge accumulators");
+  return c->cuda(launch_merge_acc(insert_acc(c), c->M, c->mixed ? nullptr : c->d_model,
+                                  c->mixed ? nullptr : c->d_weight, c->st), "merge accumulators");
 }
 
 // Epilogue arguments of the mixed compress contraction (insertion).
@@ -1144,7 +1161,7 @@ static CmpEpiArgs cmp_args(emc_context* c) {
   e.cz = c->d_cz;
   e.ins = c->d_ins;
   e.pc = c->d_pc;
-  e.ins_acc = InsertAcc{c->d_acc, c->det ? nullptr : c->d_acc_odd, c->det ? c->d_acc64 : nullptr};
+  e.ins_acc = insert_acc(c);
   return e;
 }
 
@@ -1731,7 +1748,7 @@ emc_status emc_compress_insert(emc_context* c) {
   // emc.c:1025-1026 reset, then emc_cuda.cu:292-362 insert, :414-433 normalise
   if (c->det) {
     CK(c, cudaMemsetAsync(c->d_acc64, 0, sizeof(unsigned long long) * 8 * c->M, c->st));
-  } else if (!c->mixed) {
+  } else if (!c->mixed && !c->d_acc) {
     CK(c, cudaMemsetAsync(c->d_model, 0, sizeof(float) * c->M, c->st));
     CK(c, cudaMemsetAsync(c->d_weight, 0, sizeof(float) * c->M, c->st));
   } else {
@@ -1775,8 +1792,13 @@ emc_status emc_compress_insert(emc_context* c) {
     in.model = c->d_model;
     in.weight = c->d_weight;
     in.acc64 = c->det ? c->d_acc64 : nullptr;
+    if (c->d_acc) {
+      in.pc = c->d_pc;
+      in.to = insert_acc(c);
+    }
     CK(c, launch_insert(in, c->st));
     c->launches += 1;
+    if (c->d_acc && !c->det) TRY(merge_acc(c));
   } else {
     CmpEpiArgs e = cmp_args(c);
     const bool gated = c->cmp_mode == emc_context::CMP_GATED;
@@ -1896,8 +1918,8 @@ static emc_status iterate_stages(emc_context* c) {
 }
 
 // One iteration through a CUDA graph of its launches.  Small problems are
-// bound by them (16^3, 64 patterns x 420 rotations: @G0 us launched one by
-// one, @G1 us as a graph).  The graph is captured at the third iteration in a
+// bound by them (32^3, 1,000 patterns x 3,240 rotations, FP32: 345 us launched
+// one by one, 275 us as a graph).  The graph is captured at the third iteration in a
 // row that finds the same buffers and tuning, so a context that iterates once
 // or twice never pays for it, and it holds the same launches: nothing in it
 // depends on values.  Rotation chunks, the deterministic sort, profiling,
@@ -2648,7 +2670,7 @@ static emc_status run_proposed(emc_context* c, const ProposedPlan& pl, Select se
     TRY(c->alloc(&c->d_best, N));
     TRY(c->alloc(&c->d_bestp, N));
   }
-  if (!c->d_acc) TRY(alloc_acc(c));
+  if (!c->d_acc) TRY(alloc_acc(c, true));
   if (pairs > c->pairs_cap || c->cand_m != m) {
     int64_t cap = c->pairs_cap;
     TRY(grow(c, &c->d_cand, cap, pairs));

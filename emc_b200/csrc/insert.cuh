@@ -23,6 +23,12 @@ __device__ __forceinline__ void red_add_v4(float2* p, float x0, float y0, float 
                : "memory");
 }
 
+// The copy that rotation r adds to.
+__device__ __forceinline__ InsertAcc acc_copy(const InsertAcc& a, int64_t r) {
+  const int64_t o = (r & (a.copies - 1)) * a.stride;
+  return InsertAcc{a.acc + o, a.odd ? a.odd + o : nullptr, a.acc64, a.stride, a.copies};
+}
+
 __device__ __forceinline__ void insert_add(const InsertAcc& a, int vox, float x, float y) {
   if (a.acc64) {
     add_fixed(a.acc64 + 8 * (int64_t)vox, x);

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "tc.cuh"
+
 namespace emc {
 
 enum ExpandOut { EXP_F32 = 0, EXP_LOG_F32 = 1, EXP_F16_SPLIT = 2 };
@@ -197,6 +199,10 @@ struct InsertArgs {
   // deterministic insertion: fixed-point limbs [M][8] (fixed.cuh) instead of
   // FP32 atomics into model and weight
   unsigned long long* acc64;
+  // optional: packed coordinates (cx, cy, cz, insert flag); the insertion then
+  // adds to `to` instead of model, weight and acc64
+  const float4* pc;
+  InsertAcc to;
 };
 cudaError_t launch_insert(const InsertArgs& a, cudaStream_t st);
 // The fixed-point sums (fixed.cuh) as FP32 pairs a[i stride], b[i stride].

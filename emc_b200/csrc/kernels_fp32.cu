@@ -6,6 +6,7 @@
 #include <cstdint>
 
 #include "fixed.cuh"
+#include "insert.cuh"
 #include "kernels.cuh"
 #include "tile.cuh"
 #include "voxel.h"
@@ -737,6 +738,46 @@ __global__ void __launch_bounds__(kBlock) insert_kernel(const InsertArgs a) {
   }
 }
 
+// The contexts' insertion of averaged slices U: interleaved (model, weight)
+// pairs, so a voxel is one reduction instead of two, packed coordinates with
+// four pixels in flight, and the trilinear corners by pairs (insert.cuh).
+// With the slice sums before it: 10,000 patterns x 25,680 rotations at 64^3 4.14
+// -> 3.74 ms, 2,000 x 25,680 at 128^3 4.04 -> 3.45 ms, 1,000 x 3,240 at 32^3 93
+// -> 69 us.
+template <int INTERP>
+__global__ void __launch_bounds__(kBlock) insert_slices_kernel(const InsertArgs a) {
+  constexpr int kUnroll = 4;
+  const int64_t r = blockIdx.x;
+  const float T = a.T[r];
+  if (!((a.Tskip ? a.Tskip[r] : T) > 1e-10f) || !(T > 0.0f)) return;  // emc_atomic.cu:128
+  const float w = a.rotw[r] * T;
+  const InsertAcc to = acc_copy(a.to, r);
+  float m[9];
+  emc_voxel::rotation_matrix(a.quat + 4 * r, m);
+  const float* U = a.U + r * a.ldU;
+  const int n = (int)a.npix;
+  for (int j0 = threadIdx.x; j0 < n; j0 += kUnroll * kBlock) {
+    float4 q[kUnroll];
+    float s[kUnroll];
+#pragma unroll
+    for (int k = 0; k < kUnroll; ++k) {
+      const int j = j0 + k * kBlock;
+      q[k] = j < n ? __ldg(a.pc + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+      s[k] = j < n ? U[j] : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < kUnroll; ++k) {
+      if (q[k].w == 0.0f) continue;
+      float u[3];
+      emc_voxel::position(m, a.side, q[k].x, q[k].y, q[k].z, u);
+      if constexpr (INTERP == 0)
+        insert_nearest(to, u, a.side, w * s[k], w);
+      else
+        insert_trilinear(to, u, a.side, w * s[k], w);
+    }
+  }
+}
+
 // ------------------------------------------------------------- normalise --
 // Fixed-point accumulators -> FP32 (value, weight) pairs: a[i*stride],
 // b[i*stride] (the FP32 path's model and weight, or the mixed path's
@@ -1209,7 +1250,12 @@ cudaError_t launch_compress_fp32(const CompressArgs& a, cudaStream_t st) {
 
 cudaError_t launch_insert(const InsertArgs& a, cudaStream_t st) {
   if (a.R <= 0) return cudaSuccess;
-  insert_kernel<<<(unsigned)a.R, kBlock, 0, st>>>(a);
+  if (a.pc && a.interp == 0)
+    insert_slices_kernel<0><<<(unsigned)a.R, kBlock, 0, st>>>(a);
+  else if (a.pc)
+    insert_slices_kernel<1><<<(unsigned)a.R, kBlock, 0, st>>>(a);
+  else
+    insert_kernel<<<(unsigned)a.R, kBlock, 0, st>>>(a);
   return cudaGetLastError();
 }
 

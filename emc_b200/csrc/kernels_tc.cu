@@ -504,6 +504,7 @@ struct EpiCmp {
   bool active;
   float m[9];
   float wU, wT;
+  InsertAcc to;
 
   __device__ void tile_begin(int64_t mt, int64_t nt, int tid, uint8_t* smem) {
     float4* cs = reinterpret_cast<float4*>(smem);
@@ -527,6 +528,7 @@ struct EpiCmp {
         active = true;
         const float rw = a.rotw[r];
         wT = rw * T;
+        to = acc_copy(a.ins_acc, r);
         wU = wT * a.inv_c0;  // accumulator holds U_r / T_r (rows of P' are divided by T_r)
         emc_voxel::rotation_matrix(a.quat + 4 * r, m);
       }
@@ -544,7 +546,7 @@ struct EpiCmp {
         if (q.w == 0.0f) continue;
         float u[3];
         emc_voxel::position(m, a.side, q.x, q.y, q.z, u);
-        insert_nearest(a.ins_acc, u, a.side, __uint_as_float(v[k]) * wU, wT);
+        insert_nearest(to, u, a.side, __uint_as_float(v[k]) * wU, wT);
       }
     } else {
 #pragma unroll
@@ -553,7 +555,7 @@ struct EpiCmp {
         if (q.w == 0.0f) continue;
         float u[3];
         emc_voxel::position(m, a.side, q.x, q.y, q.z, u);
-        insert_trilinear(a.ins_acc, u, a.side, __uint_as_float(v[k]) * wU, wT);
+        insert_trilinear(to, u, a.side, __uint_as_float(v[k]) * wU, wT);
       }
     }
   }
@@ -1899,6 +1901,7 @@ __global__ void __launch_bounds__(THREADS, INTERP == 0 ? (THREADS == 512 ? 3 : 6
   }
   __syncthreads();
   const float wT = e.rotw[r] * T;
+  const InsertAcc to = acc_copy(e.ins_acc, r);
   float m[9];
   emc_voxel::rotation_matrix(e.quat + 4 * r, m);
   for (int j0 = threadIdx.x; j0 < npa; j0 += kInsertUnroll * THREADS) {
@@ -1915,21 +1918,33 @@ __global__ void __launch_bounds__(THREADS, INTERP == 0 ? (THREADS == 512 ? 3 : 6
       emc_voxel::position(m, e.side, q[k].x, q[k].y, q[k].z, u);
       const float val = Us[j0 + k * THREADS] * wT;
       if constexpr (INTERP == 0)
-        insert_nearest(e.ins_acc, u, e.side, val, wT);
+        insert_nearest(to, u, e.side, val, wT);
       else
-        insert_trilinear(e.ins_acc, u, e.side, val, wT);
+        insert_trilinear(to, u, e.side, val, wT);
     }
   }
 }
 
-__global__ void merge_odd_kernel(float2* acc, const float2* odd, int64_t M) {
+__global__ void merge_acc_kernel(const InsertAcc a, int64_t M, float* model, float* weight) {
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < M;
        v += (int64_t)gridDim.x * blockDim.x) {
-    float2 a = acc[v];
-    const float2 b = odd[v + 1];
-    a.x += b.x;
-    a.y += b.y;
-    acc[v] = a;
+    double x = 0.0, y = 0.0;
+    for (int k = 0; k < a.copies; ++k) {
+      const float2 p = a.acc[k * a.stride + v];
+      x += (double)p.x;
+      y += (double)p.y;
+      if (a.odd) {
+        const float2 q = a.odd[k * a.stride + v + 1];
+        x += (double)q.x;
+        y += (double)q.y;
+      }
+    }
+    if (model) {
+      model[v] = (float)x;
+      weight[v] = (float)y;
+    } else {
+      a.acc[v] = make_float2((float)x, (float)y);
+    }
   }
 }
 
@@ -2406,8 +2421,10 @@ cudaError_t launch_list_compress(const ListCmpArgs& a, cudaStream_t st) {
   return wide ? run_list_compress<512, 1>(a, smem, st) : run_list_compress<256, 1>(a, smem, st);
 }
 
-cudaError_t launch_merge_odd(float2* acc, const float2* odd, int64_t M, cudaStream_t st) {
-  merge_odd_kernel<<<(unsigned)std::min<int64_t>((M + 255) / 256, 1184), 256, 0, st>>>(acc, odd, M);
+cudaError_t launch_merge_acc(const InsertAcc& a, int64_t M, float* model, float* weight,
+                             cudaStream_t st) {
+  merge_acc_kernel<<<(unsigned)std::min<int64_t>((M + 255) / 256, 1184), 256, 0, st>>>(a, M, model,
+                                                                                     weight);
   return cudaGetLastError();
 }
 

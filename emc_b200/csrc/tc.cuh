@@ -69,11 +69,16 @@ cudaError_t launch_maximize_pair_tc(const CUtensorMap& tmK, const CUtensorMap& t
 // deterministic mode (acc64).  odd (trilinear, optional): a second array of
 // pairs, shifted by one voxel (odd[v + 1] belongs to voxel v), so that the
 // pairs of voxels (v, v + 1) are 16-byte aligned there for odd v as they are
-// in acc for even v; launch_merge_odd adds it to acc.
+// in acc for even v.  Rotation r adds to copy r % copies of both, `stride`
+// pairs apart: the voxels near the centre take a reduction from every
+// rotation, which one address serves one after the other.  launch_merge_acc
+// sums copies and odd pairs into acc.
 struct InsertAcc {
   float2* acc;
   float2* odd;
   unsigned long long* acc64;
+  int64_t stride;
+  int copies;  // a power of two
 };
 
 // Compress contraction: acc[r][j] = sum_p (P'_hi + P'_lo)[r][p] Kt[j][p] with
@@ -98,8 +103,10 @@ struct CmpEpiArgs {
   const unsigned long long* gate_count;
   int64_t gate_cap;
 };
-// acc[v] += odd[v + 1] (InsertAcc::odd, after the insertion).
-cudaError_t launch_merge_odd(float2* acc, const float2* odd, int64_t M, cudaStream_t st);
+// acc[v] = the sum of voxel v over the copies and their odd pairs (in FP64),
+// after the insertion; or, with model and weight, the sums go there.
+cudaError_t launch_merge_acc(const InsertAcc& a, int64_t M, float* model, float* weight,
+                             cudaStream_t st);
 // raster: rotation tiles per band of the tile order.
 cudaError_t launch_compress_tc(const CUtensorMap& tmPhi, const CUtensorMap& tmPlo,
                                const CUtensorMap& tmKt, int64_t Rpad, int64_t Ppad,
