@@ -666,9 +666,9 @@ static emc_status set_y_rows(emc_context* c, int64_t rows) {
 
 // The insertion accumulators: for an FP32 context copies of up to 16 MB in all
 // (they stay in L2; measured 10-15% off the compress of 1,000 patterns x 3,240
-// rotations with an unmasked centre, and a shorter FP32 sum per voxel; a mixed
-// context would need a pass of its own to merge them and gained nothing), each
-// with the shifted array of trilinear pairs behind it, where they are a small
+// rotations with an unmasked centre, and a shorter FP32 sum per voxel; mixed
+// contexts gained nothing from them, nearest or trilinear), each with the
+// shifted array of trilinear pairs behind it, where they are a small
 // part of the memory left; otherwise one array of pairs, or, for an FP32
 // context's dense iterations (needed = false), none: they then add to its model
 // and weight arrays.
@@ -1376,6 +1376,8 @@ static emc_status gated_list_pass(emc_context* c) {
   a.list_rp = c->d_lcomp_rp;
   a.list_P = c->d_lcomp_P;
   a.list_min = kListMinP;
+  // past what lists are worth, neither the entries nor their number matter
+  a.list_stop = std::max({list_worth(c), 64 * c->N, c->lcomp_cap});
   CK(c, launch_resp_rowsums(a, c->st));
   CK(c, launch_list_from_compact(a, c->list_gate, kListRel, c->d_lrowtot, c->d_lcursor,
                                  c->d_lrowoff, c->d_lpat, c->d_lx, c->st, c->d_lcount));

@@ -59,8 +59,8 @@ __device__ float block_max(float v, float* red) {
 template <int INTERP>
 __device__ __forceinline__ float gather(const float* __restrict__ model, const float* u, int side) {
   if (INTERP == 0) {
-    int64_t v;
-    return emc_voxel::nearest(u, side, 1, &v) ? __ldg(model + v) : 0.0f;
+    int v;
+    return emc_voxel::nearest32(u, side, 1, &v) ? __ldg(model + v) : 0.0f;
   }
   float acc = 0.0f;
 #pragma unroll
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kBlock) expand_tab_kernel(const ExpandArgs a) 
   const int64_t r = blockIdx.x;
   float m[9];
   emc_voxel::rotation_matrix(a.quat + 4 * r, m);
-  const int64_t M = (int64_t)a.side * a.side * a.side;
+  const int M = a.side * a.side * a.side;  // side <= 1024
   const int npix = (int)a.npix, npairs = (int)(a.ld / 2);
   __half2* hi_row = reinterpret_cast<__half2*>(a.out_hi + r * a.ld);
   __half2* lo_row = reinterpret_cast<__half2*>(a.out_lo + r * a.ld);
@@ -218,8 +218,8 @@ __global__ void __launch_bounds__(kBlock) expand_tab_kernel(const ExpandArgs a) 
       if (i < npix) {
         float pos[3];
         emc_voxel::position(m, a.side, __ldg(a.cx + i), __ldg(a.cy + i), __ldg(a.cz + i), pos);
-        int64_t v;
-        if (!emc_voxel::nearest(pos, a.side, 1, &v)) v = M;
+        int v;
+        if (!emc_voxel::nearest32(pos, a.side, 1, &v)) v = M;
         t[u] = __ldg(a.tab + v);
       }
     }
@@ -434,18 +434,32 @@ __device__ __forceinline__ void stat_rescale(StatAcc& a, double m) {
     a.m = m;
   }
 }
-__device__ __forceinline__ void stat_merge(StatAcc& a, const StatAcc& b) {
-  if (b.m <= -DBL_MAX) return;
-  stat_rescale(a, b.m);
-  const double f = exp(b.m - a.m);
-  a.q += f > 0.0 ? f * (b.q + (b.m - a.m) * b.s) : 0.0;
-  a.s += f * b.s;
-  a.d += f * b.d;
+// The eight warps' sums of one pattern (lane), relative to their common
+// maximum: one exponential per thread, the total on warp 0.
+__device__ __forceinline__ void stat_reduce(StatAcc& a, double (&sh)[4][8][32], int w, int lane) {
+  sh[0][w][lane] = a.m;
+  __syncthreads();
+  double m = sh[0][0][lane];
+#pragma unroll
+  for (int k = 1; k < 8; ++k) m = fmax(m, sh[0][k][lane]);
+  const double dm = a.m - m, f = a.m > -DBL_MAX ? exp(dm) : 0.0;
+  sh[1][w][lane] = f * a.s;
+  sh[2][w][lane] = f * a.d;
+  sh[3][w][lane] = f > 0.0 ? f * (a.q + dm * a.s) : 0.0;
+  __syncthreads();
+  if (w != 0) return;
+  a = StatAcc{m, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    a.s += sh[1][k][lane];
+    a.d += sh[2][k][lane];
+    a.q += sh[3][k][lane];
+  }
 }
 
 template <bool POISSON>
 __global__ void __launch_bounds__(256) resp_stats_kernel(const RespF32Args a) {
-  __shared__ double sh[8][32][4];
+  __shared__ double sh[4][8][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t cols = (a.N + 31) / 32, by = blockIdx.x / cols;
   const int64_t p = (blockIdx.x - by * cols) * 32 + lane;
@@ -486,36 +500,28 @@ __global__ void __launch_bounds__(256) resp_stats_kernel(const RespF32Args a) {
     acc.d += (double)d;
     acc.q += (double)q;
   }
-  sh[w][lane][0] = acc.m;
-  sh[w][lane][1] = acc.s;
-  sh[w][lane][2] = acc.d;
-  sh[w][lane][3] = acc.q;
-  __syncthreads();
-  if (w == 0 && ok) {
-    for (int k = 1; k < 8; ++k)
-      stat_merge(acc, StatAcc{sh[k][lane][0], sh[k][lane][1], sh[k][lane][2], sh[k][lane][3]});
-    a.part[by * a.N + p] = make_double4(acc.m, acc.s, acc.d, acc.q);
-  }
+  stat_reduce(acc, sh, w, lane);
+  if (w == 0 && ok) a.part[by * a.N + p] = make_double4(acc.m, acc.s, acc.d, acc.q);
 }
 
 __global__ void __launch_bounds__(256) resp_combine_kernel(const RespF32Args a) {
-  __shared__ double sh[8][32][4];
+  __shared__ double sh[4][8][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t p = (int64_t)blockIdx.x * 32 + lane;
+  const bool ok = p < a.N;
   StatAcc acc{-DBL_MAX, 0.0, 0.0, 0.0};
-  if (p < a.N)
+  if (ok) {
+    for (int64_t k = w; k < a.nparts; k += 8) acc.m = fmax(acc.m, a.part[k * a.N + p].x);
     for (int64_t k = w; k < a.nparts; k += 8) {
       const double4 v = a.part[k * a.N + p];
-      stat_merge(acc, StatAcc{v.x, v.y, v.z, v.w});
+      const double dm = v.x - acc.m, f = exp(dm);
+      acc.s += f * v.y;
+      acc.d += f * v.z;
+      if (f > 0.0) acc.q += f * (v.w + dm * v.y);
     }
-  sh[w][lane][0] = acc.m;
-  sh[w][lane][1] = acc.s;
-  sh[w][lane][2] = acc.d;
-  sh[w][lane][3] = acc.q;
-  __syncthreads();
-  if (w != 0 || p >= a.N) return;
-  for (int k = 1; k < 8; ++k)
-    stat_merge(acc, StatAcc{sh[k][lane][0], sh[k][lane][1], sh[k][lane][2], sh[k][lane][3]});
+  }
+  stat_reduce(acc, sh, w, lane);
+  if (w != 0 || !ok) return;
   const double ls = log(acc.s);
   a.lse[p] = acc.m + ls;
   a.plogp[p] = acc.q / acc.s - ls;  // sum P (LL - lse)

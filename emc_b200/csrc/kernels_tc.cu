@@ -1301,28 +1301,49 @@ __device__ __forceinline__ void probs_from(const PatConst<POISSON>& k, float4 y,
   for (int i = 0; i < 4; ++i) P[i] = k.ok[i] ? expf(P[i]) : 0.0f;
 }
 
-// Sweep A: Tpart[pattern block][r] = sum over the block's patterns of P_rp.
-// Once the posteriors are sharp, most of P is zero in FP32: where no element
-// of a warp's four rows x 128 patterns reaches kExpZero, they are left at the
-// comparison (no exponential, no reduction, no compaction).
-constexpr float kExpZero = -105.0f;  // expf is zero below (the smallest float is e^-103.3)
+// Sweep A: Tpart[pattern block][r] = sum over the block's patterns of P_rp, and
+// the compaction of the entries P >= list_min.
+//
+// Once the posteriors are sharp, nearly every P is below list_min = 1e-30
+// (99.6% of them at 128^2 and 500 photons), and the sweep is bound by its
+// instructions, not by Y (the exponential, the compaction's scan and the row
+// reduction of every element: 44 instructions an element, 0.76 ms for the 2 GB
+// of 20,000 patterns x 25,680 rotations).  Such elements are left at the
+// comparison with kExpKeep: a warp's four rows x 128 patterns where none is
+// above it, else the exponentials and the compaction of those places where
+// some lane has one, the entries' slots coming from ballots (with the
+// rows of a block below: 0.76 -> 0.61 ms).
+// A sum T_r above 1e-10, below which rotations are not inserted, is the same
+// FP32 number without them.
+//
+// Each warp gathers its entries in shared memory and reserves room for them
+// with one atomic per flush: one counter serves the whole grid, and an atomic
+// per warp and row on it serialised the sweep (15.0 -> 10.6 ms at 50,000
+// patterns x 86,520 rotations).  A warp that finds the counter past list_stop
+// stops compacting: nothing will read the entries, or their exact number.
+constexpr float kExpKeep = -69.2f;  // e^-69.2 < 1e-30, the list_min of every caller
 template <bool POISSON>
-__global__ void __launch_bounds__(kSweepThreads, 4) rowsum_kernel(const RespArgs a) {
+__global__ void __launch_bounds__(kSweepThreads, 4) rowsum_kernel(const RespArgs a,
+                                                                  const int rows) {
   __shared__ float red[kSweepThreads / 32][kSweepRows];
-  // Each warp gathers the compacted entries of its rows in shared memory and
-  // reserves room for them with one atomic per flush: one counter serves the
-  // whole grid, and an atomic per warp and row on it serialised the sweep
-  // (measured at full size: 15.0 -> 10.6 ms per steady-state iteration)
   constexpr int kBuf = 256;
   __shared__ int2 brp[kSweepThreads / 32][kBuf];
   __shared__ float bv[kSweepThreads / 32][kBuf];
-  const int64_t p0 = (int64_t)blockIdx.x * kSweepPatterns + 4 * threadIdx.x;
-  const int64_t r0 = (int64_t)blockIdx.y * kSweepRows;
+  const int64_t nblk = (a.N + kSweepPatterns - 1) / kSweepPatterns;
+  const int64_t by = blockIdx.x / nblk, bx = blockIdx.x - by * nblk;
+  const int64_t p0 = bx * kSweepPatterns + 4 * threadIdx.x;
+  const int64_t r0 = by * rows;
   const bool any = p0 < a.N;
   PatConst<POISSON> k;
   load_consts<POISSON>(a, p0, k);
+  uint32_t real = 0;  // as `live` below: the patterns there are (Y's padding is not set)
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (k.ok[j]) real |= 0x1111u << j;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int nb = 0;  // entries in this warp's buffer (warp-uniform)
+  const uint32_t below = (1u << lane) - 1u;
+  bool list = a.list_count != nullptr;  // warp-uniform
+  int nb = 0;                           // entries in this warp's buffer (warp-uniform)
   auto flush = [&]() {
     unsigned long long base = 0;
     if (lane == 0) base = atomicAdd(a.list_count, (unsigned long long)nb);
@@ -1337,67 +1358,61 @@ __global__ void __launch_bounds__(kSweepThreads, 4) rowsum_kernel(const RespArgs
     }
     __syncwarp();
     nb = 0;
+    if (a.list_stop && (int64_t)base > a.list_stop) list = false;
   };
   // four rows per step: their loads are issued before any result is needed
-  for (int i0 = 0; i0 < kSweepRows; i0 += 4) {
+  for (int i0 = 0; i0 < rows; i0 += 4) {
     float t[4];
     float4 y[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int64_t r = r0 + i0 + u;
       y[u] = (r < a.R && any) ? *reinterpret_cast<const float4*>(a.Y + r * a.ldY + p0)
-                              : make_float4(0.f, 0.f, 0.f, 0.f);
+                              : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
     }
-    bool live = false;
-    float d[4][4];
+    uint32_t live = 0;  // bit 4 u + j: element (row u, pattern j) is to be kept
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int64_t r = r0 + i0 + u;
-      const bool in = r < a.R && any;
-      const double rs = POISSON || !in ? 0.0 : a.rowstat[r] * a.gauss_inv;
-      log_probs<POISSON>(k, y[u], rs, d[u]);
+      const double rs = POISSON || r >= a.R ? 0.0 : a.rowstat[r] * a.gauss_inv;
+      float d[4];
+      log_probs<POISSON>(k, y[u], rs, d);
+      t[u] = 0.0f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) live |= in && !(d[u][j] < kExpZero);
+      for (int j = 0; j < 4; ++j)
+        if (!(d[j] < kExpKeep)) live |= 1u << (4 * u + j);
+      if (!POISSON) y[u] = make_float4(d[0], d[1], d[2], d[3]);
     }
-    if (!__any_sync(0xffffffffu, live)) {
+    live &= real;
+    const uint32_t warp_live = __reduce_or_sync(0xffffffffu, live);
+    if (!warp_live) {
       if (lane < 4) red[w][i0 + lane] = 0.0f;
       continue;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int64_t r = r0 + i0 + u;
-      t[u] = 0.0f;
-      float P[4] = {0.f, 0.f, 0.f, 0.f};
-      if (r < a.R && any) {
+      const float yy[4] = {y[u].x, y[u].y, y[u].z, y[u].w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) P[j] = k.ok[j] ? expf(d[u][j]) : 0.0f;
-        t[u] = (P[0] + P[1]) + (P[2] + P[3]);
-      }
-      if (a.list_count) {
-        int n = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) n += (k.ok[j] && P[j] >= a.list_min) ? 1 : 0;
-        if (__any_sync(0xffffffffu, n > 0)) {
-          int inc = n;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += v;
-          }
-          const int tot = __shfl_sync(0xffffffffu, inc, 31);
-          if (nb + tot > kBuf) flush();
-          int q = nb + inc - n;
-          const float yy[4] = {y[u].x, y[u].y, y[u].z, y[u].w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (k.ok[j] && P[j] >= a.list_min) {
-              brp[w][q] = make_int2((int)(a.list_r0 + r), (int)(p0 + j));
-              bv[w][q] = a.list_store_y ? yy[j] : P[j];
-              ++q;
-            }
-          nb += tot;
-          __syncwarp();
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t bit = 1u << (4 * u + j);
+        if (!(warp_live & bit)) continue;  // uniform over the warp
+        // poisson: the difference again (cheaper than keeping it)
+        const float d = POISSON ? __fsub_rn(__fsub_rn(yy[j], k.lse_hi[j]), k.lse_lo[j]) : yy[j];
+        const float P = (live & bit) ? expf(d) : 0.0f;
+        t[u] += P;
+        const uint32_t b = list ? __ballot_sync(0xffffffffu, P >= a.list_min) : 0u;
+        if (b == 0) continue;
+        if (nb + 32 > kBuf) flush();
+        if (b >> lane & 1u) {
+          const int e = nb + __popc(b & below);
+          brp[w][e] = make_int2((int)(a.list_r0 + r0 + i0 + u), (int)(p0 + j));
+          if (POISSON || !a.list_store_y)
+            bv[w][e] = a.list_store_y ? yy[j] : P;
+          else
+            bv[w][e] = a.Y[(r0 + i0 + u) * a.ldY + p0 + j];
         }
+        nb += __popc(b);
+        __syncwarp();
       }
     }
     // four row sums by halving exchanges: lane 8 u ends with row u's
@@ -1416,11 +1431,11 @@ __global__ void __launch_bounds__(kSweepThreads, 4) rowsum_kernel(const RespArgs
   }
   if (a.list_count && nb > 0) flush();
   __syncthreads();
-  if (threadIdx.x < kSweepRows) {
+  if (threadIdx.x < rows) {
     const int64_t r = r0 + threadIdx.x;
     float t = 0.0f;
     for (int i = 0; i < kSweepThreads / 32; ++i) t += red[i][threadIdx.x];
-    if (r < a.R && a.Tpart) a.Tpart[(int64_t)blockIdx.x * a.R + r] = t;
+    if (r < a.R && a.Tpart) a.Tpart[bx * a.R + r] = t;
   }
 }
 
@@ -1868,7 +1883,7 @@ __global__ void sorted_place_kernel(const int2* rp, const float* Pv, int64_t n, 
 // of 512 threads where the slice leaves room for few blocks.
 constexpr int kInsertUnroll = 4;
 template <int THREADS, int INTERP>
-__global__ void __launch_bounds__(THREADS, INTERP == 0 ? (THREADS == 512 ? 3 : 6) : (THREADS == 512 ? 2 : 4))
+__global__ void __launch_bounds__(THREADS, (INTERP == 0 ? 1536 : 1024) / THREADS)
     list_compress_kernel(const ListCmpArgs a) {
   extern __shared__ float Us[];  // [npa]
   const int64_t r = blockIdx.x;
@@ -2189,11 +2204,16 @@ cudaError_t launch_batch_compress_tc(const TmapSet<kMaxBatch>& maps, int64_t n_t
 cudaError_t launch_resp_rowsums(RespArgs& a, cudaStream_t st) {
   combine_kernel<<<(unsigned)((a.N + 31) / 32), 256, 0, st>>>(a);
   const int64_t nblk = (a.N + kSweepPatterns - 1) / kSweepPatterns;
-  const int64_t rblk = (a.R + kSweepRows - 1) / kSweepRows;
+  // 32 rows a block, fewer where that would leave SMs without blocks (256
+  // patterns x 3,240 rotations, 102 blocks of 32 rows: the responsibility stage
+  // 64 -> 53 us with 8)
+  int rows = kSweepRows;
+  while (rows > 8 && nblk * ((a.R + rows - 1) / rows) < 4 * 148) rows /= 2;
+  const unsigned grid = (unsigned)(nblk * ((a.R + rows - 1) / rows));
   if (a.poisson)
-    rowsum_kernel<true><<<dim3((unsigned)nblk, (unsigned)rblk), kSweepThreads, 0, st>>>(a);
+    rowsum_kernel<true><<<grid, kSweepThreads, 0, st>>>(a, rows);
   else
-    rowsum_kernel<false><<<dim3((unsigned)nblk, (unsigned)rblk), kSweepThreads, 0, st>>>(a);
+    rowsum_kernel<false><<<grid, kSweepThreads, 0, st>>>(a, rows);
   return cudaGetLastError();
 }
 

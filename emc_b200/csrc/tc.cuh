@@ -244,6 +244,9 @@ struct RespArgs {
   int2* list_rp;
   float* list_P;
   float list_min;
+  // optional: once the count is past it the entries are no longer counted
+  // exactly (the count stays above it)
+  int64_t list_stop;
   // rotation chunks: the sweep covers Y rows of rotations list_r0 .. list_r0
   // + R - 1 (R, rowstat and Y are the chunk's), appends (list_r0 + r, p, y)
   // with the stored y instead of P, and writes no Tpart (nullptr)
