@@ -270,11 +270,11 @@ struct emc_context {
   unsigned long long* d_lcount = nullptr;  // entries compacted by the row-sum sweep
   int2* d_lcomp_rp = nullptr;              // their (rotation, pattern)
   float* d_lcomp_P = nullptr;              // and P
-  int64_t lcomp_cap = 0, lcomp_cap2 = 0;
+  int64_t lcomp_cap = 0;
   int64_t *d_lrowtot = nullptr, *d_lrowoff = nullptr, *d_lcursor = nullptr;
   int32_t* d_lpat = nullptr;
   float* d_lx = nullptr;
-  int64_t lcap = 0, lcap_x = 0, list_nnz = 0;
+  int64_t lcap = 0, list_nnz = 0;
   // this iteration's compress: the dense operand, the lists, or both gated on
   // the count of compacted entries (lists up to list_gate of them)
   enum { CMP_DENSE, CMP_LISTS, CMP_GATED } cmp_mode = CMP_DENSE;
@@ -344,9 +344,8 @@ struct emc_context {
   bool upload_pending = false;
 
   // pinned host staging of the proposed iteration, reused between calls
-  // [8]: the count of compacted entries (ev_count); [9], [10]: read_back
-  void* hpin[11] = {nullptr};
-  size_t hcap[11] = {0};
+  void* hpin[9] = {nullptr};  // [8]: host_back
+  size_t hcap[9] = {0};
   template <class T>
   T* pinned(int slot, size_t n) {
     const size_t bytes = n * sizeof(T) + 16;
@@ -1212,26 +1211,44 @@ static RespArgs resp_args(emc_context* c) {
   return a;
 }
 
+// The lists' counter, counts, starts and cursors: one allocation.
 static emc_status list_buffers(emc_context* c) {
-  if (!c->d_lcount) {
-    const int64_t R = c->R;
-    TRY(c->alloc(&c->d_lcount, 1));
-    TRY(c->alloc(&c->d_lrowtot, R + 1));
-    TRY(c->alloc(&c->d_lrowoff, R + 1));
-    TRY(c->alloc(&c->d_lcursor, R));
-  }
+  if (c->d_lcount) return EMC_OK;
+  const int64_t R = c->R;
+  int64_t* q = nullptr;
+  TRY(c->alloc(&q, 1 + 2 * (R + 1) + R));
+  c->d_lcount = reinterpret_cast<unsigned long long*>(q);
+  c->d_lrowtot = q + 1;
+  c->d_lrowoff = c->d_lrowtot + R + 1;
+  c->d_lcursor = c->d_lrowoff + R + 1;
   return EMC_OK;
 }
 
-// Room for `n` compacted (rotation, pattern, value) entries.
+// Room for `n` compacted (rotation, pattern, value) entries (contents not kept).
 static emc_status compact_capacity(emc_context* c, int64_t n) {
   if (c->lcomp_cap >= n && c->d_lcomp_rp) return EMC_OK;
-  int64_t cap = c->lcomp_cap;
-  TRY(grow(c, &c->d_lcomp_rp, cap, n));
-  int64_t cap2 = c->lcomp_cap2;
-  TRY(grow(c, &c->d_lcomp_P, cap2, cap));
+  if (c->d_lcomp_rp) c->release(c->d_lcomp_rp);
+  c->d_lcomp_rp = nullptr;
+  c->lcomp_cap = 0;
+  const int64_t cap = n + n / 4 + 64;
+  char* q = nullptr;
+  TRY(c->alloc(&q, (sizeof(int2) + sizeof(float)) * cap));
+  c->d_lcomp_rp = reinterpret_cast<int2*>(q);
+  c->d_lcomp_P = reinterpret_cast<float*>(q + sizeof(int2) * cap);
   c->lcomp_cap = cap;
-  c->lcomp_cap2 = cap2;
+  return EMC_OK;
+}
+
+// Room for `n` list entries (pattern, value) (contents not kept).
+static emc_status list_capacity(emc_context* c, int64_t n) {
+  if (c->lcap >= n && c->d_lpat) return EMC_OK;
+  if (c->d_lpat) c->release(c->d_lpat);
+  c->d_lpat = nullptr;
+  c->lcap = 0;
+  const int64_t cap = n + n / 4 + 64;
+  TRY(c->alloc(&c->d_lpat, 2 * cap));
+  c->d_lx = reinterpret_cast<float*>(c->d_lpat + cap);
+  c->lcap = cap;
   return EMC_OK;
 }
 
@@ -1282,10 +1299,7 @@ static emc_status det_resp_pass(emc_context* c) {
   CK(c, cudaStreamSynchronize(c->st));
   c->list_nnz = (int64_t)*hn;
   if (c->list_nnz <= std::min(worth, c->lcomp_cap)) {
-    TRY(grow(c, &c->d_lpat, c->lcap, c->list_nnz + 1));
-    int64_t cap = c->lcap_x;
-    TRY(grow(c, &c->d_lx, cap, c->list_nnz + 1));
-    c->lcap_x = cap;
+    TRY(list_capacity(c, c->list_nnz + 1));
     // the entries in (rotation, pattern) order, so the lists do not depend on
     // the order the sweep appended them
     TRY(sort_scratch(c, c->list_nnz));
@@ -1312,6 +1326,10 @@ static emc_status det_resp_pass(emc_context* c) {
 static emc_status gated_list_pass(emc_context* c);
 static emc_status batch_lists_ready(emc_context* c, int64_t entries);
 
+// One block of pinned memory for what comes back: [0] the count of compacted
+// entries, from byte 16 a HostBack and T_r.
+static char* host_back(emc_context* c) { return c->pinned<char>(8, 256 + sizeof(float) * c->R); }
+
 static bool uses_lists(const emc_context* c) {
   return c->mixed && c->tune.compress_sparse && c->npa <= kListMaxPixels;
 }
@@ -1322,18 +1340,19 @@ static bool uses_lists(const emc_context* c) {
 // room for that many entries where lists of that length would be the faster
 // form; after a pass it has the count copied back.
 static emc_status list_room(emc_context* c) {
+  if (!c->csr.valid) TRY(build_rows(c, c->d_K, c->N, c->npa, c->csr, false));
   int64_t want = std::max<int64_t>({64 * c->N, (int64_t)1 << 20, c->lcomp_cap});
   if (c->count_pending && cudaEventQuery(c->ev_count) == cudaSuccess) {
     c->count_pending = false;
-    c->list_nnz = (int64_t)*c->pinned<unsigned long long>(8, 1);
-    if (c->csr.valid && c->list_nnz <= std::max<int64_t>(list_worth(c), 64 * c->N))
+    c->list_nnz = (int64_t)*reinterpret_cast<unsigned long long*>(host_back(c));
+    if (c->list_nnz <= std::max<int64_t>(list_worth(c), 64 * c->N))
       want = std::max(want, c->list_nnz);
   }
   return batch_lists_ready(c, want);
 }
 static emc_status list_count_back(emc_context* c) {
   if (c->count_pending) return EMC_OK;
-  unsigned long long* hn = c->pinned<unsigned long long>(8, 1);
+  unsigned long long* hn = reinterpret_cast<unsigned long long*>(host_back(c));
   if (!hn) return c->fail(EMC_ERR_OOM, "pinned host staging");
   if (!c->ev_count) CK(c, cudaEventCreateWithFlags(&c->ev_count, cudaEventDisableTiming));
   CK(c, cudaMemcpyAsync(hn, c->d_lcount, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
@@ -1395,10 +1414,7 @@ static emc_status gated_list_pass(emc_context* c) {
 static emc_status batch_lists_ready(emc_context* c, int64_t entries) {
   TRY(list_buffers(c));
   TRY(compact_capacity(c, entries));
-  TRY(grow(c, &c->d_lpat, c->lcap, c->lcomp_cap + 1));
-  int64_t cap = c->lcap_x;
-  TRY(grow(c, &c->d_lx, cap, c->lcomp_cap + 1));
-  c->lcap_x = cap;
+  TRY(list_capacity(c, c->lcomp_cap + 1));
   if (!c->csr.valid) TRY(build_rows(c, c->d_K, c->N, c->npa, c->csr, false));
   return EMC_OK;
 }
@@ -1470,10 +1486,7 @@ static emc_status chunked_maximize(emc_context* c) {
   }
   c->mark(2);
   TRY(grow(c, &c->d_cand_P, c->cand_P_cap, c->cand_n + 1));
-  TRY(grow(c, &c->d_lpat, c->lcap, c->cand_n + 1));
-  int64_t cap = c->lcap_x;
-  TRY(grow(c, &c->d_lx, cap, c->cand_n + 1));
-  c->lcap_x = cap;
+  TRY(list_capacity(c, c->cand_n + 1));
   a.R = R;
   a.rowstat = c->d_rowstat;
   a.list_r0 = 0;
@@ -1515,14 +1528,14 @@ static emc_status build_rows(emc_context* c, const float* M, int64_t rows, int64
   for (int64_t r = 0; r < rows; ++r) ptr[r + 1] = ptr[r] + cnt[r];
   const int64_t nnz = ptr[rows];
   if (nnz + 1 > s.cap || (with_aux && !s.aux)) {
-    for (void* q : {(void*)s.idx, (void*)s.val, (void*)s.aux})
+    for (void* q : {(void*)s.idx, (void*)s.aux})
       if (q) c->release(q);
     s.idx = nullptr;
     s.val = nullptr;
     s.aux = nullptr;
     s.cap = 0;
-    TRY(c->alloc(&s.idx, nnz + 1));
-    TRY(c->alloc(&s.val, nnz + 1));
+    TRY(c->alloc(&s.idx, 2 * (nnz + 1)));
+    s.val = reinterpret_cast<float*>(s.idx + nnz + 1);
     if (with_aux) TRY(c->alloc(&s.aux, nnz + 1));
     s.cap = nnz + 1;
   }
@@ -1874,13 +1887,14 @@ emc_status emc_compress(emc_context* c) {
 // What a waited-for call reads back: the status word of the device-side waits
 // and, with stats, the statistics and T_r, in pinned memory behind one wait.
 struct HostBack {
-  TcStatus status;
   double stats[4];
+  TcStatus status;
 };
 static emc_status read_back(emc_context* c, HostBack** out, float** T) {
-  HostBack* h = c->pinned<HostBack>(9, 1);
-  float* t = T ? c->pinned<float>(10, c->R) : nullptr;
-  if (!h || (T && !t)) return c->fail(EMC_ERR_OOM, "pinned host staging");
+  char* q = host_back(c);
+  if (!q) return c->fail(EMC_ERR_OOM, "pinned host staging");
+  HostBack* h = reinterpret_cast<HostBack*>(q + 16);
+  float* t = reinterpret_cast<float*>(h + 1);
   CK(c, cudaMemcpyAsync(&h->status, c->d_status, sizeof(TcStatus), cudaMemcpyDeviceToHost, c->st));
   if (T) {
     CK(c, cudaMemcpyAsync(h->stats, c->d_stats, sizeof(h->stats), cudaMemcpyDeviceToHost, c->st));
@@ -2948,17 +2962,10 @@ static emc_status run_proposed(emc_context* c, const ProposedPlan& pl, Select se
     c->mark(2);
     CK(c, launch_group_softmax(g, c->st));
     if (lists) {
-      if (!c->d_lrowoff) {
-        TRY(c->alloc(&c->d_lrowtot, R + 1));
-        TRY(c->alloc(&c->d_lrowoff, R + 1));
-      }
-      if (!c->d_lcursor) TRY(c->alloc(&c->d_lcursor, R));
+      TRY(list_buffers(c));
       // a list entry is an evaluated (rotation, pattern) pair: `evals` bounds
       // their number, so the lists need no count from the device
-      TRY(grow(c, &c->d_lpat, c->lcap, evals + 1));
-      int64_t cap = c->lcap_x;
-      TRY(grow(c, &c->d_lx, cap, evals + 1));
-      c->lcap_x = cap;
+      TRY(list_capacity(c, evals + 1));
       CK(c, launch_group_list_count(g, kListRel, c->d_lrowtot, c->st));
       CK(c, launch_list_alloc(c->d_lrowtot, R, c->d_lrowoff, c->d_lcursor, c->st));
       CK(c, launch_group_list_fill(g, kListRel, c->d_lcursor, c->d_lpat, c->d_lx, c->st));
