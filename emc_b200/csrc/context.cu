@@ -186,6 +186,7 @@ struct emc_context {
   float* d_T = nullptr;
   float* d_Tskip = nullptr;  // T_r for the insertion skip: this context's T, or all shards' sum
   double* d_rowstat = nullptr;
+  double* d_statpart = nullptr;  // the expansion's partials of d_rowstat (FP32: and d_rowmax)
   uint2* d_vtab = nullptr;  // mixed + nearest: per-voxel (W, split operand) table of the expand
   float4* d_tri = nullptr;  // trilinear: the expansion's stencil table (8 corners per base voxel)
   double* d_scratch = nullptr;  // reductions
@@ -691,6 +692,9 @@ static emc_status alloc_work(emc_context* c) {
   const int64_t R = c->R, N = c->N, npa = c->npa;
   if (c->cfg.interp == EMC_INTERP_TRILINEAR)
     TRY(c->alloc(&c->d_tri, tri_table_entries(c->cfg.side)));
+  // (FP32 contexts: half as many again for the row maxima)
+  const int64_t parts = expand_parts(c->mixed ? round_up(npa, 256) : npa) * R;
+  TRY(c->alloc(&c->d_statpart, c->mixed ? parts : parts + (parts + 1) / 2));
   if (!c->mixed) {
     TRY(c->alloc(&c->d_S, R * npa));
     TRY(c->alloc(&c->d_LL, R * N));
@@ -704,9 +708,12 @@ static emc_status alloc_work(emc_context* c) {
     const int64_t chunk = resp_f32_chunk(R, N), nparts = (R + chunk - 1) / chunk;
     const int64_t nb = resp_f32_blocks(N);
     double* w = nullptr;
-    TRY(c->alloc(&w, 4 * nparts * N + nb * R + 2 * N + (nb * R + R + 1) / 2));
+    // (the partials' room also serves the CUDA-core cross term, ceil(R / 128) a
+    // pattern)
+    const int64_t part = std::max(4 * nparts, (R + 127) / 128) * N;
+    TRY(c->alloc(&w, part + nb * R + 2 * N + (nb * R + R + 1) / 2));
     c->d_part64 = reinterpret_cast<double4*>(w);
-    c->d_Tpart64 = w + 4 * nparts * N;
+    c->d_Tpart64 = w + part;
     c->d_plogp32 = c->d_Tpart64 + nb * R;
     c->d_lse32 = c->d_plogp32 + N;
     c->d_Mpart = reinterpret_cast<float*>(c->d_lse32 + N);
@@ -1076,12 +1083,14 @@ emc_status emc_expand(emc_context* c) {
   a.interp = c->cfg.interp;
   a.floor_ = c->cfg.poisson_floor;
   a.rowstat = c->d_rowstat;
+  a.statpart = c->d_statpart;
   if (!c->mixed) {
     a.ld = c->npa;
     a.out = c->gauss ? EXP_F32 : EXP_LOG_F32;
     a.stat = c->gauss ? STAT_SUMSQ : STAT_SUM;
     a.out_f32 = c->d_S;
     a.rowmax = c->d_rowmax;
+    a.maxpart = reinterpret_cast<float*>(c->d_statpart + expand_parts(c->npa) * c->R);
   } else {
     a.ld = c->Ppad;
     a.out = EXP_F16_SPLIT;
@@ -1103,7 +1112,7 @@ emc_status emc_expand(emc_context* c) {
     c->launches += 1;
   }
   CK(c, launch_expand(a, c->st));
-  c->launches += 1;
+  c->launches += 2;
   c->mark(1);
   c->stage = 1;
   return EMC_OK;

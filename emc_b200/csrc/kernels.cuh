@@ -17,7 +17,6 @@ struct ExpandArgs {
   const float* cx;      // [npix] pixel coordinates (compact or full grid)
   const float* cy;
   const float* cz;
-  const int32_t* stat_mask;  // pixels counted in the row statistic (nullptr: all)
   int64_t R, npix, ld;  // ld: output row stride in elements (>= npix; extra columns zeroed)
   int side, interp;
   int out;              // ExpandOut
@@ -27,14 +26,17 @@ struct ExpandArgs {
   float* out_f32;
   __half* out_hi;
   __half* out_lo;
-  double* rowstat;      // [R] or nullptr
+  double* rowstat;      // [R] (stat != STAT_NONE)
   float* rowmax;        // [R] largest magnitude of the row's output, or nullptr (FP32 outputs)
-  // optional, nearest + EXP_F16_SPLIT: per-voxel table from launch_expand_table
+  double* statpart;     // scratch of rowstat, and
+  float* maxpart;       // of rowmax: [expand_parts(ld)][R]
+  // nearest + EXP_F16_SPLIT: per-voxel table from launch_expand_table
   // ([side^3 + 1], the last entry for pixels that fall outside the grid)
   const uint2* tab;
   // optional, trilinear: the stencil table of launch_tri_table
   const float4* tri;
 };
+int64_t expand_parts(int64_t ld);
 cudaError_t launch_expand(const ExpandArgs& a, cudaStream_t st);
 // Trilinear stencil table: per base voxel of [-1, side)^3 the model at its 8
 // corners (0 outside the grid), tri_table_entries(side) float4.

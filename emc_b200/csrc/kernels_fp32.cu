@@ -53,8 +53,8 @@ __device__ float block_max(float v, float* red) {
 }
 
 // ------------------------------------------------------------------ expand --
-// One block per rotation; threads stride over pixels.  emc_cuda.cu:51-111 for
-// the nearest mode (exclusive lower bound), trilinear otherwise.
+// emc_cuda.cu:51-111 for the nearest mode (exclusive lower bound), trilinear
+// otherwise.
 // Slice value W at continuous voxel position u (0 outside the grid).
 template <int INTERP>
 __device__ __forceinline__ float gather(const float* __restrict__ model, const float* u, int side) {
@@ -117,66 +117,6 @@ __global__ void tri_table_kernel(const float* __restrict__ model, int side, floa
   tri[2 * e + 1] = make_float4(v[4], v[5], v[6], v[7]);
 }
 
-// Four pixels per thread and iteration: their gathers are independent, so
-// four L2 round trips are in flight per thread.
-constexpr int kExpandUnroll = 4;
-template <int INTERP, int OUT>
-__global__ void __launch_bounds__(kBlock) expand_kernel(const ExpandArgs a) {
-  __shared__ double red[32];
-  const int64_t r = blockIdx.x;
-  float m[9];
-  emc_voxel::rotation_matrix(a.quat + 4 * r, m);
-  double stat = 0.0;
-  float big = 0.0f;
-  const int64_t step = (int64_t)blockDim.x * kExpandUnroll;
-  for (int64_t i0 = threadIdx.x; i0 < a.ld; i0 += step) {
-    float w[kExpandUnroll];
-#pragma unroll
-    for (int u = 0; u < kExpandUnroll; ++u) {
-      const int64_t i = i0 + (int64_t)u * blockDim.x;
-      w[u] = 0.0f;
-      if (i < a.npix) {
-        float pos[3];
-        emc_voxel::position(m, a.side, __ldg(a.cx + i), __ldg(a.cy + i), __ldg(a.cz + i), pos);
-        w[u] = (INTERP == 1 && a.tri) ? gather_tri(a.tri, pos, a.side)
-                                      : gather<INTERP>(a.model, pos, a.side);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kExpandUnroll; ++u) {
-      const int64_t i = i0 + (int64_t)u * blockDim.x;
-      if (i < a.ld) {
-        const bool real = i < a.npix;
-        if (real && a.stat != STAT_NONE && (!a.stat_mask || a.stat_mask[i] != 0))
-          stat += a.stat == STAT_SUMSQ ? (double)w[u] * w[u] : (double)w[u];
-        const int64_t o = r * a.ld + i;
-        if (OUT == EXP_F32) {
-          a.out_f32[o] = w[u];
-          big = fmaxf(big, fabsf(w[u]));
-        } else if (OUT == EXP_LOG_F32) {
-          const float x = real ? logf(fmaxf(w[u], a.floor_)) : 0.0f;
-          a.out_f32[o] = x;
-          big = fmaxf(big, fabsf(x));
-        } else {
-          const float x = real ? (a.log_split ? logf(fmaxf(w[u], a.floor_)) : w[u]) : 0.0f;
-          const __half hi = __float2half_rn(x);
-          a.out_hi[o] = hi;
-          a.out_lo[o] = __float2half_rn(x - __half2float(hi));
-        }
-      }
-    }
-  }
-  if (a.rowstat) {
-    const double s = block_sum(stat, red);
-    if (threadIdx.x == 0) a.rowstat[r] = s;
-  }
-  if (a.rowmax) {
-    __syncthreads();  // red is free again
-    const float mx = block_max(big, reinterpret_cast<float*>(red));
-    if (threadIdx.x == 0) a.rowmax[r] = mx;
-  }
-}
-
 // The operand value of the split expansion and its FP16 hi / lo halves,
 // packed hi | lo << 16.
 __device__ __forceinline__ uint32_t split_bits(float w, float floor_, int log_split) {
@@ -194,56 +134,161 @@ __global__ void expand_table_kernel(const float* model, int64_t M, float floor_,
   tab[v] = make_uint2(__float_as_uint(w), split_bits(w, floor_, log_split));
 }
 
-// Nearest-voxel expansion into the FP16 hi + lo operands through the voxel
-// table: one 8-byte gather per pixel gives the slice value (for the row
-// statistic) and its split operand, so no logarithm or split runs per
-// element; each thread takes pixel pairs and writes them as half2.  Outputs
-// are those of expand_kernel<0, EXP_F16_SPLIT> bit for bit.
-__global__ void __launch_bounds__(kBlock) expand_tab_kernel(const ExpandArgs a) {
-  __shared__ double red[32];
-  const int64_t r = blockIdx.x;
-  float m[9];
-  emc_voxel::rotation_matrix(a.quat + 4 * r, m);
-  const int M = a.side * a.side * a.side;  // side <= 1024
-  const int npix = (int)a.npix, npairs = (int)(a.ld / 2);
-  __half2* hi_row = reinterpret_cast<__half2*>(a.out_hi + r * a.ld);
-  __half2* lo_row = reinterpret_cast<__half2*>(a.out_lo + r * a.ld);
-  double stat = 0.0;
-  for (int p0 = threadIdx.x; p0 < npairs; p0 += 2 * kBlock) {
-    uint2 t[4];
+// A block expands `rot` <= 16 consecutive rotations over 256 pixels (of each of
+// its `per` chunks of the detector): a thread keeps its two pixels' coordinates in
+// registers and walks the rotations, four at a time, so eight gathers are in
+// flight.  The gathers bound it: an SM asks the L2 for about one sector a
+// clock.  Consecutive rotations of the samplings are neighbours, so what one
+// of them gathered for a compact patch of pixels (contexts list them along a
+// Morton curve) is often in L1 for the next, and neither coordinates nor
+// rotation matrices are loaded per pixel.  A block per rotation, as before,
+// found 19% of its gathers in L1; 86,520 rotations x 16,384 pixels, nearest,
+// through the table: 5.0 -> 3.9 ms; 25,680 x 4,096: 0.36 -> 0.29 ms.
+//
+// Row statistics leave as one FP64 partial per (chunk group, rotation), summed
+// in order by expand_rows_kernel, so they do not depend on the blocks' order.
+constexpr int kExpThreads = 128, kExpChunk = 256, kExpRot = 16, kExpParts = 64;
+
+template <int INTERP, int OUT>
+__global__ void __launch_bounds__(kExpThreads) expand_kernel(const ExpandArgs a, int rot,
+                                                             int groups, int per) {
+  __shared__ float4 ms[kExpRot][3];
+  __shared__ double red[kExpThreads / 32][kExpRot];
+  __shared__ uint32_t big[kExpThreads / 32][kExpRot];
+  constexpr bool kHalf = OUT == EXP_F16_SPLIT;
+  constexpr int kStep = INTERP == 0 ? 4 : 2;  // rotations in flight
+  const int64_t rg = blockIdx.x / groups, r0 = rg * rot;
+  const int cg = (int)(blockIdx.x - rg * groups);
+  const int nr = (int)(a.R - r0 < rot ? a.R - r0 : rot);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (threadIdx.x < nr) {
+    float m[9];
+    emc_voxel::rotation_matrix(a.quat + 4 * (r0 + threadIdx.x), m);
+    ms[threadIdx.x][0] = make_float4(m[0], m[1], m[2], 0.0f);
+    ms[threadIdx.x][1] = make_float4(m[3], m[4], m[5], 0.0f);
+    ms[threadIdx.x][2] = make_float4(m[6], m[7], m[8], 0.0f);
+  }
+  for (int k = lane; k < kExpRot; k += 32) {
+    red[w][k] = 0.0;
+    big[w][k] = 0;
+  }
+  __syncthreads();
+  const int M = a.side * a.side * a.side;  // side <= 1290
+  const int npix = (int)a.npix, ld = (int)a.ld;
+  for (int c = cg * per; c < cg * per + per && c * kExpChunk < ld; ++c) {
+    // two adjacent pixels (stored as half2), or two 128 apart (FP32 rows)
+    int px[2];
+    float x[2], y[2], z[2];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = 2 * (p0 + (u >> 1) * kBlock) + (u & 1);
-      t[u] = make_uint2(0u, 0u);  // padding columns: zero
-      if (i < npix) {
-        float pos[3];
-        emc_voxel::position(m, a.side, __ldg(a.cx + i), __ldg(a.cy + i), __ldg(a.cz + i), pos);
-        int v;
-        if (!emc_voxel::nearest32(pos, a.side, 1, &v)) v = M;
-        t[u] = __ldg(a.tab + v);
+    for (int u = 0; u < 2; ++u) {
+      px[u] = c * kExpChunk + (kHalf ? 2 * threadIdx.x + u : threadIdx.x + u * kExpThreads);
+      const bool in = px[u] < npix;
+      x[u] = in ? a.cx[px[u]] : 0.0f;
+      y[u] = in ? a.cy[px[u]] : 0.0f;
+      z[u] = in ? a.cz[px[u]] : 0.0f;
+    }
+#pragma unroll 1
+    for (int k0 = 0; k0 < nr; k0 += kStep) {
+      double st[kStep];
+      uint32_t mx[kStep];
+#pragma unroll
+      for (int kk = 0; kk < kStep; ++kk) {
+        const int k = k0 + kk;
+        st[kk] = 0.0;
+        mx[kk] = 0;
+        if (k >= nr) continue;
+        const float4 m0 = ms[k][0], m1 = ms[k][1], m2 = ms[k][2];
+        const float m[9] = {m0.x, m0.y, m0.z, m1.x, m1.y, m1.z, m2.x, m2.y, m2.z};
+        float v[2];
+        uint32_t b[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          v[u] = 0.0f;
+          b[u] = 0;
+          if (px[u] >= npix) continue;  // padding columns: zero
+          float pos[3];
+          emc_voxel::position(m, a.side, x[u], y[u], z[u], pos);
+          if constexpr (INTERP == 0 && kHalf) {
+            int vox;
+            if (!emc_voxel::nearest32(pos, a.side, 1, &vox)) vox = M;
+            const uint2 t = __ldg(a.tab + vox);
+            v[u] = __uint_as_float(t.x);
+            b[u] = t.y;
+          } else {
+            v[u] = (INTERP == 1 && a.tri) ? gather_tri(a.tri, pos, a.side)
+                                          : gather<INTERP>(a.model, pos, a.side);
+            if constexpr (kHalf) b[u] = split_bits(v[u], a.floor_, a.log_split);
+          }
+        }
+        if (a.stat != STAT_NONE)
+          st[kk] = a.stat == STAT_SUMSQ ? (double)v[0] * v[0] + (double)v[1] * v[1]
+                                        : (double)v[0] + (double)v[1];
+        const int64_t row = (r0 + k) * a.ld;
+        if constexpr (kHalf) {
+          if (px[0] < ld) {  // ld is even
+            *reinterpret_cast<uint32_t*>(a.out_hi + row + px[0]) = __byte_perm(b[0], b[1], 0x5410);
+            *reinterpret_cast<uint32_t*>(a.out_lo + row + px[0]) = __byte_perm(b[0], b[1], 0x7632);
+          }
+        } else {
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            if (px[u] >= ld) continue;
+            const float o = OUT == EXP_LOG_F32 && px[u] < npix ? logf(fmaxf(v[u], a.floor_)) : v[u];
+            a.out_f32[row + px[u]] = o;
+            mx[kk] = max(mx[kk], __float_as_uint(fabsf(o)));
+          }
+        }
+      }
+      if (a.stat != STAT_NONE) {
+        // kStep row sums by halving exchanges
+#pragma unroll
+        for (int o = 16, n = kStep / 2; n >= 1; o >>= 1, n >>= 1) {
+          const bool hi = lane & o;
+#pragma unroll
+          for (int q = 0; q < n; ++q) {
+            const double keep = hi ? st[q + n] : st[q], send = hi ? st[q] : st[q + n];
+            st[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+          }
+        }
+#pragma unroll
+        for (int o = 16 / kStep; o > 0; o >>= 1) st[0] += __shfl_xor_sync(0xffffffffu, st[0], o);
+        if (lane % (32 / kStep) == 0) red[w][k0 + lane / (32 / kStep)] += st[0];
+      }
+      if (!kHalf && a.rowmax) {
+#pragma unroll
+        for (int kk = 0; kk < kStep; ++kk) {
+          const uint32_t q = __reduce_max_sync(0xffffffffu, mx[kk]);
+          if (lane == 0) big[w][k0 + kk] = max(big[w][k0 + kk], q);
+        }
       }
     }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int pp = p0 + h * kBlock;
-      if (pp >= npairs) continue;
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-        if (2 * pp + e < npix && a.stat != STAT_NONE) {
-          const float w = __uint_as_float(t[2 * h + e].x);
-          stat += a.stat == STAT_SUMSQ ? (double)w * w : (double)w;
-        }
-      const uint32_t b0 = t[2 * h].y, b1 = t[2 * h + 1].y;
-      hi_row[pp] = __halves2half2(__ushort_as_half((unsigned short)(b0 & 0xFFFFu)),
-                                  __ushort_as_half((unsigned short)(b1 & 0xFFFFu)));
-      lo_row[pp] = __halves2half2(__ushort_as_half((unsigned short)(b0 >> 16)),
-                                  __ushort_as_half((unsigned short)(b1 >> 16)));
+  }
+  if (a.stat == STAT_NONE && !a.rowmax) return;
+  __syncthreads();
+  if (threadIdx.x < nr) {
+    double s = 0.0;
+    uint32_t q = 0;
+    for (int i = 0; i < kExpThreads / 32; ++i) {
+      s += red[i][threadIdx.x];
+      q = max(q, big[i][threadIdx.x]);
     }
+    const int64_t o = (int64_t)cg * a.R + r0 + threadIdx.x;
+    if (a.stat != STAT_NONE) a.statpart[o] = s;
+    if (a.rowmax) a.maxpart[o] = __uint_as_float(q);
   }
-  if (a.rowstat) {
-    const double s = block_sum(stat, red);
-    if (threadIdx.x == 0) a.rowstat[r] = s;
+}
+
+__global__ void expand_rows_kernel(const ExpandArgs a, int groups) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= a.R) return;
+  double s = 0.0;
+  float mx = 0.0f;
+  for (int g = 0; g < groups; ++g) {
+    if (a.stat != STAT_NONE) s += a.statpart[g * a.R + r];
+    if (a.rowmax) mx = fmaxf(mx, a.maxpart[g * a.R + r]);
   }
+  if (a.stat != STAT_NONE) a.rowstat[r] = s;
+  if (a.rowmax) a.rowmax[r] = mx;
 }
 
 __device__ __forceinline__ int64_t col_of(const int32_t* pix, int64_t j) { return pix ? pix[j] : j; }
@@ -434,8 +479,19 @@ __device__ __forceinline__ void stat_rescale(StatAcc& a, double m) {
     a.m = m;
   }
 }
+__device__ __forceinline__ void stat_merge(StatAcc& a, const StatAcc& b) {
+  if (b.m <= -DBL_MAX) return;
+  stat_rescale(a, b.m);
+  const double f = exp(b.m - a.m);
+  a.q += f > 0.0 ? f * (b.q + (b.m - a.m) * b.s) : 0.0;
+  a.s += f * b.s;
+  a.d += f * b.d;
+}
+
 // The eight warps' sums of one pattern (lane), relative to their common
-// maximum: one exponential per thread, the total on warp 0.
+// maximum: one exponential per thread, the total on warp 0.  (The stats sweep
+// merges them one after the other on warp 0 instead: with this reduction in it
+// its main loop compiled to 1.14 instead of 0.74 ms at 10,000 x 25,680.)
 __device__ __forceinline__ void stat_reduce(StatAcc& a, double (&sh)[4][8][32], int w, int lane) {
   sh[0][w][lane] = a.m;
   __syncthreads();
@@ -459,7 +515,7 @@ __device__ __forceinline__ void stat_reduce(StatAcc& a, double (&sh)[4][8][32], 
 
 template <bool POISSON>
 __global__ void __launch_bounds__(256) resp_stats_kernel(const RespF32Args a) {
-  __shared__ double sh[4][8][32];
+  __shared__ double sh[8][32][4];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t cols = (a.N + 31) / 32, by = blockIdx.x / cols;
   const int64_t p = (blockIdx.x - by * cols) * 32 + lane;
@@ -500,8 +556,16 @@ __global__ void __launch_bounds__(256) resp_stats_kernel(const RespF32Args a) {
     acc.d += (double)d;
     acc.q += (double)q;
   }
-  stat_reduce(acc, sh, w, lane);
-  if (w == 0 && ok) a.part[by * a.N + p] = make_double4(acc.m, acc.s, acc.d, acc.q);
+  sh[w][lane][0] = acc.m;
+  sh[w][lane][1] = acc.s;
+  sh[w][lane][2] = acc.d;
+  sh[w][lane][3] = acc.q;
+  __syncthreads();
+  if (w == 0 && ok) {
+    for (int k = 1; k < 8; ++k)
+      stat_merge(acc, StatAcc{sh[k][lane][0], sh[k][lane][1], sh[k][lane][2], sh[k][lane][3]});
+    a.part[by * a.N + p] = make_double4(acc.m, acc.s, acc.d, acc.q);
+  }
 }
 
 __global__ void __launch_bounds__(256) resp_combine_kernel(const RespF32Args a) {
@@ -916,27 +980,44 @@ inline int grid_for(int64_t n) {
 // ------------------------------------------------------------- launchers --
 
 template <int INTERP>
-void expand_dispatch(const ExpandArgs& a, cudaStream_t st) {
+static void expand_dispatch(const ExpandArgs& a, unsigned grid, int rot, int groups, int per,
+                            cudaStream_t st) {
   if (a.out == EXP_F32)
-    expand_kernel<INTERP, EXP_F32><<<(unsigned)a.R, kBlock, 0, st>>>(a);
+    expand_kernel<INTERP, EXP_F32><<<grid, kExpThreads, 0, st>>>(a, rot, groups, per);
   else if (a.out == EXP_LOG_F32)
-    expand_kernel<INTERP, EXP_LOG_F32><<<(unsigned)a.R, kBlock, 0, st>>>(a);
+    expand_kernel<INTERP, EXP_LOG_F32><<<grid, kExpThreads, 0, st>>>(a, rot, groups, per);
   else
-    expand_kernel<INTERP, EXP_F16_SPLIT><<<(unsigned)a.R, kBlock, 0, st>>>(a);
+    expand_kernel<INTERP, EXP_F16_SPLIT><<<grid, kExpThreads, 0, st>>>(a, rot, groups, per);
 }
 
+int64_t expand_parts(int64_t ld) {
+  const int64_t chunks = (ld + kExpChunk - 1) / kExpChunk;
+  return chunks < kExpParts ? chunks : kExpParts;
+}
+
+// The voxel index is 32 bits wide (nearest32), so side^3 must fit.
 cudaError_t launch_expand(const ExpandArgs& a, cudaStream_t st) {
   if (a.R <= 0) return cudaSuccess;
-  if (a.tab && a.interp == 0 && a.out == EXP_F16_SPLIT) {
-    if (a.ld % 2 != 0 || a.npix > a.ld || a.ld > (int64_t)1 << 30 || a.stat_mask)
-      return cudaErrorInvalidValue;
-    expand_tab_kernel<<<(unsigned)a.R, kBlock, 0, st>>>(a);
-    return cudaGetLastError();
-  }
+  if (a.npix > a.ld || a.ld > (int64_t)1 << 30 || a.side > 1290 ||
+      (a.out == EXP_F16_SPLIT && (a.ld % 2 != 0 || a.rowmax || (a.interp == 0 && !a.tab))) ||
+      (a.stat != STAT_NONE && !(a.rowstat && a.statpart)) || (a.rowmax && !a.maxpart))
+    return cudaErrorInvalidValue;
+  const int64_t chunks = (a.ld + kExpChunk - 1) / kExpChunk;
+  const int per = (int)((chunks + kExpParts - 1) / kExpParts);
+  const int groups = (int)((chunks + per - 1) / per);
+  // Fewer rotations a block where 16 would not give each SM four blocks: 1,000
+  // rotations x 1,024 pixels is 252 blocks of 16, and one wave of them lasts as
+  // long as 16 rotations take in a row.
+  int rot = kExpRot;
+  while (rot > 4 && groups * ((a.R + rot - 1) / rot) < 4 * 148) rot /= 2;
+  const int64_t grid = groups * ((a.R + rot - 1) / rot);
+  if (grid > 2147483647) return cudaErrorInvalidConfiguration;
   if (a.interp == 0)
-    expand_dispatch<0>(a, st);
+    expand_dispatch<0>(a, (unsigned)grid, rot, groups, per, st);
   else
-    expand_dispatch<1>(a, st);
+    expand_dispatch<1>(a, (unsigned)grid, rot, groups, per, st);
+  if (a.stat != STAT_NONE || a.rowmax)
+    expand_rows_kernel<<<(unsigned)((a.R + 255) / 256), 256, 0, st>>>(a, groups);
   return cudaGetLastError();
 }
 
@@ -1180,7 +1261,7 @@ int64_t resp_f32_chunk(int64_t R, int64_t N) {
   const int64_t most = (R + 63) / 64;
   if (parts > most) parts = most;
   int64_t chunk = (R + parts - 1) / parts;
-  if (chunk > 512) chunk = 512;  // the partials then also hold ceil(R / 128) doubles per pattern
+  if (chunk > 2048) chunk = 2048;
   return (chunk + 63) / 64 * 64;
 }
 
