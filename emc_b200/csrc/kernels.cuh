@@ -30,8 +30,8 @@ struct ExpandArgs {
   float* rowmax;        // [R] largest magnitude of the row's output, or nullptr (FP32 outputs)
   double* statpart;     // scratch of rowstat, and
   float* maxpart;       // of rowmax: [expand_parts(ld)][R]
-  // nearest + EXP_F16_SPLIT: per-voxel table from launch_expand_table
-  // ([side^3 + 1], the last entry for pixels that fall outside the grid)
+  // nearest: per-voxel table from launch_expand_table (EXP_F16_SPLIT needs it,
+  // EXP_LOG_F32 can do without)
   const uint2* tab;
   // optional, trilinear: the stencil table of launch_tri_table
   const float4* tri;
@@ -42,10 +42,13 @@ cudaError_t launch_expand(const ExpandArgs& a, cudaStream_t st);
 // corners (0 outside the grid), tri_table_entries(side) float4.
 int64_t tri_table_entries(int side);
 cudaError_t launch_tri_table(const float* model, int side, float4* tri, cudaStream_t st);
-// tab[v] = (bits of model[v], FP16 hi | lo << 16 of the split operand value:
-// log(max(model[v], floor)) when log_split, else model[v]) for v < M, and
-// tab[M] the same for a pixel outside the grid (value 0).
-cudaError_t launch_expand_table(const float* model, int64_t M, float floor_, int log_split,
+// Per voxel, in the order of the kernel's table_entry: (bits of model[v], the
+// output value) and at the end the same for a pixel outside the grid (value 0)
+// and for a column past the last pixel.  The output value is the bits of
+// log(max(model[v], floor)) for EXP_LOG_F32; for EXP_F16_SPLIT, FP16 hi | lo << 16
+// of that (log_split) or of model[v].
+int64_t expand_table_entries(int side);
+cudaError_t launch_expand_table(const float* model, int side, int out, float floor_, int log_split,
                                 uint2* tab, cudaStream_t st);
 
 // LL[r][p] (ld = ldLL) from slices A[R][ldA] and counts K[N][ldK] over npa

@@ -55,12 +55,31 @@ __device__ float block_max(float v, float* red) {
 // ------------------------------------------------------------------ expand --
 // emc_cuda.cu:51-111 for the nearest mode (exclusive lower bound), trilinear
 // otherwise.
+
+// The nearest voxel (emc_voxel::nearest with lower bound 1) less one in each
+// coordinate, false outside [1, side).  Rounding half away from zero is
+// truncation of u + 1/2 where a voxel below 1 is outside anyway; that sum is
+// rounded toward zero, so no u below a half reaches 1, and adding 2^23 leaves the
+// whole number in the low bits.  Whatever is out of range, NaN included, gives a
+// larger unsigned number.  Three instructions a coordinate, where roundf and its
+// conversion to an integer (a unit that takes a warp every eight clocks) took
+// seven: the expansion was bound by its instructions, 80 a pixel.  The same in
+// the insertions and in the trilinear expansion changed nothing.
+__device__ __forceinline__ bool nearest_from_1(const float* u, int side, uint32_t* k) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    k[i] = __float_as_uint(__fadd_rz(__fadd_rz(u[i], 0.5f), 8388608.0f)) - 0x4b000001u;
+  return max(max(k[0], k[1]), k[2]) < (uint32_t)(side - 1);
+}
+
 // Slice value W at continuous voxel position u (0 outside the grid).
 template <int INTERP>
 __device__ __forceinline__ float gather(const float* __restrict__ model, const float* u, int side) {
   if (INTERP == 0) {
-    int v;
-    return emc_voxel::nearest32(u, side, 1, &v) ? __ldg(model + v) : 0.0f;
+    uint32_t k[3];
+    return nearest_from_1(u, side, k)
+               ? __ldg(model + (((int)k[2] + 1) * side + (int)k[1] + 1) * side + (int)k[0] + 1)
+               : 0.0f;
   }
   float acc = 0.0f;
 #pragma unroll
@@ -126,30 +145,62 @@ __device__ __forceinline__ uint32_t split_bits(float w, float floor_, int log_sp
   return (uint32_t)__half_as_ushort(hi) | ((uint32_t)__half_as_ushort(lo) << 16);
 }
 
-__global__ void expand_table_kernel(const float* model, int64_t M, float floor_, int log_split,
+// The table's order, coordinates less one (voxels below 1 are never read):
+// squares of 2 x 2 voxels in (y, z), 32 bytes each, along x, so a cache line
+// holds 4 x 2 x 2 voxels.  A warp's pixels lie on a plane of any orientation and
+// meet fewer sectors than with rows of voxels, which a plane across x meets
+// one voxel at a time (86,520 rotations x 16,384 pixels: 3.9 -> 3.6 ms).
+__host__ __device__ __forceinline__ int table_outside(int side) {
+  return 4 * (side >> 1) * (side >> 1) * side;
+}
+__device__ __forceinline__ int table_entry(int x, int y, int z, int side) {
+  // 4 ((z / 2 * (side / 2) + y / 2) * side + x) + 2 (z % 2) + y % 2
+  const int row = 4 * side - 2, plane = 4 * (side >> 1) * side - 4;
+  return (z >> 1) * plane + (y >> 1) * row + 4 * x + 2 * z + y;
+}
+
+template <int OUT>
+__global__ void expand_table_kernel(const float* model, int side, float floor_, int log_split,
                                     uint2* tab) {
-  const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v > M) return;
-  const float w = v < M ? model[v] : 0.0f;
-  tab[v] = make_uint2(__float_as_uint(w), split_bits(w, floor_, log_split));
+  auto value = [&](float w) {
+    return OUT == EXP_LOG_F32 ? __float_as_uint(logf(fmaxf(w, floor_)))
+                              : split_bits(w, floor_, log_split);
+  };
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  const int M = side * side * side, end = table_outside(side);
+  if (v >= M) {
+    // a pixel outside the grid; a column past the last pixel
+    if (v == M) tab[end] = make_uint2(0u, value(0.0f));
+    if (v == M + 1) tab[end + 1] = make_uint2(0u, 0u);
+    return;
+  }
+  const int q = v / side, x = v - q * side, z = q / side, y = q - z * side;
+  if (x < 1 || y < 1 || z < 1) return;
+  const float w = model[v];
+  tab[table_entry(x - 1, y - 1, z - 1, side)] =
+      make_uint2(__float_as_uint(w), value(w));
 }
 
 // A block expands `rot` <= 16 consecutive rotations over 256 pixels (of each of
 // its `per` chunks of the detector): a thread keeps its two pixels' coordinates in
 // registers and walks the rotations, four at a time, so eight gathers are in
-// flight.  The gathers bound it: an SM asks the L2 for about one sector a
-// clock.  Consecutive rotations of the samplings are neighbours, so what one
+// flight.  Consecutive rotations of the samplings are neighbours, so what one
 // of them gathered for a compact patch of pixels (contexts list them along a
 // Morton curve) is often in L1 for the next, and neither coordinates nor
 // rotation matrices are loaded per pixel.  A block per rotation, as before,
-// found 19% of its gathers in L1; 86,520 rotations x 16,384 pixels, nearest,
-// through the table: 5.0 -> 3.9 ms; 25,680 x 4,096: 0.36 -> 0.29 ms.
+// found 19% of its gathers in L1.  Nearest, through the table, is bound by its
+// instructions, trilinear by the L2 sector that each pixel takes:
+//   86,520 rotations x 16,384 pixels, FP16 pair   5.0 -> 3.9, with the table's
+//     order 3.6, with nearest_from_1 2.95 ms (5.7 GB written: 0.9 ms)
+//   25,680 x 4,096  0.36 -> 0.29 -> 0.235 ms
+//   25,680 x 12,800, FP32 logarithms 1.77 -> 1.38, with the table 0.98 ms
 //
 // Row statistics leave as one FP64 partial per (chunk group, rotation), summed
 // in order by expand_rows_kernel, so they do not depend on the blocks' order.
 constexpr int kExpThreads = 128, kExpChunk = 256, kExpRot = 16, kExpParts = 64;
 
-template <int INTERP, int OUT>
+// TAB: nearest, through the voxel table.
+template <int INTERP, int OUT, bool TAB>
 __global__ void __launch_bounds__(kExpThreads) expand_kernel(const ExpandArgs a, int rot,
                                                              int groups, int per) {
   __shared__ float4 ms[kExpRot][3];
@@ -173,19 +224,22 @@ __global__ void __launch_bounds__(kExpThreads) expand_kernel(const ExpandArgs a,
     big[w][k] = 0;
   }
   __syncthreads();
-  const int M = a.side * a.side * a.side;  // side <= 1290
+  const int outside = table_outside(a.side);
   const int npix = (int)a.npix, ld = (int)a.ld;
   for (int c = cg * per; c < cg * per + per && c * kExpChunk < ld; ++c) {
     // two adjacent pixels (stored as half2), or two 128 apart (FP32 rows)
     int px[2];
     float x[2], y[2], z[2];
+    int none[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       px[u] = c * kExpChunk + (kHalf ? 2 * threadIdx.x + u : threadIdx.x + u * kExpThreads);
       const bool in = px[u] < npix;
-      x[u] = in ? a.cx[px[u]] : 0.0f;
-      y[u] = in ? a.cy[px[u]] : 0.0f;
-      z[u] = in ? a.cz[px[u]] : 0.0f;
+      // columns past the last pixel are outside the grid (and zero)
+      x[u] = in ? a.cx[px[u]] : NAN;
+      y[u] = in ? a.cy[px[u]] : NAN;
+      z[u] = in ? a.cz[px[u]] : NAN;
+      none[u] = outside + (in ? 0 : 1);
     }
 #pragma unroll 1
     for (int k0 = 0; k0 < nr; k0 += kStep) {
@@ -205,19 +259,23 @@ __global__ void __launch_bounds__(kExpThreads) expand_kernel(const ExpandArgs a,
         for (int u = 0; u < 2; ++u) {
           v[u] = 0.0f;
           b[u] = 0;
-          if (px[u] >= npix) continue;  // padding columns: zero
           float pos[3];
-          emc_voxel::position(m, a.side, x[u], y[u], z[u], pos);
-          if constexpr (INTERP == 0 && kHalf) {
-            int vox;
-            if (!emc_voxel::nearest32(pos, a.side, 1, &vox)) vox = M;
-            const uint2 t = __ldg(a.tab + vox);
+          if constexpr (TAB) {
+            emc_voxel::position(m, a.side, x[u], y[u], z[u], pos);
+            uint32_t e[3];
+            const bool in = nearest_from_1(pos, a.side, e);
+            const uint2 t = __ldg(a.tab + (in ? table_entry(e[0], e[1], e[2], a.side) : none[u]));
             v[u] = __uint_as_float(t.x);
             b[u] = t.y;
           } else {
+            if (px[u] >= npix) continue;
+            emc_voxel::position(m, a.side, x[u], y[u], z[u], pos);
             v[u] = (INTERP == 1 && a.tri) ? gather_tri(a.tri, pos, a.side)
                                           : gather<INTERP>(a.model, pos, a.side);
-            if constexpr (kHalf) b[u] = split_bits(v[u], a.floor_, a.log_split);
+            if (kHalf)
+              b[u] = split_bits(v[u], a.floor_, a.log_split);
+            else
+              b[u] = __float_as_uint(OUT == EXP_LOG_F32 ? logf(fmaxf(v[u], a.floor_)) : v[u]);
           }
         }
         if (a.stat != STAT_NONE)
@@ -233,7 +291,7 @@ __global__ void __launch_bounds__(kExpThreads) expand_kernel(const ExpandArgs a,
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
             if (px[u] >= ld) continue;
-            const float o = OUT == EXP_LOG_F32 && px[u] < npix ? logf(fmaxf(v[u], a.floor_)) : v[u];
+            const float o = __uint_as_float(b[u]);
             a.out_f32[row + px[u]] = o;
             mx[kk] = max(mx[kk], __float_as_uint(fabsf(o)));
           }
@@ -979,15 +1037,10 @@ inline int grid_for(int64_t n) {
 
 // ------------------------------------------------------------- launchers --
 
-template <int INTERP>
-static void expand_dispatch(const ExpandArgs& a, unsigned grid, int rot, int groups, int per,
-                            cudaStream_t st) {
-  if (a.out == EXP_F32)
-    expand_kernel<INTERP, EXP_F32><<<grid, kExpThreads, 0, st>>>(a, rot, groups, per);
-  else if (a.out == EXP_LOG_F32)
-    expand_kernel<INTERP, EXP_LOG_F32><<<grid, kExpThreads, 0, st>>>(a, rot, groups, per);
-  else
-    expand_kernel<INTERP, EXP_F16_SPLIT><<<grid, kExpThreads, 0, st>>>(a, rot, groups, per);
+template <int INTERP, int OUT, bool TAB>
+static void run_expand(const ExpandArgs& a, unsigned grid, int rot, int groups, int per,
+                       cudaStream_t st) {
+  expand_kernel<INTERP, OUT, TAB><<<grid, kExpThreads, 0, st>>>(a, rot, groups, per);
 }
 
 int64_t expand_parts(int64_t ld) {
@@ -995,7 +1048,7 @@ int64_t expand_parts(int64_t ld) {
   return chunks < kExpParts ? chunks : kExpParts;
 }
 
-// The voxel index is 32 bits wide (nearest32), so side^3 must fit.
+// The voxel index is 32 bits wide (nearest_from_1), so side^3 must fit.
 cudaError_t launch_expand(const ExpandArgs& a, cudaStream_t st) {
   if (a.R <= 0) return cudaSuccess;
   if (a.npix > a.ld || a.ld > (int64_t)1 << 30 || a.side > 1290 ||
@@ -1012,10 +1065,14 @@ cudaError_t launch_expand(const ExpandArgs& a, cudaStream_t st) {
   while (rot > 4 && groups * ((a.R + rot - 1) / rot) < 4 * 148) rot /= 2;
   const int64_t grid = groups * ((a.R + rot - 1) / rot);
   if (grid > 2147483647) return cudaErrorInvalidConfiguration;
-  if (a.interp == 0)
-    expand_dispatch<0>(a, (unsigned)grid, rot, groups, per, st);
-  else
-    expand_dispatch<1>(a, (unsigned)grid, rot, groups, per, st);
+  const bool near = a.interp == 0;
+  auto run = a.out == EXP_F32       ? (near ? run_expand<0, EXP_F32, false> : run_expand<1, EXP_F32, false>)
+             : a.out == EXP_LOG_F32 ? (!near   ? run_expand<1, EXP_LOG_F32, false>
+                                       : a.tab ? run_expand<0, EXP_LOG_F32, true>
+                                               : run_expand<0, EXP_LOG_F32, false>)
+                                    : (near ? run_expand<0, EXP_F16_SPLIT, true>
+                                            : run_expand<1, EXP_F16_SPLIT, false>);
+  run(a, (unsigned)grid, rot, groups, per, st);
   if (a.stat != STAT_NONE || a.rowmax)
     expand_rows_kernel<<<(unsigned)((a.R + 255) / 256), 256, 0, st>>>(a, groups);
   return cudaGetLastError();
@@ -1029,10 +1086,17 @@ cudaError_t launch_tri_table(const float* model, int side, float4* tri, cudaStre
   return cudaGetLastError();
 }
 
-cudaError_t launch_expand_table(const float* model, int64_t M, float floor_, int log_split,
+int64_t expand_table_entries(int side) { return (int64_t)table_outside(side) + 2; }
+
+cudaError_t launch_expand_table(const float* model, int side, int out, float floor_, int log_split,
                                 uint2* tab, cudaStream_t st) {
-  expand_table_kernel<<<(unsigned)((M + 1 + 255) / 256), 256, 0, st>>>(model, M, floor_, log_split,
-                                                                      tab);
+  const int64_t M = (int64_t)side * side * side;
+  if (out == EXP_LOG_F32)
+    expand_table_kernel<EXP_LOG_F32><<<(unsigned)((M + 2 + 255) / 256), 256, 0, st>>>(
+        model, side, floor_, log_split, tab);
+  else
+    expand_table_kernel<EXP_F16_SPLIT><<<(unsigned)((M + 2 + 255) / 256), 256, 0, st>>>(
+        model, side, floor_, log_split, tab);
   return cudaGetLastError();
 }
 

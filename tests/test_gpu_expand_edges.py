@@ -12,6 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("prec,lik,interp", [("fp32", "gauss", "nearest"), ("fp32", "poisson", "trilinear"),
+                                             ("fp32", "poisson", "nearest"),
                                              ("mixed", "poisson", "nearest"),
                                              ("mixed", "gauss", "trilinear")])
 @pytest.mark.parametrize("side,R,npa", [(16, 1, 1), (17, 3, 255), (17, 17, 257), (19, 33, 361),
@@ -49,3 +50,34 @@ def test_slices_and_row_sums(prec, lik, interp, side, R, npa):
         want = counts[:, act].sum(1) / (P.T @ ref.sum(1))
         # trilinear weights are FP32 products; the sums themselves are FP64
         np.testing.assert_allclose(phi, want, rtol=2e-6)
+
+
+@pytest.mark.parametrize("side", [2, 15, 16, 37])
+def test_table_gives_the_voxels_themselves(side):
+    """FP32 poisson reads (W, log W) from a table where there is room for it;
+    without room, the model and the logarithm: the same bits."""
+    import emc_b200 as E
+    rng = np.random.default_rng(side)
+    # any pixel positions, many of them on the rounding's halves and the edges
+    n = side * side
+    x, y, z = (rng.integers(-side, side + 1, n).astype(np.float32) * np.float32(0.5) for _ in range(3))
+    q, w = E.generate_rotations(3)
+    q = q[:200].copy()
+    q[0] = [1, 0, 0, 0]  # the identity keeps the halves
+    counts = np.ones((3, n), np.float32)
+    model = rng.random(side ** 3).astype(np.float32)
+    out = []
+    for limit in (False, True):
+        with E.Context(side, 3, len(q), likelihood="poisson") as ctx:
+            ctx.set_geometry(x, y, z, np.ones(n, np.int32))
+            ctx.set_rotations(q, w[:200].copy())
+            ctx.set_patterns(counts)
+            ctx.set_model(model)
+            if limit:
+                ctx.set_memory_limit(ctx.memory_used - 1)
+            ctx.expand()
+            out.append(ctx.get_buffer(E.BUF_SLICES))
+    np.testing.assert_array_equal(out[0], out[1])
+    cfg = O.make_config(side, 3, len(q), likelihood=O.LL_POISSON)
+    ref = np.log(np.maximum(O.expand(cfg, model, q, x, y, z), 1e-10))
+    np.testing.assert_allclose(out[0], ref, rtol=1e-6, atol=1e-6)
