@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(kBlock) softmax_kernel(float* X, int64_t R, in
 // Two sweeps over the FP64 log-likelihood, both bound by its HBM traffic.  One
 // block walking every rotation of 32 patterns (63 blocks on 148 SMs at 2,000
 // patterns) took 3.6 ms at 2,000 x 25,680 and 4.1 ms at 10,000 x 25,680; with
-// the rotations split over blocks the two sweeps take 0.4 and 1.5 ms:
+// the rotations split over blocks the two sweeps take 0.3 and 1.4 ms:
 //   stats    per (row chunk, pattern) the online log-sum-exp and the sums the
 //            scaling and sum P log P need, merged by resp_combine_kernel;
 //   resp     P = exp(LL - lse), its row totals and row maxima.
@@ -652,57 +652,87 @@ __global__ void __launch_bounds__(256) resp_combine_kernel(const RespF32Args a) 
   if (a.new_scaling) a.new_scaling[p] = num > 0.0 && den > 0.0 ? (float)(num / den) : a.scaling[p];
 }
 
-constexpr int kRespRows = 32;
+constexpr int kRespRows = 32, kRespStep = 8;
 
-// 256 patterns x 32 rows per block, a warp 32 patterns; 16 rows at a time are
-// reduced over the warp by halving exchanges (16 + 1 shuffles instead of 80).
-__global__ void __launch_bounds__(256) resp_kernel(const RespF32Args a) {
+// 256 COLS patterns x `rows` rows per block, 8 rows at a time.  A thread sums its
+// patterns' responsibilities first; the warp's 32 lanes are then reduced by
+// halving exchanges (4 + 2 + 1 + 2 for 8 rows).  One pattern per thread, 16
+// rows at a time and a division for the row maxima took 78 instructions an
+// element and bound the sweep (73% of the issue slots).  The whole pass, with two
+// patterns and the reciprocal: 10,000 x 25,680 1.50 -> 1.38 ms, 2,000 x 25,680
+// 0.43 -> 0.30 ms; with four patterns, or 16 rows, there are fewer loads in
+// flight (1.39 to 2.0 ms).
+template <int COLS>
+__global__ void __launch_bounds__(256) resp_kernel(const RespF32Args a, const int rows) {
   __shared__ double st[8][kRespRows];
   __shared__ uint32_t sm[8][kRespRows];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t cols = (a.N + 255) / 256, by = blockIdx.x / cols, bx = blockIdx.x - by * cols;
-  const int64_t p = bx * 256 + threadIdx.x;
-  const bool ok = p < a.N;
-  const double lse = ok ? a.lse[p] : 0.0;
-  const float phi = ok ? (a.new_scaling ? a.new_scaling : a.scaling)[p] : 1.0f;
-  const int64_t r0 = by * kRespRows;
+  constexpr int kCols = 256 * COLS;
+  const int64_t cols = (a.N + kCols - 1) / kCols, by = blockIdx.x / cols, bx = blockIdx.x - by * cols;
+  double lse[COLS];
+  float inv[COLS];  // the maxima may be one rounding off: launch_quant_rows has room for it
+  int64_t p[COLS];
 #pragma unroll
-  for (int h = 0; h < kRespRows; h += 16) {
-    double v[16];
-    uint32_t b[16];
+  for (int c = 0; c < COLS; ++c) {
+    p[c] = bx * kCols + c * 256 + threadIdx.x;
+    const bool ok = p[c] < a.N;
+    lse[c] = ok ? a.lse[p[c]] : 0.0;
+    inv[c] = ok ? 1.0f / (a.new_scaling ? a.new_scaling : a.scaling)[p[c]] : 0.0f;
+  }
+  const int64_t r0 = by * rows;
+#pragma unroll 1
+  for (int h = 0; h < rows; h += kRespStep) {
+    double t[kRespStep];
+    uint32_t b[kRespStep];
 #pragma unroll
-    for (int k = 0; k < 16; ++k)
-      v[k] = ok && r0 + h + k < a.R ? a.LL[(r0 + h + k) * a.N + p] : -DBL_MAX;
+    for (int k = 0; k < kRespStep; ++k) {
+      t[k] = 0.0;
+      b[k] = 0;
+    }
+    double v[COLS][kRespStep];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      float P = 0.0f;
-      if (ok && r0 + h + k < a.R) {
-        P = expf((float)(v[k] - lse));
-        a.P[(r0 + h + k) * a.N + p] = P;
-      }
-      v[k] = (double)P;
-      b[k] = __float_as_uint(P / phi);  // >= 0; a NaN stays the largest
+    for (int c = 0; c < COLS; ++c) {
+      const double* x = a.LL + (r0 + h) * a.N + p[c];
+#pragma unroll
+      for (int k = 0; k < kRespStep; ++k)
+        v[c][k] = p[c] < a.N && r0 + h + k < a.R ? x[k * a.N] : -DBL_MAX;
     }
 #pragma unroll
-    for (int o = 16, n = 8; n >= 1; o >>= 1, n >>= 1) {
+    for (int c = 0; c < COLS; ++c) {
+      const bool ok = p[c] < a.N;
+      float* y = a.P + (r0 + h) * a.N + p[c];
+#pragma unroll
+      for (int k = 0; k < kRespStep; ++k) {
+        if (!(ok && r0 + h + k < a.R)) continue;
+        const float P = expf((float)(v[c][k] - lse[c]));
+        y[k * a.N] = P;
+        t[k] += (double)P;
+        b[k] = max(b[k], __float_as_uint(P * inv[c]));  // >= 0; a NaN stays the largest
+      }
+    }
+#pragma unroll
+    for (int o = 16, n = kRespStep / 2; n >= 1; o >>= 1, n >>= 1) {
       const bool hi = lane & o;
 #pragma unroll
       for (int i = 0; i < n; ++i) {
-        const double keep = hi ? v[i + n] : v[i], send = hi ? v[i] : v[i + n];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        const double keep = hi ? t[i + n] : t[i], send = hi ? t[i] : t[i + n];
+        t[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
         const uint32_t kb = hi ? b[i + n] : b[i], sb = hi ? b[i] : b[i + n];
         b[i] = max(kb, __shfl_xor_sync(0xffffffffu, sb, o));
       }
     }
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-    b[0] = max(b[0], __shfl_xor_sync(0xffffffffu, b[0], 1));
-    if (!(lane & 1)) {
-      st[w][h + (lane >> 1)] = v[0];
-      sm[w][h + (lane >> 1)] = b[0];
+#pragma unroll
+    for (int o = 16 / kRespStep; o > 0; o >>= 1) {
+      t[0] += __shfl_xor_sync(0xffffffffu, t[0], o);
+      b[0] = max(b[0], __shfl_xor_sync(0xffffffffu, b[0], o));
+    }
+    if (lane % (32 / kRespStep) == 0) {
+      st[w][h + lane / (32 / kRespStep)] = t[0];
+      sm[w][h + lane / (32 / kRespStep)] = b[0];
     }
   }
   __syncthreads();
-  if (threadIdx.x < kRespRows && r0 + threadIdx.x < a.R) {
+  if (threadIdx.x < rows && r0 + threadIdx.x < a.R) {
     double t = 0.0;
     uint32_t mx = 0;
     for (int k = 0; k < 8; ++k) {
@@ -1330,15 +1360,25 @@ int64_t resp_f32_chunk(int64_t R, int64_t N) {
 }
 
 cudaError_t launch_resp_f32(const RespF32Args& a, cudaStream_t st) {
-  const int64_t cols = (a.N + 31) / 32, nb = resp_f32_blocks(a.N);
+  const int64_t cols = (a.N + 31) / 32;
   const unsigned gs = (unsigned)(cols * a.nparts);
-  const unsigned gp = (unsigned)(nb * ((a.R + kRespRows - 1) / kRespRows));
   if (a.poisson)
     resp_stats_kernel<true><<<gs, 256, 0, st>>>(a);
   else
     resp_stats_kernel<false><<<gs, 256, 0, st>>>(a);
   resp_combine_kernel<<<(unsigned)cols, 256, 0, st>>>(a);
-  resp_kernel<<<gp, 256, 0, st>>>(a);
+  // two patterns a thread, one (then fewer rows a block) where that would not
+  // give each SM eight blocks (four): 1,000 x 3,240 is 204 blocks, the pass 58
+  // -> 52 us with one pattern, and 64 x 420 34 -> 28 us with 8 rows
+  int rows = kRespRows, c = 2;
+  auto blocks = [&](int c, int rows) {
+    return ((a.N + 256 * c - 1) / (256 * c)) * ((a.R + rows - 1) / rows);
+  };
+  if (blocks(c, rows) < 8 * 148) c = 1;
+  while (rows > kRespStep && blocks(c, rows) < 4 * 148) rows /= 2;
+  const int64_t nb = (a.N + 256 * c - 1) / (256 * c);
+  auto run = c == 2 ? resp_kernel<2> : resp_kernel<1>;
+  run<<<(unsigned)blocks(c, rows), 256, 0, st>>>(a, rows);
   resp_rows_kernel<<<(unsigned)((a.R + 255) / 256), 256, 0, st>>>(a, nb);
   return cudaGetLastError();
 }

@@ -358,55 +358,94 @@ cudaError_t run_i8(const CUtensorMap& tmA, const CUtensorMap& tmB, int64_t m, in
 // ------------------------------------------------------------- operands --
 
 // Balanced base-256 digits of q (|q| <= 127 (2^24 + 2^16 + 2^8 + 1)), lowest
-// first, one byte each.
+// first, one byte each: with 128 added to the three low ones they are the
+// bytes of a sum.
 __device__ __forceinline__ uint32_t digits_of(int q) {
-  uint32_t out = 0;
-#pragma unroll
-  for (int s = 0; s < kDigits; ++s) {
-    const int d = (int)(signed char)(q & 0xff);
-    out |= (uint32_t)(d & 0xff) << (8 * s);
-    q = (q - d) >> 8;
-  }
-  return out;
+  return (uint32_t)(q + 0x00808080) ^ 0x00808080u;
 }
 
-// One block per row of X [R][cols] (div: X = P / phi of the column): the
-// digit planes D [4][R][ld] and the row's unit 2^-k.  2^k puts the row's
-// largest magnitude below 2^31 and the top digit within a byte.
+// Rows of X [R][cols] (DIV: of X / phi of the column) as digit planes
+// D [4][R][ld] and the row's unit 2^-k.  2^k puts the row's largest magnitude
+// (rowmax, which may be a rounding below it) below 2^31 and the top digit within
+// a byte.  A block takes 1024 columns of `rows` rows, a thread four neighbouring
+// columns, so a reciprocal serves every row.  A row per block with a division
+// and shifts for the bytes took 57 instructions an element and bound it (88% of
+// the issue slots); the compress stage of 10,000 columns x 25,680 rows 3.73 ->
+// 3.63 ms, the maximize stage of 12,800 x 25,680 2.92 -> 2.84 ms.
+constexpr int kQuantRows = 8, kQuantStep = 4;
+
+template <bool DIV>
 __global__ void __launch_bounds__(256) quant_rows_kernel(const float* X, const float* div,
                                                          const float* rowmax, int64_t R,
-                                                         int64_t cols, int64_t ld, int8_t* D,
-                                                         float* unit) {
-  const int64_t r = blockIdx.x;
-  const float mx = rowmax[r];
-  const int ex = (int)((__float_as_uint(mx) >> 23) & 0xff) - 127;
-  float up = 0.0f, one = 0.0f;  // a row of zeros (or denormals): all digits 0
-  if (ex == 128) {
-    one = __int_as_float(0x7fffffff);  // an infinite or NaN element: the row's sums are NaN
-  } else if (ex > -127) {
-    int k = 30 - ex;
-    if (k > 126) k = 126;
-    if (ldexpf(mx, k) > 2130706432.0f) --k;
-    up = ldexpf(1.0f, k);
-    one = ldexpf(1.0f, -k);
+                                                         int64_t cols, int64_t ld, int rows,
+                                                         int8_t* D, float* unit) {
+  __shared__ float ups[kQuantRows];
+  const int64_t chunks = (ld + 1023) / 1024, rb = blockIdx.x / chunks;
+  const int64_t r0 = rb * rows, c0 = (blockIdx.x - rb * chunks) * 1024;
+  if (threadIdx.x < rows && r0 + threadIdx.x < R) {
+    const float mx = rowmax[r0 + threadIdx.x];
+    const int ex = (int)((__float_as_uint(mx) >> 23) & 0xff) - 127;
+    float up = 0.0f, one = 0.0f;  // a row of zeros (or denormals): all digits 0
+    if (ex == 128) {
+      one = __int_as_float(0x7fffffff);  // an infinite or NaN element: the row's sums are NaN
+    } else if (ex > -127) {
+      int k = 30 - ex;
+      if (k > 126) k = 126;
+      if (ldexpf(mx, k) > 2130706432.0f) --k;
+      up = ldexpf(1.0f, k);
+      one = ldexpf(1.0f, -k);
+    }
+    ups[threadIdx.x] = up;
+    if (c0 == 0) unit[r0 + threadIdx.x] = one;
   }
-  if (threadIdx.x == 0) unit[r] = one;
-  const float* x = X + r * cols;
-  for (int64_t j0 = 4 * (int64_t)threadIdx.x; j0 < cols; j0 += 4 * blockDim.x) {
-    uint32_t w[4];
+  const int64_t j0 = c0 + 4 * threadIdx.x;
+  // 1 / phi = r + r (1 - r phi), to first order in the rounding of r
+  float r[4], rl[4];
+  if (DIV) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int64_t j = j0 + i;
-      float v = j < cols ? x[j] : 0.0f;
-      if (div && j < cols) v /= div[j];
-      w[i] = digits_of(__float2int_rn(v * up));
+      const float d = j0 + i < cols ? div[j0 + i] : 1.0f;
+      r[i] = 1.0f / d;
+      rl[i] = r[i] * fmaf(-r[i], d, 1.0f);
+    }
+  }
+  __syncthreads();
+  if (j0 >= ld) return;
+  const bool wide = cols % 4 == 0;  // then so is j0 < cols for the four columns
+  for (int h = 0; h < rows; h += kQuantStep) {
+    float v[kQuantStep][4];
+#pragma unroll
+    for (int k = 0; k < kQuantStep; ++k) {
+      const float* x = X + (r0 + h + k) * cols + j0;
+      const bool in = r0 + h + k < R;
+      if (wide) {
+        const float4 q = in && j0 < cols ? *reinterpret_cast<const float4*>(x)
+                                         : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        v[k][0] = q.x, v[k][1] = q.y, v[k][2] = q.z, v[k][3] = q.w;
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[k][i] = in && j0 + i < cols ? x[i] : 0.0f;
+      }
     }
 #pragma unroll
-    for (int s = 0; s < kDigits; ++s) {
-      uint32_t b = 0;
+    for (int k = 0; k < kQuantStep; ++k) {
+      if (r0 + h + k >= R) break;
+      const float up = ups[h + k];
+      uint32_t w[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) b |= ((w[i] >> (8 * s)) & 0xffu) << (8 * i);
-      *reinterpret_cast<uint32_t*>(D + ((int64_t)s * R + r) * ld + j0) = b;
+      for (int i = 0; i < 4; ++i) {
+        const float q = DIV ? fmaf(v[k][i], r[i], v[k][i] * rl[i]) : v[k][i];
+        w[i] = digits_of(__float2int_rn(q * up));
+      }
+      // four columns' digits to four digits' columns
+      const uint32_t a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140);
+      const uint32_t c = __byte_perm(w[0], w[1], 0x7362), d = __byte_perm(w[2], w[3], 0x7362);
+      int8_t* o = D + (r0 + h + k) * ld + j0;
+      const int64_t plane = R * ld;
+      *reinterpret_cast<uint32_t*>(o) = __byte_perm(a, b, 0x5410);
+      *reinterpret_cast<uint32_t*>(o + plane) = __byte_perm(a, b, 0x7632);
+      *reinterpret_cast<uint32_t*>(o + 2 * plane) = __byte_perm(c, d, 0x5410);
+      *reinterpret_cast<uint32_t*>(o + 3 * plane) = __byte_perm(c, d, 0x7632);
     }
   }
 }
@@ -486,7 +525,14 @@ cudaError_t launch_quant_rows(const float* X, const float* div, const float* row
                               int64_t cols, int64_t ld, int8_t* D, float* unit, cudaStream_t st) {
   if (R <= 0) return cudaSuccess;
   if (ld % 16 != 0 || ld < cols) return cudaErrorInvalidValue;
-  quant_rows_kernel<<<(unsigned)R, 256, 0, st>>>(X, div, rowmax, R, cols, ld, D, unit);
+  int rows = kQuantRows;
+  const int64_t chunks = (ld + 1023) / 1024;
+  while (rows > kQuantStep && chunks * ((R + rows - 1) / rows) < 4 * 148) rows /= 2;
+  const unsigned grid = (unsigned)(chunks * ((R + rows - 1) / rows));
+  if (div)
+    quant_rows_kernel<true><<<grid, 256, 0, st>>>(X, div, rowmax, R, cols, ld, rows, D, unit);
+  else
+    quant_rows_kernel<false><<<grid, 256, 0, st>>>(X, div, rowmax, R, cols, ld, rows, D, unit);
   return cudaGetLastError();
 }
 
