@@ -517,13 +517,17 @@ __global__ void __launch_bounds__(kBlock) softmax_kernel(float* X, int64_t R, in
 // Two sweeps over the FP64 log-likelihood, both bound by its HBM traffic.  One
 // block walking every rotation of 32 patterns (63 blocks on 148 SMs at 2,000
 // patterns) took 3.6 ms at 2,000 x 25,680 and 4.1 ms at 10,000 x 25,680; with
-// the rotations split over blocks the two sweeps take 0.3 and 1.4 ms:
+// the rotations split over blocks the two sweeps take 0.3 and 1.2 ms:
 //   stats    per (row chunk, pattern) the online log-sum-exp and the sums the
 //            scaling and sum P log P need, merged by resp_combine_kernel;
 //   resp     P = exp(LL - lse), its row totals and row maxima.
-// Exponentials are FP32 of FP64 differences; eight of them are summed in FP32
+// Exponentials are FP32 of FP64 differences; four of them are summed in FP32
 // and folded into FP64.
-constexpr int kStatRows = 8;  // rows in flight per warp
+// Rows in flight per warp.  Four, in 64 registers, leave room for a fourth block
+// on an SM, which hides the sweep's loads better than eight in three blocks
+// (45% of the issue slots): the pass of 10,000 x 25,680 1.38 -> 1.24 ms, 2,000 x
+// 25,680 0.295 -> 0.272 ms.  Loading the next rows ahead: 1.27 to 1.36 ms.
+constexpr int kStatRows = 4;
 
 struct StatAcc {
   double m, s, d, q;  // max; sum e, sum e X, sum e (LL - m), e = exp(LL - m)
@@ -572,7 +576,7 @@ __device__ __forceinline__ void stat_reduce(StatAcc& a, double (&sh)[4][8][32], 
 }
 
 template <bool POISSON>
-__global__ void __launch_bounds__(256) resp_stats_kernel(const RespF32Args a) {
+__global__ void __launch_bounds__(256, 4) resp_stats_kernel(const RespF32Args a) {
   __shared__ double sh[8][32][4];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t cols = (a.N + 31) / 32, by = blockIdx.x / cols;
@@ -1347,7 +1351,7 @@ cudaError_t launch_ll_fp32(const LLArgs& a, cudaStream_t st) {
 
 int64_t resp_f32_blocks(int64_t N) { return (N + 255) / 256; }
 
-// Rows per block of the stats sweep: at least 64 (eight per warp in flight),
+// Rows per block of the stats sweep: at least 64 (eight per warp),
 // more where the patterns alone fill the GPU several times.
 int64_t resp_f32_chunk(int64_t R, int64_t N) {
   const int64_t cols = (N + 31) / 32, want = 8 * 148;  // blocks
