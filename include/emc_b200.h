@@ -108,7 +108,10 @@ emc_status emc_set_model(emc_context *ctx, const float *model);
 emc_status emc_set_scaling(emc_context *ctx, const float *scaling);
 
 /* One iteration.  stats may be NULL; with stats the call waits for the
- * iteration, without it the work is only enqueued on the context stream. */
+ * iteration, without it the work is enqueued on the context stream.  A mixed
+ * context with more pairs (pattern, rotation) than its responsibility lists
+ * have room for first waits for the responsibilities of the iteration before,
+ * whose count sizes the lists: the host runs at most one iteration ahead. */
 emc_status emc_iterate(emc_context *ctx, emc_iter_stats *stats);
 /* Stage-by-stage form of emc_iterate (the three calls in order == one iteration). */
 emc_status emc_expand(emc_context *ctx);
