@@ -873,18 +873,33 @@ emc_status emc_set_rotations(emc_context* c, const float* q, const float* w) {
   return upload_enqueued(c);
 }
 
+// Whether the context's stream is being captured by the caller (or a batch),
+// not by iterate_graph.  Such a graph is replayed after later uploads, so what
+// is captured must only read buffers that live as long as the context and hold
+// the counts of the day: the dense compress operand instead of lists, and for
+// FP32 contexts the CUDA-core contractions and no voxel table (the byte
+// operands and the photon lists are laid out anew for other counts, and the
+// first two give way to other allocations).  Nothing is waited for, and no
+// event of the context's own is recorded: a captured event cannot be waited for.
+static bool caller_captures(const emc_context* c) {
+  if (c->capturing) return false;
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(c->st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
+}
+static bool uses_i8(const emc_context* c) { return c->i8_planes && !caller_captures(c); }
+
 // Uploads of models, scalings and rotations are enqueued, and their source may
 // be pinned memory that the copy reads later.  An iteration of a mixed context
 // returns only once they have been read, as it always has.
 static emc_status upload_enqueued(emc_context* c) {
-  if (!c->mixed) return EMC_OK;
+  if (!c->mixed || caller_captures(c)) return EMC_OK;
   if (!c->ev_upload) CK(c, cudaEventCreateWithFlags(&c->ev_upload, cudaEventDisableTiming));
   CK(c, cudaEventRecord(c->ev_upload, c->st));
   c->upload_pending = true;
   return EMC_OK;
 }
 static emc_status uploads_read(emc_context* c) {
-  if (!c->upload_pending || c->capturing) return EMC_OK;
+  if (!c->upload_pending || c->capturing || caller_captures(c)) return EMC_OK;
   c->upload_pending = false;
   return c->cuda(cudaEventSynchronize(c->ev_upload), "uploads");
 }
@@ -1113,7 +1128,7 @@ emc_status emc_expand(emc_context* c) {
     a.out_lo = c->d_Blo;
   }
   c->mark(0);
-  if (c->d_vtab) {
+  if (c->d_vtab && (c->mixed || !caller_captures(c))) {
     CK(c, launch_expand_table(c->d_model, c->cfg.side, a.out, a.floor_, a.log_split, c->d_vtab,
                               c->st));
     a.tab = c->d_vtab;
@@ -1393,7 +1408,7 @@ static emc_status list_count_back(emc_context* c) {
 
 static emc_status mixed_resp_pass(emc_context* c, bool allow_lists = true) {
   c->cmp_mode = emc_context::CMP_DENSE;
-  if (allow_lists && uses_lists(c)) {
+  if (allow_lists && uses_lists(c) && (c->det || !caller_captures(c))) {
     // the compress operand as per-rotation lists of its non-zero entries
     if (c->det) return det_resp_pass(c);
     if (!c->capturing) TRY(list_room(c));
@@ -1692,9 +1707,10 @@ emc_status emc_maximize(emc_context* c) {
   const int64_t R = c->R, N = c->N;
   CK(c, cudaMemcpyAsync(c->d_scaling_prev, c->d_scaling, sizeof(float) * N,
                         cudaMemcpyDeviceToDevice, c->st));
+  const bool i8 = !c->mixed && !c->tune.maximize_sparse && uses_i8(c);
   if (!c->mixed && c->tune.maximize_sparse) {
     TRY(sparse_loglik(c));
-  } else if (!c->mixed && c->i8_planes) {
+  } else if (i8) {
     TRY(i8_loglik(c));
   } else if (!c->mixed) {
     LLArgs l{};
@@ -1736,7 +1752,7 @@ emc_status emc_maximize(emc_context* c) {
     // is one of its terms) where that is exact to FP64; the CUDA-core form
     // sums (S - K / phi)^2 in FP32, which leaves C too few digits where phi is
     // far off, so there the cross term is contracted by itself
-    const bool cross = c->gauss && !c->i8_planes;
+    const bool cross = c->gauss && !i8;
     a.new_scaling = cross ? nullptr : c->d_scaling;
     a.P = c->d_LL;
     a.Tpart = c->d_Tpart64;
@@ -1801,7 +1817,7 @@ emc_status emc_compress_insert(emc_context* c) {
   if (!c->mixed) {
     if (c->tune.compress_sparse) {
       TRY(sparse_slicesums(c));
-    } else if (c->i8_planes) {
+    } else if (uses_i8(c)) {
       TRY(i8_slicesums(c));
     } else {
       CompressArgs a{};
@@ -1968,7 +1984,8 @@ static emc_status iterate_stages(emc_context* c) {
 // row that finds the same buffers and tuning, so a context that iterates once
 // or twice never pays for it, and it holds the same launches: nothing in it
 // depends on values.  Rotation chunks, the deterministic sort, profiling,
-// batches and a caller's own capture keep the separate launches.
+// batches and a caller's own capture (caller_captures) keep the separate
+// launches.
 static emc_context::GraphKey graph_key(const emc_context* c) {
   emc_context::GraphKey k{};
   k.tune = c->tune;
@@ -1988,9 +2005,7 @@ static emc_status iterate_graph(emc_context* c, bool* done) {
   if (c->graph_off || c->prof || c->batched || c->det || (c->mixed && c->y_rows < c->R) ||
       c->stage != 0 || !c->have_geom || !c->have_rot || !c->have_pat || !c->have_model)
     return EMC_OK;
-  cudaStreamCaptureStatus busy = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(c->st, &busy) != cudaSuccess || busy != cudaStreamCaptureStatusNone)
-    return EMC_OK;
+  if (caller_captures(c)) return EMC_OK;
   if (c->graph_seen > 0 && uses_lists(c)) TRY(list_room(c));
   const emc_context::GraphKey k = graph_key(c);
   if (!(c->graph_seen > 0 && k == c->graph_key)) {

@@ -111,7 +111,13 @@ emc_status emc_set_scaling(emc_context *ctx, const float *scaling);
  * iteration, without it the work is enqueued on the context stream.  A mixed
  * context with more pairs (pattern, rotation) than its responsibility lists
  * have room for first waits for the responsibilities of the iteration before,
- * whose count sizes the lists: the host runs at most one iteration ahead. */
+ * whose count sizes the lists: the host runs at most one iteration ahead.
+ * Dense iterations (stats NULL) and their stages may be captured by the caller
+ * into a CUDA graph on the context stream; they then take the forms whose
+ * buffers live as long as the context (mixed: the dense compress; FP32: the
+ * CUDA-core contractions), so a replay after later uploads is right.  The
+ * photon-list forms of FP32 contexts, rotation chunks and the deterministic
+ * lists of mixed contexts cannot be captured. */
 emc_status emc_iterate(emc_context *ctx, emc_iter_stats *stats);
 /* Stage-by-stage form of emc_iterate (the three calls in order == one iteration). */
 emc_status emc_expand(emc_context *ctx);
