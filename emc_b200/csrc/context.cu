@@ -337,6 +337,7 @@ struct emc_context {
   int graph_seen = 0;
   bool graph_off = false;   // a capture failed: iterations stay eager
   bool capturing = false;
+  bool whole = false;       // inside emc_iterate: nothing changes between its stages
   cudaGraphExec_t graph_exec = nullptr;
   int64_t graph_launches = 0;
   int64_t version = 0;      // allocations and releases so far
@@ -1618,10 +1619,27 @@ static emc_status sparse_loglik(emc_context* c) {
   return EMC_OK;
 }
 
+// The fixed point of a row follows its largest magnitude, which the stage before
+// leaves in d_rowmax.  Between the stages of a call-by-call iteration the program
+// may change slices, responsibilities or scaling (emc_set_scaling, the device
+// buffers), so there the maxima are taken again, from what is quantised; a value
+// past the maximum it was scaled by would wrap.  The same for the sums of S^2,
+// which the gaussian form takes from the expansion.
+static emc_status current_maxima(emc_context* c, const float* X, const float* div, int64_t cols) {
+  if (c->whole) return EMC_OK;
+  c->launches += 1;
+  return c->cuda(launch_row_maxima(X, div, c->R, cols, c->d_rowmax, c->st), "row maxima");
+}
+
 // The FP32 contexts' log-likelihood on the byte tensor cores: the slices as
 // digit planes, then the contraction with the counts (twice when a count
 // exceeds 127).
 static emc_status i8_loglik(emc_context* c) {
+  TRY(current_maxima(c, c->d_S, nullptr, c->npa));
+  if (!c->whole && c->gauss) {
+    CK(c, launch_pattern_stats(c->d_S, nullptr, c->R, c->npa, c->npa, 1, c->d_rowstat, c->st));
+    c->launches += 1;
+  }
   CK(c, launch_quant_rows(c->d_S, nullptr, c->d_rowmax, c->R, c->npa, round_up(c->npa, 16),
                           c->d_digits, c->d_unit, c->st));
   I8LLArgs a{};
@@ -1646,6 +1664,7 @@ static emc_status i8_loglik(emc_context* c) {
 // The slice sums the same way: P / phi as digit planes (its row maxima come
 // from the responsibility sweep), contracted with the counts by pixel.
 static emc_status i8_slicesums(emc_context* c) {
+  TRY(current_maxima(c, c->d_LL, c->d_scaling, c->N));
   CK(c, launch_quant_rows(c->d_LL, c->d_scaling, c->d_rowmax, c->R, c->N, round_up(c->N, 16),
                           c->d_digits, c->d_unit, c->st));
   I8UArgs a{};
@@ -1973,9 +1992,12 @@ emc_status emc_wait_probe(emc_context* c, uint32_t limit_us) {
 }
 
 static emc_status iterate_stages(emc_context* c) {
-  TRY(emc_expand(c));
-  TRY(emc_maximize(c));
-  return emc_compress(c);
+  c->whole = true;
+  emc_status s = emc_expand(c);
+  if (s == EMC_OK) s = emc_maximize(c);
+  if (s == EMC_OK) s = emc_compress(c);
+  c->whole = false;
+  return s;
 }
 
 // One iteration through a CUDA graph of its launches.  Small problems are

@@ -50,6 +50,9 @@ cudaError_t launch_i8_slices(const CUtensorMap& tmKt, const CUtensorMap& tmX, in
 // rowmax [R]: the largest |X| of the row (after the division by div[column]).
 cudaError_t launch_quant_rows(const float* X, const float* div, const float* rowmax, int64_t R,
                               int64_t cols, int64_t ld, int8_t* D, float* unit, cudaStream_t st);
+// The same rowmax from X and div.
+cudaError_t launch_row_maxima(const float* X, const float* div, int64_t R, int64_t cols,
+                              float* rowmax, cudaStream_t st);
 cudaError_t launch_pack_counts_i8(const float* K, int64_t N, int64_t npa, int planes, int64_t ldK,
                                   int64_t ldT, int8_t* K8, int8_t* Kt8, cudaStream_t st);
 // out[0] = bits of the largest entry, out[1] = entries that are not integers

@@ -450,6 +450,26 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const float* X, const f
   }
 }
 
+// rowmax[r] = the largest |X| (or |X / div|, within a rounding, as
+// quant_rows_kernel allows) of row r; a NaN stays the largest.  One block per row.
+__global__ void __launch_bounds__(256) row_maxima_kernel(const float* X, const float* div,
+                                                         int64_t cols, float* rowmax) {
+  __shared__ uint32_t red[8];
+  const float* x = X + blockIdx.x * cols;
+  uint32_t mx = 0;
+  for (int64_t j = threadIdx.x; j < cols; j += 256) {
+    const float v = div ? x[j] * (1.0f / div[j]) : x[j];
+    mx = max(mx, __float_as_uint(fabsf(v)));
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; ++k) mx = max(mx, red[k]);
+    rowmax[blockIdx.x] = __uint_as_float(mx);
+  }
+}
+
 // Counts K [N][npa] as bytes by pattern (K8 [planes][N][ldK]) and by pixel
 // (Kt8 [planes][npa][ldT]), base-128 digits when planes == 2.
 __global__ void pack_counts_i8_kernel(const float* K, int64_t N, int64_t npa, int planes,
@@ -533,6 +553,13 @@ cudaError_t launch_quant_rows(const float* X, const float* div, const float* row
     quant_rows_kernel<true><<<grid, 256, 0, st>>>(X, div, rowmax, R, cols, ld, rows, D, unit);
   else
     quant_rows_kernel<false><<<grid, 256, 0, st>>>(X, div, rowmax, R, cols, ld, rows, D, unit);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_row_maxima(const float* X, const float* div, int64_t R, int64_t cols,
+                              float* rowmax, cudaStream_t st) {
+  if (R <= 0) return cudaSuccess;
+  row_maxima_kernel<<<(unsigned)R, 256, 0, st>>>(X, div, cols, rowmax);
   return cudaGetLastError();
 }
 
