@@ -3209,6 +3209,7 @@ struct emc_batch {
   cudaEvent_t forked = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  std::vector<emc_context::GraphKey> keys;  // what each dataset's part was captured for
   std::string err;
   emc_status fail(emc_status s, const std::string& m) {
     err = m;
@@ -3530,7 +3531,7 @@ emc_status emc_batch_create(emc_context* const* ctxs, int32_t n, emc_batch** out
   return EMC_OK;
 }
 
-emc_status emc_batch_iterate(emc_batch* b) {
+static emc_status batch_iteration(emc_batch* b) {
   StageRange range("emc batch iteration");
   if (!b) return EMC_ERR_ARG;
   const int n = (int)b->ctx.size();
@@ -3619,6 +3620,28 @@ emc_status emc_batch_iterate(emc_batch* b) {
   return each_dataset(b, [&](int i) { return shared(i) && !b->lists[i]; }, finish);
 }
 
+// The photon lists and list buffers of the datasets that compress from lists:
+// built before an iteration is launched or captured, since building them waits.
+// An upload through a dataset's own call leaves its photon lists to be built anew.
+static emc_status batch_ready(emc_batch* b) {
+  for (size_t i = 0; i < b->ctx.size(); ++i) {
+    emc_context* c = b->ctx[i];
+    if (b->lists[i]) BTRY(b, c, batch_lists_ready(c, c->lcomp_cap));
+  }
+  return EMC_OK;
+}
+
+emc_status emc_batch_iterate(emc_batch* b) {
+  if (!b) return EMC_ERR_ARG;
+  cudaStreamCaptureStatus busy = cudaStreamCaptureStatusNone;
+  BCK(b, cudaStreamIsCapturing(b->st, &busy));
+  if (busy == cudaStreamCaptureStatusNone) {
+    const emc_status s = batch_ready(b);
+    if (s != EMC_OK) return s;
+  }
+  return batch_iteration(b);
+}
+
 emc_status emc_batch_capture(emc_batch* b) {
   if (!b) return EMC_ERR_ARG;
   if (b->exec) {
@@ -3629,16 +3652,20 @@ emc_status emc_batch_capture(emc_batch* b) {
     cudaGraphDestroy(b->graph);
     b->graph = nullptr;
   }
+  const emc_status ready = batch_ready(b);
+  if (ready != EMC_OK) return ready;
   std::vector<int64_t> l0;
   std::vector<bool> prof;
+  b->keys.clear();
   for (emc_context* c : b->ctx) {
+    b->keys.push_back(graph_key(c));
     l0.push_back(c->launches);
     prof.push_back(c->prof);
     c->prof = false;  // no stage events inside the graph
   }
   BCK(b, cudaStreamSynchronize(b->st));
   BCK(b, cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
-  const emc_status s = emc_batch_iterate(b);
+  const emc_status s = batch_iteration(b);
   cudaGraph_t g = nullptr;
   const cudaError_t e = cudaStreamEndCapture(b->st, &g);
   b->per_iter.assign(b->ctx.size(), 0);
@@ -3662,6 +3689,12 @@ emc_status emc_batch_capture(emc_batch* b) {
 emc_status emc_batch_launch(emc_batch* b, int32_t iterations) {
   if (!b || iterations < 0) return EMC_ERR_ARG;
   if (!b->exec) return b->fail(EMC_ERR_STATE, "emc_batch_capture first");
+  // a dataset's own calls may have replaced buffers that the graph reads
+  emc_status s = batch_ready(b);
+  bool same = true;
+  for (size_t i = 0; i < b->ctx.size(); ++i) same = same && b->keys[i] == graph_key(b->ctx[i]);
+  if (s == EMC_OK && !same) s = emc_batch_capture(b);
+  if (s != EMC_OK) return s;
   for (int32_t k = 0; k < iterations; ++k) BCK(b, cudaGraphLaunch(b->exec, b->st));
   for (size_t i = 0; i < b->ctx.size(); ++i) {
     emc_context* c = b->ctx[i];

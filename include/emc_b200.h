@@ -232,7 +232,9 @@ emc_status emc_orientation_stats(emc_context *ctx, int32_t *best_rot, float *bes
  * captured graph again).  The contexts keep that stream until
  * emc_batch_destroy; their own calls (get_model, ...) stay ordered with the
  * batch.  emc_batch_capture records one batched iteration into a CUDA graph;
- * emc_batch_launch replays it.  Destroy a batch before its contexts. */
+ * emc_batch_launch replays it, recording it again first when a dataset's own
+ * calls (an upload, an iteration, a tuning) replaced what the graph reads.
+ * Destroy a batch before its contexts. */
 typedef struct emc_batch emc_batch;
 emc_status emc_batch_create(emc_context *const *ctxs, int32_t n, emc_batch **out);
 emc_status emc_batch_destroy(emc_batch *batch);
