@@ -380,7 +380,8 @@ struct emc_context {
   emc_status alloc(T** p, size_t count, bool zero = false) {
     void* q = nullptr;
     const size_t bytes = count * sizeof(T) ? count * sizeof(T) : 16;
-    if (mem_limit && mem_used + bytes > mem_limit) make_room();
+    if (mem_limit && mem_used + bytes > mem_limit && mem_used - spare() + bytes <= mem_limit)
+      make_room();
     if (mem_limit && mem_used + bytes > mem_limit)
       return fail(EMC_ERR_OOM, "device memory limit of %zu bytes reached (%zu held, %zu requested)",
                   mem_limit, mem_used, bytes);
@@ -420,7 +421,13 @@ struct emc_context {
     d_i8 = nullptr;
   }
   // The byte operands and an FP32 context's voxel table are faster routes, not
-  // needs: they make room.
+  // needs: they make room, where that is enough (spare: the bytes they hold).
+  size_t size_of(const void* p) const {
+    for (size_t k = 0; k < allocs.size(); ++k)
+      if (p && allocs[k] == p) return alloc_bytes[k];
+    return 0;
+  }
+  size_t spare() const { return size_of(d_i8) + (mixed ? 0 : size_of(d_vtab)); }
   void make_room() {
     drop_i8();
     if (mixed || !d_vtab) return;
@@ -551,10 +558,10 @@ int64_t emc_launch_count(const emc_context* ctx) { return ctx ? ctx->launches : 
 
 emc_status emc_set_memory_limit(emc_context* c, size_t bytes) {
   if (!c) return EMC_ERR_ARG;
-  if (bytes && bytes < c->mem_used) c->make_room();
-  if (bytes && bytes < c->mem_used)
+  if (bytes && bytes < c->mem_used - c->spare())
     return c->fail(EMC_ERR_ARG, "limit %zu is below the %zu bytes already held", bytes,
-                   c->mem_used);
+                   c->mem_used - c->spare());
+  if (bytes && bytes < c->mem_used) c->make_room();
   c->mem_limit = bytes;
   return EMC_OK;
 }

@@ -154,8 +154,14 @@ emc_status emc_stage_times(emc_context *ctx, float ms[5]);
 /* Cap on the device memory this context allocates, in bytes (0: no cap; the
  * default).  A call whose allocations would pass it fails with EMC_ERR_OOM
  * before allocating; the context is then only good for emc_destroy, which
- * frees what it holds.  EMC_ERR_ARG when the cap is below what is already
- * held.  emc_memory_used: device bytes the context holds. */
+ * frees what it holds.  EMC_ERR_ARG, with nothing changed, when the cap is
+ * below what the context needs to hold.  An FP32 context also holds operands
+ * that only make it faster (the counts and digit planes of its byte
+ * contractions, a voxel table): they are given back when a cap or a later
+ * allocation needs their room and gets it that way, and emc_memory_used falls
+ * by them.  The iterations then run on the CUDA cores, up to 50 times slower,
+ * until a pattern upload with room for the operands.
+ * emc_memory_used: device bytes the context holds. */
 emc_status emc_set_memory_limit(emc_context *ctx, size_t bytes);
 size_t emc_memory_used(const emc_context *ctx);
 /* Rotation chunks (mixed contexts).  The log-likelihood Y of a dense
