@@ -276,6 +276,7 @@ struct emc_context {
   int32_t* d_lpat = nullptr;
   float* d_lx = nullptr;
   int64_t lcap = 0, list_nnz = 0;
+  int64_t lcap_for = 0;  // the entries that lcap was to hold, where there was room
   // this iteration's compress: the dense operand, the lists, or both gated on
   // the count of compacted entries (lists up to list_gate of them)
   enum { CMP_DENSE, CMP_LISTS, CMP_GATED } cmp_mode = CMP_DENSE;
@@ -1297,7 +1298,25 @@ static emc_status list_capacity(emc_context* c, int64_t n) {
   return EMC_OK;
 }
 
-// Scratch of the deterministic (rotation, pattern) sort of n entries.
+// Lists for as many of the compacted entries as there is memory for: all of
+// them, or half as often as it takes.  Sharp posteriors keep a few entries a
+// pattern, so a context whose memory limit has no room for lists of every entry
+// that the compaction could hold still iterates from lists; above what they hold
+// (list_gate) the compress is the dense one.
+static emc_status list_capacity_or_less(emc_context* c, int64_t n) {
+  if (c->lcap > 0 && c->lcap_for >= n) return EMC_OK;
+  const std::string err = c->err;
+  emc_status s;
+  int64_t m = n;
+  while ((s = list_capacity(c, m)) == EMC_ERR_OOM && m > 1024) {
+    cudaGetLastError();
+    c->err = err;
+    m /= 2;
+  }
+  if (s == EMC_OK) c->lcap_for = n;
+  return s;
+}
+
 static emc_status sort_scratch(emc_context* c, int64_t n) {
   TRY(grow(c, &c->d_sort_rp, c->sort_cap, n + 1));
   TRY(grow(c, &c->d_sort_v, c->sort_cap2, n + 1));
@@ -1318,6 +1337,12 @@ static int64_t list_worth(const emc_context* c) {
   const double dense = 2.0 * pairs * (double)c->npa / 6.5e14 + 8.0 * pairs / 5e12;
   const double photons = (double)c->csr.nnz / (double)c->N;
   return (int64_t)std::min(dense * 6.4e11 / std::max(photons, 1.0), 9e15);
+}
+
+// Entries up to which an iteration compresses from lists: what is worth it, what
+// the compaction holds, what the lists hold.
+static int64_t list_limit(const emc_context* c) {
+  return std::min({std::max<int64_t>(list_worth(c), 64 * c->N), c->lcomp_cap, c->lcap});
 }
 
 // The deterministic lists: the host reads the entries' count (one wait), since
@@ -1440,7 +1465,7 @@ static emc_status mixed_resp_pass(emc_context* c, bool allow_lists = true) {
 // batch_lists_ready sized every buffer.
 static emc_status gated_list_pass(emc_context* c) {
   RespArgs a = resp_args(c);
-  c->list_gate = std::min(std::max<int64_t>(list_worth(c), 64 * c->N), c->lcomp_cap);
+  c->list_gate = list_limit(c);
   CK(c, cudaMemsetAsync(c->d_lcount, 0, sizeof(unsigned long long), c->st));
   a.list_count = c->d_lcount;
   a.list_cap = c->lcomp_cap;
@@ -1466,7 +1491,7 @@ static emc_status gated_list_pass(emc_context* c) {
 static emc_status batch_lists_ready(emc_context* c, int64_t entries) {
   TRY(list_buffers(c));
   TRY(compact_capacity(c, entries));
-  TRY(list_capacity(c, c->lcomp_cap + 1));
+  TRY(list_capacity_or_less(c, c->lcomp_cap + 1));
   if (!c->csr.valid) TRY(build_rows(c, c->d_K, c->N, c->npa, c->csr, false));
   return EMC_OK;
 }
@@ -2025,7 +2050,7 @@ static emc_context::GraphKey graph_key(const emc_context* c) {
   k.csr = c->csr.valid;
   k.csc = c->csc.valid;
   if (uses_lists(c) && c->csr.valid)
-    k.gate = std::min(std::max<int64_t>(list_worth(c), 64 * c->N), c->lcomp_cap);
+    k.gate = list_limit(c);
   return k;
 }
 
