@@ -76,10 +76,11 @@ __device__ __forceinline__ bool nearest_from_1(const float* u, int side, uint32_
 template <int INTERP>
 __device__ __forceinline__ float gather(const float* __restrict__ model, const float* u, int side) {
   if (INTERP == 0) {
+    // rows of voxels fit 32 bits; the drop-in API has no bound on side^3
     uint32_t k[3];
-    return nearest_from_1(u, side, k)
-               ? __ldg(model + (((int)k[2] + 1) * side + (int)k[1] + 1) * side + (int)k[0] + 1)
-               : 0.0f;
+    if (!nearest_from_1(u, side, k)) return 0.0f;
+    const uint32_t row = (k[2] + 1) * (uint32_t)side + k[1] + 1;
+    return __ldg(model + ((uint64_t)row * (uint32_t)side + k[0] + 1));
   }
   float acc = 0.0f;
 #pragma unroll
@@ -1083,10 +1084,11 @@ int64_t expand_parts(int64_t ld) {
   return chunks < kExpParts ? chunks : kExpParts;
 }
 
-// The voxel index is 32 bits wide (nearest_from_1), so side^3 must fit.
+// Without the voxel table any side whose model fits the GPU; the table's index
+// is 32 bits wide (contexts: side <= 1024).
 cudaError_t launch_expand(const ExpandArgs& a, cudaStream_t st) {
   if (a.R <= 0) return cudaSuccess;
-  if (a.npix > a.ld || a.ld > (int64_t)1 << 30 || a.side > 1290 ||
+  if (a.npix > a.ld || a.ld > (int64_t)1 << 30 || a.side > 32768 || (a.tab && a.side > 1290) ||
       (a.out == EXP_F16_SPLIT && (a.ld % 2 != 0 || a.rowmax || (a.interp == 0 && !a.tab))) ||
       (a.stat != STAT_NONE && !(a.rowstat && a.statpart)) || (a.rowmax && !a.maxpart))
     return cudaErrorInvalidValue;
