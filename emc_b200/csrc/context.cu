@@ -895,7 +895,13 @@ static bool caller_captures(const emc_context* c) {
   cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(c->st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
 }
-static bool uses_i8(const emc_context* c) { return c->i8_planes && !caller_captures(c); }
+// The contractions on byte digits.  Whether their operands fit depends on the
+// memory that happens to be free, and they round differently from the CUDA-core
+// form, so deterministic contexts, whose runs are bitwise the same wherever they
+// are continued, keep the latter.
+static bool uses_i8(const emc_context* c) {
+  return c->i8_planes && !c->det && !caller_captures(c);
+}
 
 // Uploads of models, scalings and rotations are enqueued, and their source may
 // be pinned memory that the copy reads later.  An iteration of a mixed context
@@ -1346,7 +1352,10 @@ static int64_t list_limit(const emc_context* c) {
 }
 
 // The deterministic lists: the host reads the entries' count (one wait), since
-// the sort's launches depend on it.
+// the sort's launches depend on it.  More entries than the compaction holds, and
+// worth lists: it grows and the sweep runs again (its sums have a fixed order), so
+// lists or the dense operand follows from the data, not from earlier iterations,
+// and a run resumed in a fresh context is bitwise the same.
 static emc_status det_resp_pass(emc_context* c) {
   const int64_t N = c->N;
   RespArgs a = resp_args(c);
@@ -1354,21 +1363,27 @@ static emc_status det_resp_pass(emc_context* c) {
   if (!c->csr.valid) TRY(build_rows(c, c->d_K, N, c->npa, c->csr, false));
   const int64_t worth = std::max<int64_t>(list_worth(c), 64 * N);
   TRY(compact_capacity(c, std::max<int64_t>(64 * N, (int64_t)1 << 20)));
-  CK(c, cudaMemsetAsync(c->d_lcount, 0, sizeof(unsigned long long), c->st));
-  a.list_count = c->d_lcount;
-  a.list_cap = c->lcomp_cap;
-  a.list_rp = c->d_lcomp_rp;
-  a.list_P = c->d_lcomp_P;
-  a.list_min = kListMinP;
-  CK(c, launch_resp_rowsums(a, c->st));
   unsigned long long* hn = c->pinned<unsigned long long>(7, 1);
   if (!hn) return c->fail(EMC_ERR_OOM, "pinned host staging");
   c->count_pending = false;
-  CK(c, cudaMemcpyAsync(hn, c->d_lcount, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                        c->st));
-  CK(c, cudaStreamSynchronize(c->st));
-  c->list_nnz = (int64_t)*hn;
-  if (c->list_nnz <= std::min(worth, c->lcomp_cap)) {
+  for (int attempt = 0;; ++attempt) {
+    CK(c, cudaMemsetAsync(c->d_lcount, 0, sizeof(unsigned long long), c->st));
+    a.list_count = c->d_lcount;
+    a.list_cap = c->lcomp_cap;
+    a.list_rp = c->d_lcomp_rp;
+    a.list_P = c->d_lcomp_P;
+    a.list_min = kListMinP;
+    CK(c, launch_resp_rowsums(a, c->st));
+    CK(c, cudaMemcpyAsync(hn, c->d_lcount, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                          c->st));
+    CK(c, cudaStreamSynchronize(c->st));
+    c->list_nnz = (int64_t)*hn;
+    if (c->list_nnz <= c->lcomp_cap || c->list_nnz > worth) break;
+    if (attempt) return c->fail(EMC_ERR_CUDA, "entry count changed between identical sweeps");
+    TRY(compact_capacity(c, c->list_nnz));
+    c->launches += 2;
+  }
+  if (c->list_nnz <= worth) {
     TRY(list_capacity(c, c->list_nnz + 1));
     // the entries in (rotation, pattern) order, so the lists do not depend on
     // the order the sweep appended them
@@ -1382,10 +1397,7 @@ static emc_status det_resp_pass(emc_context* c) {
     c->cmp_mode = emc_context::CMP_LISTS;
     c->launches += 6;  // combine, row sums, T, sort, count, place
   } else {
-    // more entries than the compaction holds: the dense operand this time,
-    // room for them next time if they are worth it
     CK(c, launch_resp_write(a, c->st));
-    if (c->list_nnz <= worth) TRY(compact_capacity(c, c->list_nnz));
     c->launches += 3;
   }
   CK(c, launch_sum2_f64(c->d_plogp, c->d_lse, N, c->d_stats + 2, c->st));

@@ -195,8 +195,9 @@ int64_t emc_rotation_chunk(const emc_context *ctx);
  * and rounded once; the responsibility lists are sorted by (rotation,
  * pattern) and each rotation's slice sums its patterns in that order.  Two
  * runs of the same iterations then give bitwise the same model, weight and
- * scaling, chunked or not, in either precision.  Costs 64 bytes of device
- * memory per voxel.  EMC_ERR_UNSUPPORTED for the proposed iterations; a
+ * scaling, chunked or not, in either precision, and so does a run resumed in
+ * another context.  Costs 64 bytes of device memory per voxel; an FP32
+ * context's contractions stay on the CUDA cores.  EMC_ERR_UNSUPPORTED for the proposed iterations; a
  * batch takes contexts without it. */
 emc_status emc_set_deterministic(emc_context *ctx, int on);
 /* Checkpoint (emc.c:715-716 resumes from a model file at start_iteration;
