@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(256, 4) resp_stats_kernel(const RespF32Args a)
       const double rs = a.rowstat[r + k];
       const float x = POISSON ? (float)rs : (float)(fma(v[k], ginv, rs + k2) * half_phi);
       s += e;
-      d = fmaf(e, x, d);
+      if (e > 0.0f) d = fmaf(e, x, d);  // x is infinite where LL is
       q = fmaf(e, dl, q);
     }
     acc.s += (double)s;
@@ -652,7 +652,7 @@ __global__ void __launch_bounds__(256) resp_combine_kernel(const RespF32Args a) 
   if (w != 0 || !ok) return;
   const double ls = log(acc.s);
   a.lse[p] = acc.m + ls;
-  a.plogp[p] = acc.q / acc.s - ls;  // sum P (LL - lse)
+  a.plogp[p] = acc.s > 0.0 ? acc.q / acc.s - ls : 0.0;  // sum P (LL - lse)
   // emc_cuda.cu:226; a pattern without photons or weight keeps its scale
   const double num = a.poisson ? a.patsum[p] : a.patstat[p], den = acc.d / acc.s;
   if (a.new_scaling) a.new_scaling[p] = num > 0.0 && den > 0.0 ? (float)(num / den) : a.scaling[p];
@@ -710,7 +710,9 @@ __global__ void __launch_bounds__(256) resp_kernel(const RespF32Args a, const in
 #pragma unroll
       for (int k = 0; k < kRespStep; ++k) {
         if (!(ok && r0 + h + k < a.R)) continue;
-        const float P = expf((float)(v[c][k] - lse[c]));
+        // 0 also where LL or every LL of the pattern is not finite: the pattern
+        // then takes no part (emc_cuda.cu:463-468 skips such terms)
+        const float P = expf(fmaxf((float)(v[c][k] - lse[c]), -200.0f));
         y[k * a.N] = P;
         t[k] += (double)P;
         b[k] = max(b[k], __float_as_uint(P * inv[c]));  // >= 0; a NaN stays the largest
