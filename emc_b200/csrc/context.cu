@@ -207,6 +207,15 @@ struct emc_context {
   int i8_planes = 0;
   int8_t *d_i8 = nullptr, *d_K8 = nullptr, *d_Kt8 = nullptr, *d_digits = nullptr;
   float* d_unit = nullptr;
+  uint32_t* d_ktot = nullptr;  // photons at each pixel
+  // the patterns' photon lists (room for i8_nonzero entries)
+  int64_t i8_nonzero = 0, *d_kbeg = nullptr, *d_kend = nullptr;
+  int32_t* d_kidx = nullptr;
+  float* d_kval = nullptr;
+  unsigned long long* d_ktotal = nullptr;
+  int32_t* d_small = nullptr;  // rows whose slice sums need the remainders
+  uint32_t* d_rembits = nullptr;  // elements that may have one
+  int32_t* d_remcount = nullptr;  // their number in each row (zeroed by the maximize)
   CUtensorMap tmK8[2], tmKt8[2], tmXp, tmXn;
   // mixed path
   int64_t Npad = 0, Ppad = 0, Rpad = 0, nrt = 0;
@@ -950,7 +959,7 @@ emc_status emc_set_patterns(emc_context* c, const float* counts) {
 // count an integer): one digit plane up to 127, two above.  They are kept only
 // where they take less than half of the memory that is left, and the CUDA-core
 // contractions run without them.
-static void i8_prepare(emc_context* c, float top) {
+static void i8_prepare(emc_context* c, float top, int64_t nonzero) {
   const int64_t N = c->N, R = c->R, npa = c->npa;
   const int planes = top <= (float)kI8MaxCount ? 1 : 2;
   // 32-bit sums: 128 x the total of a row of counts
@@ -959,12 +968,18 @@ static void i8_prepare(emc_context* c, float top) {
   auto pad = [](size_t n) { return (n + 255) / 256 * 256; };
   const size_t digits = pad((size_t)kI8Digits * (size_t)R * (size_t)std::max(ldK, ldT));
   const size_t k8 = pad((size_t)planes * (size_t)(N * ldK)), kt8 = pad((size_t)planes * (size_t)(npa * ldT));
-  const size_t bytes = k8 + kt8 + digits + sizeof(float) * (size_t)R;
+  const size_t unit = pad(sizeof(float) * (size_t)R), ktot = pad(sizeof(uint32_t) * (size_t)npa);
+  const size_t small = pad(sizeof(int32_t) * (size_t)(2 * R));
+  const size_t lists = sizeof(int64_t) * (size_t)(2 * N + 1) + 8 * (size_t)nonzero;
+  const size_t rembits = pad(sizeof(uint32_t) * (size_t)(R * i8_bit_words(N)));
+  const size_t bytes = k8 + kt8 + digits + unit + ktot + small + rembits + lists;
   const bool fits = top <= (float)kI8MaxCount2 && most <= kI8MaxTotal &&
                     (double)R * kI8Digits < 2147483647.0 &&
-                    ((bytes <= ((size_t)64 << 20) && !c->mem_limit) || c->i8_planes == planes ||
-                     bytes <= avail_bytes(c, 0) / 2);
-  if (c->i8_planes == planes && fits) return;  // sized for these patterns already
+                    ((bytes <= ((size_t)64 << 20) && !c->mem_limit) ||
+                     (c->i8_planes == planes && nonzero <= c->i8_nonzero) ||
+                     bytes <= avail_bytes(c, c->size_of(c->d_i8)) / 2);
+  const bool sized = c->i8_planes == planes && nonzero <= c->i8_nonzero;
+  if (sized && fits) return;  // sized for these patterns already
   c->drop_i8();
   if (!fits) return;
   const std::string err = c->err;
@@ -979,6 +994,16 @@ static void i8_prepare(emc_context* c, float top) {
   c->d_Kt8 = c->d_K8 + k8;
   c->d_digits = c->d_Kt8 + kt8;
   c->d_unit = reinterpret_cast<float*>(c->d_digits + digits);
+  c->d_ktot = reinterpret_cast<uint32_t*>(c->d_digits + digits + unit);
+  c->d_small = reinterpret_cast<int32_t*>(c->d_digits + digits + unit + ktot);
+  c->d_remcount = c->d_small + R;
+  c->d_rembits = reinterpret_cast<uint32_t*>(c->d_digits + digits + unit + ktot + small);
+  c->d_kbeg = reinterpret_cast<int64_t*>(reinterpret_cast<int8_t*>(c->d_rembits) + rembits);
+  c->d_kend = c->d_kbeg + N;
+  c->d_ktotal = reinterpret_cast<unsigned long long*>(c->d_kend + N);
+  c->d_kidx = reinterpret_cast<int32_t*>(c->d_ktotal + 1);
+  c->d_kval = reinterpret_cast<float*>(c->d_kidx + nonzero);
+  c->i8_nonzero = nonzero;
   bool ok = i8_encode(&c->tmXp, c->d_digits, npa, kI8Digits * R, ldK, false) &&
             i8_encode(&c->tmXn, c->d_digits, N, kI8Digits * R, ldT, false);
   for (int k = 0; k < planes && ok; ++k)
@@ -994,19 +1019,18 @@ static emc_status finish_patterns(emc_context* c) {
   cudaError_t e = launch_pattern_stats(compact, nullptr, N, npa, npa, 1, c->d_patsq, c->st);
   if (e == cudaSuccess) e = launch_pattern_stats(compact, nullptr, N, npa, npa, 0, c->d_patsum, c->st);
   int bad = 0;
-  // mixed: [0] counts the path cannot take; FP32: largest count (bits),
-  // non-integers, invalid counts
-  unsigned int seen[3] = {0, 0, 0};
-  unsigned int* d_seen = reinterpret_cast<unsigned int*>(c->d_scratch);
+  // mixed: the first word takes the number of counts the path cannot take
+  CountRange seen{};
+  CountRange* d_seen = reinterpret_cast<CountRange*>(c->d_scratch);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_seen, 0, sizeof(seen), c->st);
   if (e == cudaSuccess && c->mixed)
     e = launch_pack_patterns(compact, N, npa, c->Npad, c->Ppad, c->d_Kh, c->d_Kt,
                              reinterpret_cast<int*>(d_seen), c->st);
   else if (e == cudaSuccess)
     e = launch_count_range(compact, N * npa, (float)kI8MaxCount2, d_seen, c->st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(seen, d_seen, sizeof(seen), cudaMemcpyDeviceToHost, c->st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&seen, d_seen, sizeof(seen), cudaMemcpyDeviceToHost, c->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
-  bad = (int)(c->mixed ? seen[0] : seen[2]);
+  bad = (int)(c->mixed ? seen.largest : seen.bad);
   if (e != cudaSuccess) return c->cuda(e, "emc_set_patterns");
   c->have_pat = false;
   if (bad && c->mixed)
@@ -1015,13 +1039,16 @@ static emc_status finish_patterns(emc_context* c) {
                    bad);
   if (bad)
     return c->fail(EMC_ERR_RANGE, "%d counts are negative, NaN or infinite", bad);
-  if (!c->mixed && seen[1] == 0) {
+  if (!c->mixed && seen.odd == 0) {
     float top;
-    std::memcpy(&top, &seen[0], sizeof(top));
-    i8_prepare(c, top);
-    if (c->i8_planes)
+    std::memcpy(&top, &seen.largest, sizeof(top));
+    i8_prepare(c, top, (int64_t)seen.nonzero);
+    if (c->i8_planes) {
       CK(c, launch_pack_counts_i8(compact, N, npa, c->i8_planes, round_up(npa, 16),
-                                  round_up(N, 16), c->d_K8, c->d_Kt8, c->st));
+                                  round_up(N, 16), c->d_K8, c->d_Kt8, c->d_ktot, c->st));
+      CK(c, launch_photon_lists(compact, N, npa, c->d_kbeg, c->d_kend, c->d_kidx, c->d_kval,
+                                c->d_ktotal, c->st));
+    }
   } else {
     c->drop_i8();
   }
@@ -1685,7 +1712,7 @@ static emc_status i8_loglik(emc_context* c) {
     c->launches += 1;
   }
   CK(c, launch_quant_rows(c->d_S, nullptr, c->d_rowmax, c->R, c->npa, round_up(c->npa, 16),
-                          c->d_digits, c->d_unit, c->st));
+                          c->d_digits, c->d_unit, nullptr, nullptr, nullptr, c->st));
   I8LLArgs a{};
   a.R = c->R;
   a.N = c->N;
@@ -1710,19 +1737,40 @@ static emc_status i8_loglik(emc_context* c) {
 static emc_status i8_slicesums(emc_context* c) {
   TRY(current_maxima(c, c->d_LL, c->d_scaling, c->N));
   CK(c, launch_quant_rows(c->d_LL, c->d_scaling, c->d_rowmax, c->R, c->N, round_up(c->N, 16),
-                          c->d_digits, c->d_unit, c->st));
+                          c->d_digits, c->d_unit, c->d_small, c->d_rembits,
+                          c->d_remcount, c->st));
   I8UArgs a{};
   a.R = c->R;
   a.npa = c->npa;
   a.unit = c->d_unit;
   a.T = c->d_T;
   a.U = c->d_S;  // the averaged slices replace the expanded ones (emc_atomic.cu:96)
+  a.ktot = c->d_ktot;
+  a.flag = c->d_small;
   for (int k = c->i8_planes - 1; k >= 0; --k) {
     a.pass = c->i8_planes == 1 ? I8_ONLY : k ? I8_HIGH : I8_LOW;
     a.mult = k ? 128.0 : 1.0;
     CK(c, launch_i8_slices(c->tmKt8[k], c->tmXn, c->N, a, c->d_status, c->num_sms, c->st));
   }
-  c->launches += 1 + c->i8_planes;
+  I8SmallArgs f{};
+  f.R = c->R;
+  f.N = c->N;
+  f.npa = c->npa;
+  f.P = c->d_LL;
+  f.phi = c->d_scaling;
+  f.unit = c->d_unit;
+  f.T = c->d_T;
+  f.Tskip = c->d_Tskip;
+  f.flag = c->d_small;
+  f.bits = c->d_rembits;
+  f.count = c->d_remcount;
+  f.kbeg = c->d_kbeg;
+  f.kend = c->d_kend;
+  f.kidx = c->d_kidx;
+  f.kval = c->d_kval;
+  f.U = c->d_S;
+  CK(c, launch_small_terms(f, c->num_sms, c->st));
+  c->launches += 2 + c->i8_planes;
   return EMC_OK;
 }
 
@@ -1822,6 +1870,7 @@ emc_status emc_maximize(emc_context* c) {
     a.Mpart = c->d_Mpart;
     a.T = c->d_T;
     a.rowmax = c->d_rowmax;
+    a.zero = c->i8_planes ? c->d_remcount : nullptr;
     CK(c, launch_resp_f32(a, c->st));
     if (cross) {
       CrossArgs x{};

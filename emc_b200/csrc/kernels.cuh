@@ -142,6 +142,7 @@ struct RespF32Args {
   float* Mpart;            // [resp_f32_blocks(N)][R]
   float* T;                // [R]
   float* rowmax;           // [R]
+  int32_t* zero;           // [R] zeroed (optional)
 };
 int64_t resp_f32_chunk(int64_t R, int64_t N);
 int64_t resp_f32_blocks(int64_t N);

@@ -762,6 +762,7 @@ __global__ void resp_rows_kernel(const RespF32Args a, int64_t nblk) {
   }
   a.T[r] = (float)t;
   a.rowmax[r] = __uint_as_float(mx);
+  if (a.zero) a.zero[r] = 0;
 }
 
 __global__ void xlogx_partial(const float* x, int64_t n, double* part) {

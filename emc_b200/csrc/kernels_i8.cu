@@ -9,9 +9,13 @@
 // in two passes).  tcgen05.mma kind::i8 multiplies the bytes and accumulates
 // in 32-bit integers, one TMEM accumulator per digit, and the epilogue
 // recombines the four sums as one 64-bit integer: no rounding happens between
-// the quantisation and the final conversion to FP64.  The quantisation error
-// (2^-31 of the row maximum per element) is below the rounding of the FP32
-// partial sums it replaces.
+// the quantisation and the final conversion to FP64.  The quantisation error is
+// absolute, 2^-31 of the row maximum per element.  For the log-likelihood, a sum
+// over the same row, that is below the rounding of the FP32 partial sums it
+// replaces.  The slice sums need relative precision: a pixel may have photons
+// only from patterns whose responsibility is far below the row's largest.  Where a
+// sum is so small that the fixed point shows, small_terms_kernel adds what it
+// left out.
 //
 // What bounds it: the tensor pipe; four byte digits cost the MMA time of two
 // FP16 operand halves.  Measured (10,000 patterns x 25,680 rotations x 4,044
@@ -67,6 +71,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&v)[8]) {
 struct ColConst {
   double unit;  // value of one unit of the column's integer sum
   double c;     // per-column term of the epilogue
+  float few;    // slice sums: kSmallUnits units
 };
 
 // LL[n][m], n = rotation, m = pattern:
@@ -101,26 +106,47 @@ struct EpiLL {
     if (a.pass == I8_LOW) x += *o;
     *o = a.poisson ? fma(-c1, k.c, x) : fma(x, c1, c0 - k.c);
   }
+  __device__ void stored(int64_t, int) {}
 };
 
-// U[n][m] = sum / T_n, n = rotation, m = active pixel (emc_atomic.cu:105-111)
+// U[n][m] = sum / T_n, n = rotation, m = active pixel (emc_atomic.cu:105-111).
+// A term is off by half a unit at most, so a sum of at least kSmallUnits units
+// per photon at the pixel is within 2^-21, and within that over the root of the
+// number of terms where the errors are independent.  Rows with a smaller sum are
+// flagged: none of them with broad posteriors (10,000 patterns x 25,680 rotations
+// gaussian), nearly all with sharp ones.
+constexpr float kSmallUnits = 1048576.0f;
 struct EpiU {
   I8UArgs a;
+  float kt;
+  uint32_t small = 0;
   __device__ void column(int64_t n, ColConst& k) const {
     const bool ok = n < a.R;
     const float T = ok ? a.T[n] : 1.0f;
-    k.unit = ok ? (double)a.unit[n] * a.mult / (T > 1e-30f ? (double)T : 1.0) : 0.0;
+    const double u = ok ? (double)a.unit[n] / (T > 1e-30f ? (double)T : 1.0) : 0.0;
+    k.unit = u * a.mult;
     k.c = 0.0;
+    k.few = (float)u * kSmallUnits;
   }
-  __device__ void row(int64_t) {}
-  __device__ void store(int64_t m, int64_t n, long long v, const ColConst& k) const {
+  __device__ void row(int64_t m) { kt = m < a.npa ? (float)a.ktot[m] : 0.0f; }
+  __device__ void store(int64_t m, int64_t n, long long v, const ColConst& k) {
     if (m >= a.npa || n >= a.R) return;
     float* o = a.U + n * a.npa + m;
     double x = (double)v * k.unit;
     if (a.pass == I8_LOW) x += (double)*o;
-    *o = (float)x;
+    const float y = (float)x;
+    *o = y;
+    if (y <= kt * k.few) small |= 1u << (n & 31);
+  }
+  // One store of 32 flags per warp: every SM is at the same rows, and a store per
+  // element to them took longer than the contraction.
+  __device__ void stored(int64_t n0, int lane) {
+    const uint32_t b = __reduce_or_sync(0xffffffffu, kt > 0.0f ? small : 0u);
+    if (a.pass != I8_HIGH && n0 + lane < a.R && (b >> lane & 1u)) a.flag[n0 + lane] = 1;
+    small = 0;
   }
 };
+static_assert(kWarpCols == 32, "EpiU keeps a bit per column");
 
 template <class Epi>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + kEpiThreads, 1)
@@ -327,6 +353,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + kEpiThreads, 1)
       const int64_t n0 = nt * kTileN + col0;
 #pragma unroll
       for (int c = 0; c < kWarpCols; ++c) e.store(m, n0 + c, sum[c], cc[col0 + c]);
+      e.stored(n0, lane);
     }
   }
   tc_fence_before();
@@ -374,11 +401,20 @@ __device__ __forceinline__ uint32_t digits_of(int q) {
 // 3.63 ms, the maximize stage of 12,800 x 25,680 2.92 -> 2.84 ms.
 constexpr int kQuantRows = 8, kQuantStep = 4;
 
+// 1 / d = r + rl, rl to first order in the rounding of r; x / d from them.
+__device__ __forceinline__ void reciprocal(float d, float& r, float& rl) {
+  r = 1.0f / d;
+  rl = r * fmaf(-r, d, 1.0f);
+}
+__device__ __forceinline__ float quotient(float x, float r, float rl) { return fmaf(x, r, x * rl); }
+
 template <bool DIV>
 __global__ void __launch_bounds__(256) quant_rows_kernel(const float* X, const float* div,
                                                          const float* rowmax, int64_t R,
                                                          int64_t cols, int64_t ld, int rows,
-                                                         int8_t* D, float* unit) {
+                                                         int8_t* D, float* unit,
+                                                         int32_t* flag, uint32_t* bits,
+                                                         int32_t* count) {
   __shared__ float ups[kQuantRows];
   const int64_t chunks = (ld + 1023) / 1024, rb = blockIdx.x / chunks;
   const int64_t r0 = rb * rows, c0 = (blockIdx.x - rb * chunks) * 1024;
@@ -397,20 +433,18 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const float* X, const f
     }
     ups[threadIdx.x] = up;
     if (c0 == 0) unit[r0 + threadIdx.x] = one;
+    if (c0 == 0 && flag) flag[r0 + threadIdx.x] = 0;
   }
   const int64_t j0 = c0 + 4 * threadIdx.x;
-  // 1 / phi = r + r (1 - r phi), to first order in the rounding of r
   float r[4], rl[4];
   if (DIV) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float d = j0 + i < cols ? div[j0 + i] : 1.0f;
-      r[i] = 1.0f / d;
-      rl[i] = r[i] * fmaf(-r[i], d, 1.0f);
-    }
+    for (int i = 0; i < 4; ++i) reciprocal(j0 + i < cols ? div[j0 + i] : 1.0f, r[i], rl[i]);
   }
   __syncthreads();
+  const uint32_t live = __ballot_sync(0xffffffffu, j0 < ld);
   if (j0 >= ld) return;
+  const int64_t words = i8_bit_words(cols), word = 4 * (j0 / 128);
   const bool wide = cols % 4 == 0;  // then so is j0 < cols for the four columns
   for (int h = 0; h < rows; h += kQuantStep) {
     float v[kQuantStep][4];
@@ -431,11 +465,20 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const float* X, const f
     for (int k = 0; k < kQuantStep; ++k) {
       if (r0 + h + k >= R) break;
       const float up = ups[h + k];
-      uint32_t w[4];
+      uint32_t w[4], rem[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float q = DIV ? fmaf(v[k][i], r[i], v[k][i] * rl[i]) : v[k][i];
-        w[i] = digits_of(__float2int_rn(q * up));
+        const float q = DIV ? quotient(v[k][i], r[i], rl[i]) : v[k][i];
+        const float t = q * up;
+        w[i] = digits_of(__float2int_rn(t));
+        // 0 < t < 2^23: there may be a remainder
+        if (DIV) rem[i] = __ballot_sync(live, __float_as_uint(t) - 1u < 0x4affffffu);
+      }
+      if (DIV && threadIdx.x % 32 == 0) {
+        *reinterpret_cast<uint4*>(bits + (r0 + h + k) * words + word) =
+            make_uint4(rem[0], rem[1], rem[2], rem[3]);
+        const int n = __popc(rem[0]) + __popc(rem[1]) + __popc(rem[2]) + __popc(rem[3]);
+        if (n) atomicAdd(count + r0 + h + k, n);
       }
       // four columns' digits to four digits' columns
       const uint32_t a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140);
@@ -447,6 +490,158 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const float* X, const f
       *reinterpret_cast<uint32_t*>(o + 2 * plane) = __byte_perm(c, d, 0x5410);
       *reinterpret_cast<uint32_t*>(o + 3 * plane) = __byte_perm(c, d, 0x7632);
     }
+  }
+}
+
+// U[r][j] += sum_p e_rp K_pj / T_r with e = P / phi - q unit, what launch_quant_rows
+// left of an element (exact in FP32: q below 2^23 where there is a remainder, and
+// all of the element where q is 0), for the rows that are flagged and inserted.
+//
+// A block takes a row at a time: the elements that may have a remainder are a bit
+// each (launch_quant_rows), so it lists them, a thread an element; then a warp
+// takes an element, or a part of one where there are few, and adds its pattern's
+// photon list into the row's slice in shared memory.  With sharp posteriors few P
+// are above zero: 2,000 x 25,680 at 128^2 (37% of the rows inserted, 53 remainders
+// in the median one, 700 at most) 0.94 ms, the shared-memory additions, 3.4e11 a
+// second; 10,000 x 25,680 at 64^2, poisson (34%, 3 and 284) 0.39 ms, latency; 64 x
+// 420 at 16^2 14 us.  Without a flagged row a block reads its flags and ends: 2 us.
+// Scanning the row of P for the elements: 1.2 to 1.4 ms; count bytes instead of
+// photon lists: 2.9 ms at 128^2, every pixel of a pattern looked at.
+constexpr int kSmallThreads = 512, kSmallWarps = kSmallThreads / 32;
+constexpr int kSmallList = 384, kSmallUnroll = 4;
+constexpr int64_t kSmallPixels = 48 << 10;  // of a slice in shared memory
+
+// Blocks that share a row of `count` elements: with broad posteriors a row may have
+// a thousand (1,000 x 3,240 at 32^2 gaussian: one block took 95 us over it).
+constexpr int kSmallParts = 8, kSmallShare = 128;
+__device__ __forceinline__ int small_parts(int count) {
+  const int n = count / kSmallShare;
+  return n < 1 ? 1 : n < kSmallParts ? n : kSmallParts;
+}
+
+__global__ void __launch_bounds__(kSmallThreads, 3) small_terms_kernel(const I8SmallArgs a,
+                                                              const int64_t tile) {
+  extern __shared__ float slice[];  // [tile]
+  __shared__ uint32_t need[kSmallWarps];
+  __shared__ int part[kSmallWarps];
+  __shared__ int32_t lp[kSmallList], ln[kSmallList];
+  __shared__ float le[kSmallList];
+  __shared__ int64_t lb[kSmallList];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t words = i8_bit_words(a.N);
+  const int64_t units = a.R * kSmallParts;
+  for (int64_t base = blockIdx.x; base < units; base += (int64_t)gridDim.x * kSmallThreads) {
+    const int64_t mine = base + (int64_t)threadIdx.x * gridDim.x, row = mine % a.R;
+    bool n = false;
+    if (mine < units) {
+      const float T = a.T[row];
+      n = a.flag[row] != 0 && (a.Tskip ? a.Tskip[row] : T) > 1e-10f && T > 0.0f &&
+          mine / a.R < small_parts(a.count[row]);
+    }
+    const uint32_t b = __ballot_sync(0xffffffffu, n);
+    if (lane == 0) need[w] = b;
+    if (!__syncthreads_or(n)) continue;
+    // (row, part, pixel tile) after another, the same for every thread
+    for (int i = 0; i < kSmallWarps; ++i)
+      for (uint32_t rest = need[i]; rest; rest &= rest - 1)
+        for (int64_t j0 = 0; j0 < a.npa; j0 += tile) {
+          const int64_t unit = base + (32 * i + __ffs(rest) - 1) * (int64_t)gridDim.x;
+          const int64_t r = unit % a.R, share = unit / a.R;
+          // elements lo .. hi - 1 of the row's, `seen` of them before these words
+          const int count = a.count[r], shares = small_parts(count);
+          const int lo = (int)(count * share / shares), hi = (int)(count * (share + 1) / shares);
+          int seen = 0;
+          const int px = (int)(a.npa - j0 < tile ? a.npa - j0 : tile);
+          const float one = a.unit[r], up = one > 0.0f ? 1.0f / one : 0.0f;
+          bool any = false;
+          for (int64_t g0 = 0; g0 < words; g0 += kSmallThreads) {
+            const int64_t g = g0 + threadIdx.x;
+            const uint32_t word = g < words ? a.bits[r * words + g] : 0u;
+            // each thread's place among the elements of these words
+            int place = __popc(word), total = 0;
+            const int own = place;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const int v = __shfl_up_sync(0xffffffffu, place, o);
+              if (lane >= o) place += v;
+            }
+            if (lane == 31) part[w] = place;
+            __syncthreads();
+            place -= own;
+            for (int k = 0; k < kSmallWarps; ++k) {
+              const int v = part[k];
+              if (k < w) place += v;
+              total += v;
+            }
+            const int from = lo > seen ? lo - seen : 0, to = hi - seen < total ? hi - seen : total;
+            if (from < to && !any) {
+              for (int j = threadIdx.x; j < px; j += kSmallThreads) slice[j] = 0.0f;
+              any = true;
+            }
+            for (int done = from; done < to; done += kSmallList) {
+              const int m = to - done < kSmallList ? to - done : kSmallList;
+              int at = place - done;
+              for (uint32_t z = word; z; z &= z - 1, ++at)
+                if ((unsigned)at < (unsigned)m)
+                  lp[at] = (int32_t)((g >> 2) * 128 + 4 * (__ffs(z) - 1) + (g & 3));
+              __syncthreads();
+              for (int q = threadIdx.x; q < m; q += kSmallThreads) {
+                const int64_t p = lp[q], beg = a.kbeg[p];
+                float rc, rl;
+                reciprocal(a.phi[p], rc, rl);
+                const float x = quotient(a.P[r * a.N + p], rc, rl);
+                le[q] = fmaf(-(float)__float2int_rn(x * up), one, x);
+                lb[q] = beg;
+                ln[q] = (int)(a.kend[p] - beg);
+              }
+              __syncthreads();
+              // few elements: several warps each, a part of its list
+              const int parts = m < kSmallWarps ? kSmallWarps / m : 1;
+              for (int u = w; u < m * parts; u += kSmallWarps) {
+                const int q = u % m, nq = ln[q];
+                const int64_t t0 = lb[q];
+                const float x = le[q];
+                const int step = 32 * kSmallUnroll;
+                for (int t = u / m * step + lane; t < nq; t += parts * step) {
+                  int j[kSmallUnroll];
+                  float c[kSmallUnroll];
+#pragma unroll
+                  for (int z = 0; z < kSmallUnroll; ++z) {
+                    const bool in = t + 32 * z < nq;
+                    j[z] = in ? a.kidx[t0 + t + 32 * z] - (int)j0 : -1;
+                    c[z] = in ? a.kval[t0 + t + 32 * z] : 0.0f;
+                  }
+#pragma unroll
+                  for (int z = 0; z < kSmallUnroll; ++z)
+                    if ((unsigned)j[z] < (unsigned)px) atomicAdd(slice + j[z], x * c[z]);
+                }
+              }
+              __syncthreads();  // lists and `part` are written again
+            }
+            if (from >= to) __syncthreads();
+            seen += total;
+          }
+          if (!any) continue;
+          const float T = a.T[r], inv = T > 1e-30f ? 1.0f / T : 1.0f;
+          float* o = a.U + r * a.npa + j0;
+          for (int j = threadIdx.x; j < px; j += kSmallThreads * kSmallUnroll) {
+            float u[kSmallUnroll];
+#pragma unroll
+            for (int z = 0; z < kSmallUnroll; ++z)
+              u[z] = j + z * kSmallThreads < px ? o[j + z * kSmallThreads] : 0.0f;
+#pragma unroll
+            for (int z = 0; z < kSmallUnroll; ++z)
+              if (j + z * kSmallThreads < px) {
+                const float x = slice[j + z * kSmallThreads];
+                if (shares == 1)
+                  o[j + z * kSmallThreads] = fmaf(x, inv, u[z]);
+                else if (x != 0.0f)
+                  atomicAdd(o + j + z * kSmallThreads, x * inv);
+              }
+          }
+          __syncthreads();
+        }
+    __syncthreads();  // `need` is written again
   }
 }
 
@@ -471,9 +666,11 @@ __global__ void __launch_bounds__(256) row_maxima_kernel(const float* X, const f
 }
 
 // Counts K [N][npa] as bytes by pattern (K8 [planes][N][ldK]) and by pixel
-// (Kt8 [planes][npa][ldT]), base-128 digits when planes == 2.
+// (Kt8 [planes][npa][ldT]), base-128 digits when planes == 2, and each pixel's
+// total (kI8MaxTotal keeps it below 2^32).
 __global__ void pack_counts_i8_kernel(const float* K, int64_t N, int64_t npa, int planes,
-                                      int64_t ldK, int64_t ldT, int8_t* K8, int8_t* Kt8) {
+                                      int64_t ldK, int64_t ldT, int8_t* K8, int8_t* Kt8,
+                                      uint32_t* ktot) {
   __shared__ int tile[32][33];
   const int64_t jb = (npa + 31) / 32;
   const int64_t j0 = blockIdx.x % jb * 32, p0 = blockIdx.x / jb * 32;
@@ -489,16 +686,54 @@ __global__ void pack_counts_i8_kernel(const float* K, int64_t N, int64_t npa, in
   __syncthreads();
   for (int i = ty; i < 32; i += 8) {
     const int64_t j = j0 + i, p = p0 + tx;
+    const uint32_t sum = __reduce_add_sync(0xffffffffu, (uint32_t)tile[tx][i]);
+    if (tx == 0 && j < npa && sum) atomicAdd(ktot + j, sum);
     if (p < N && j < npa)
       for (int s = 0; s < planes; ++s)
         Kt8[((int64_t)s * npa + j) * ldT + p] = (int8_t)((tile[tx][i] >> (7 * s)) & 127);
   }
 }
 
+// The photon lists of the patterns: pattern p's non-zero pixels and counts at
+// beg[p] .. end[p] - 1, the lists one after the other in no particular order of
+// patterns (total[0]: 0 on entry), so no scan over them is needed.  One warp per
+// pattern, which counts and then fills.
+__global__ void photon_lists_kernel(const float* K, int64_t N, int64_t npa, int64_t* beg,
+                                    int64_t* end, int32_t* idx, float* val,
+                                    unsigned long long* total) {
+  const int64_t p = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (p >= N) return;
+  const float* row = K + p * npa;
+  uint32_t n = 0;
+  for (int64_t j = lane; j < npa; j += 32) n += row[j] != 0.0f;
+  n = __reduce_add_sync(0xffffffffu, n);
+  unsigned long long at = 0;
+  if (lane == 0) {
+    at = atomicAdd(total, (unsigned long long)n);
+    beg[p] = (int64_t)at;
+    end[p] = (int64_t)at + n;
+  }
+  at = __shfl_sync(0xffffffffu, at, 0);
+  for (int64_t j0 = 0; j0 < npa; j0 += 32) {
+    const int64_t j = j0 + lane;
+    const float k = j < npa ? row[j] : 0.0f;
+    const uint32_t nz = __ballot_sync(0xffffffffu, k != 0.0f);
+    if (k != 0.0f) {
+      const unsigned long long o = at + __popc(nz & ((1u << lane) - 1u));
+      idx[o] = (int32_t)j;
+      val[o] = k;
+    }
+    at += __popc(nz);
+  }
+}
+
 // out[0] = bits of the largest entry, out[1] += entries that are not integers
-// in [0, limit], out[2] += entries that are negative, NaN or infinite.
-__global__ void count_range_kernel(const float* x, int64_t n, float limit, unsigned int* out) {
-  unsigned int mx = 0, odd = 0, bad = 0;
+// in [0, limit], out[2] += entries that are negative, NaN or infinite; nonzero[0]
+// += the entries that are not 0.
+__global__ void count_range_kernel(const float* x, int64_t n, float limit, unsigned int* out,
+                                   unsigned long long* nonzero) {
+  unsigned int mx = 0, odd = 0, bad = 0, nz = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const float v = x[i];
@@ -507,15 +742,18 @@ __global__ void count_range_kernel(const float* x, int64_t n, float limit, unsig
       continue;
     }
     if (!(v <= limit && v == floorf(v))) ++odd;
+    if (v != 0.0f) ++nz;
     mx = max(mx, __float_as_uint(fabsf(v)));
   }
   mx = __reduce_max_sync(0xffffffffu, mx);
   odd = __reduce_add_sync(0xffffffffu, odd);
   bad = __reduce_add_sync(0xffffffffu, bad);
+  nz = __reduce_add_sync(0xffffffffu, nz);  // fewer than 2^32 a warp
   if ((threadIdx.x & 31) == 0) {
     if (mx) atomicMax(out, mx);
     if (odd) atomicAdd(out + 1, odd);
     if (bad) atomicAdd(out + 2, bad);
+    if (nz) atomicAdd(nonzero, (unsigned long long)nz);
   }
 }
 
@@ -542,17 +780,34 @@ cudaError_t launch_i8_slices(const CUtensorMap& tmKt, const CUtensorMap& tmX, in
 }
 
 cudaError_t launch_quant_rows(const float* X, const float* div, const float* rowmax, int64_t R,
-                              int64_t cols, int64_t ld, int8_t* D, float* unit, cudaStream_t st) {
+                              int64_t cols, int64_t ld, int8_t* D, float* unit, int32_t* flag,
+                              uint32_t* bits, int32_t* count, cudaStream_t st) {
   if (R <= 0) return cudaSuccess;
-  if (ld % 16 != 0 || ld < cols) return cudaErrorInvalidValue;
+  if (ld % 16 != 0 || ld < cols || (div && !(flag && bits && count))) return cudaErrorInvalidValue;
   int rows = kQuantRows;
   const int64_t chunks = (ld + 1023) / 1024;
   while (rows > kQuantStep && chunks * ((R + rows - 1) / rows) < 4 * 148) rows /= 2;
   const unsigned grid = (unsigned)(chunks * ((R + rows - 1) / rows));
   if (div)
-    quant_rows_kernel<true><<<grid, 256, 0, st>>>(X, div, rowmax, R, cols, ld, rows, D, unit);
+    quant_rows_kernel<true><<<grid, 256, 0, st>>>(X, div, rowmax, R, cols, ld, rows, D, unit,
+                                                    flag, bits, count);
   else
-    quant_rows_kernel<false><<<grid, 256, 0, st>>>(X, div, rowmax, R, cols, ld, rows, D, unit);
+    quant_rows_kernel<false><<<grid, 256, 0, st>>>(X, div, rowmax, R, cols, ld, rows, D, unit,
+                                                    flag, bits, count);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_small_terms(const I8SmallArgs& a, int num_sms, cudaStream_t st) {
+  if (a.R <= 0 || a.N <= 0) return cudaSuccess;
+  const int64_t tile = std::min<int64_t>((a.npa + 31) / 32 * 32, kSmallPixels);
+  const size_t smem = sizeof(float) * (size_t)tile;
+  const cudaError_t e = cudaFuncSetAttribute(
+      small_terms_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  // as many blocks an SM, up to three, as slices and lists (20 bytes an element) fit
+  const int64_t per_sm = std::clamp<int64_t>((227 << 10) / (smem + 20 * kSmallList + 1400), 1, 3);
+  const int64_t grid = std::min<int64_t>(a.R * kSmallParts, per_sm * num_sms);
+  small_terms_kernel<<<(unsigned)grid, kSmallThreads, smem, st>>>(a, tile);
   return cudaGetLastError();
 }
 
@@ -564,18 +819,32 @@ cudaError_t launch_row_maxima(const float* X, const float* div, int64_t R, int64
 }
 
 cudaError_t launch_pack_counts_i8(const float* K, int64_t N, int64_t npa, int planes, int64_t ldK,
-                                  int64_t ldT, int8_t* K8, int8_t* Kt8, cudaStream_t st) {
+                                  int64_t ldT, int8_t* K8, int8_t* Kt8, uint32_t* ktot,
+                                  cudaStream_t st) {
+  const cudaError_t e = cudaMemsetAsync(ktot, 0, sizeof(uint32_t) * npa, st);
+  if (e != cudaSuccess) return e;
   const int64_t grid = ((npa + 31) / 32) * ((N + 31) / 32);
-  pack_counts_i8_kernel<<<(unsigned)grid, dim3(32, 8), 0, st>>>(K, N, npa, planes, ldK, ldT, K8, Kt8);
+  pack_counts_i8_kernel<<<(unsigned)grid, dim3(32, 8), 0, st>>>(K, N, npa, planes, ldK, ldT, K8,
+                                                               Kt8, ktot);
   return cudaGetLastError();
 }
 
-cudaError_t launch_count_range(const float* x, int64_t n, float limit, unsigned int* out,
+cudaError_t launch_photon_lists(const float* K, int64_t N, int64_t npa, int64_t* beg, int64_t* end,
+                                int32_t* idx, float* val, unsigned long long* total,
+                                cudaStream_t st) {
+  const cudaError_t e = cudaMemsetAsync(total, 0, sizeof(unsigned long long), st);
+  if (e != cudaSuccess || N <= 0) return e;
+  photon_lists_kernel<<<(unsigned)((N + 7) / 8), 256, 0, st>>>(K, N, npa, beg, end, idx, val,
+                                                               total);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_count_range(const float* x, int64_t n, float limit, CountRange* out,
                                cudaStream_t st) {
-  const cudaError_t e = cudaMemsetAsync(out, 0, 3 * sizeof(unsigned int), st);
+  const cudaError_t e = cudaMemsetAsync(out, 0, sizeof(CountRange), st);
   if (e != cudaSuccess || n <= 0) return e;
-  count_range_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 1184), 256, 0, st>>>(x, n,
-                                                                                        limit, out);
+  count_range_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 1184), 256, 0, st>>>(
+      x, n, limit, &out->largest, &out->nonzero);
   return cudaGetLastError();
 }
 
