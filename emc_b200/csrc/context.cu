@@ -242,6 +242,7 @@ struct emc_context {
   float2* d_acc = nullptr;  // interleaved (model, weight) accumulators
   float2* d_acc_odd = nullptr;  // trilinear: the shifted pairs (InsertAcc), behind d_acc
   int64_t acc_stride = 0;       // pairs from one copy of both to the next
+  int64_t acc_odd_at = 0;       // where d_acc_odd lies, 0: nowhere
   int acc_copies = 1;
   double *d_lse = nullptr, *d_plogp = nullptr;
   float* d_Tpart = nullptr;
@@ -386,10 +387,43 @@ struct emc_context {
     return fail(e == cudaErrorMemoryAllocation ? EMC_ERR_OOM : EMC_ERR_CUDA, "%s: %s", what,
                 cudaGetErrorString(e));
   }
+  // Allocations between begin_group and end_group are one cudaMalloc (a millisecond
+  // each above a megabyte, and as long to free): what is never released by itself.
+  // Their pointers are set by end_group.
+  struct Grouped {
+    void** p;
+    size_t offset, bytes;
+    bool zero;
+  };
+  std::vector<Grouped> group;
+  size_t group_bytes = 0;
+  bool grouping = false;
+  void begin_group() {
+    grouping = true;
+    group.clear();
+    group_bytes = 0;
+  }
+  emc_status end_group() {
+    grouping = false;
+    char* q = nullptr;
+    emc_status s = alloc(&q, group_bytes);
+    for (const Grouped& g : group) {
+      if (s != EMC_OK) break;
+      *g.p = q + g.offset;
+      if (g.zero) s = cuda(cudaMemsetAsync(*g.p, 0, g.bytes, st), "memset");
+    }
+    group_bytes = 0;
+    return s;
+  }
   template <class T>
   emc_status alloc(T** p, size_t count, bool zero = false) {
     void* q = nullptr;
     const size_t bytes = count * sizeof(T) ? count * sizeof(T) : 16;
+    if (grouping) {
+      group.push_back({reinterpret_cast<void**>(p), group_bytes, bytes, zero});
+      group_bytes += (bytes + 1023) / 1024 * 1024;
+      return EMC_OK;
+    }
     if (mem_limit && mem_used + bytes > mem_limit && mem_used - spare() + bytes <= mem_limit)
       make_room();
     if (mem_limit && mem_used + bytes > mem_limit)
@@ -689,6 +723,14 @@ static emc_status set_y_rows(emc_context* c, int64_t rows) {
   return EMC_OK;
 }
 
+// Whether `bytes` are an eighth or less of the memory left (besides `pending`).
+// Without a limit a few megabytes always are; asking takes 0.1 ms.
+static bool small_part(emc_context* c, size_t bytes, size_t pending) {
+  if (!c->mem_limit && bytes <= ((size_t)4 << 20)) return true;
+  const size_t a = avail_bytes(c, 0);
+  return a > pending && bytes <= (a - pending) / 8;
+}
+
 // The insertion accumulators: for an FP32 context copies of up to 16 MB in all
 // (they stay in L2; measured 10-15% off the compress of 1,000 patterns x 3,240
 // rotations with an unmasked centre, and a shorter FP32 sum per voxel; mixed
@@ -703,18 +745,22 @@ static emc_status alloc_acc(emc_context* c, bool needed) {
   int copies = 1;
   while (!c->mixed && copies < 8 && (int64_t)sizeof(float2) * stride * copies * 2 <= (16 << 20)) copies *= 2;
   const size_t bytes = sizeof(float2) * (size_t)(stride * copies);
-  const bool room = bytes <= avail_bytes(c, 0) / 8;
+  const bool room = small_part(c, bytes, c->group_bytes);
   if (!room && !needed) return EMC_OK;
   c->acc_copies = room ? copies : 1;
   c->acc_stride = room ? stride : c->M;
   TRY(c->alloc(&c->d_acc, c->acc_stride * c->acc_copies, true));
-  if (room && tri) c->d_acc_odd = c->d_acc + one;
+  c->acc_odd_at = room && tri ? one : 0;
   return EMC_OK;
+}
+static void place_acc(emc_context* c) {
+  c->d_acc_odd = c->acc_odd_at ? c->d_acc + c->acc_odd_at : nullptr;
 }
 
 static emc_status alloc_work(emc_context* c) {
   // called once geometry is known (npa fixes every pixel dimension)
   const int64_t R = c->R, N = c->N, npa = c->npa;
+  c->begin_group();
   if (c->cfg.interp == EMC_INTERP_TRILINEAR)
     TRY(c->alloc(&c->d_tri, tri_table_entries(c->cfg.side)));
   // (FP32 contexts: half as many again for the row maxima)
@@ -729,25 +775,24 @@ static emc_status alloc_work(emc_context* c) {
     TRY(c->alloc(&c->d_LL64, R * N));
     TRY(c->alloc(&c->d_K, N * npa));
     TRY(alloc_acc(c, false));
-    // the responsibility pass's scratch, one allocation
+    // the responsibility pass's scratch (the partials' room also serves the
+    // CUDA-core cross term, ceil(R / 128) a pattern)
     const int64_t chunk = resp_f32_chunk(R, N), nparts = (R + chunk - 1) / chunk;
     const int64_t nb = resp_f32_blocks(N);
-    double* w = nullptr;
-    // (the partials' room also serves the CUDA-core cross term, ceil(R / 128) a
-    // pattern)
     const int64_t part = std::max(4 * nparts, (R + 127) / 128) * N;
-    TRY(c->alloc(&w, part + nb * R + 2 * N + (nb * R + R + 1) / 2));
-    c->d_part64 = reinterpret_cast<double4*>(w);
-    c->d_Tpart64 = w + part;
-    c->d_plogp32 = c->d_Tpart64 + nb * R;
-    c->d_lse32 = c->d_plogp32 + N;
-    c->d_Mpart = reinterpret_cast<float*>(c->d_lse32 + N);
-    c->d_rowmax = c->d_Mpart + nb * R;
+    TRY(c->alloc(reinterpret_cast<double**>(&c->d_part64), part));
+    TRY(c->alloc(&c->d_Tpart64, nb * R));
+    TRY(c->alloc(&c->d_plogp32, N));
+    TRY(c->alloc(&c->d_lse32, N));
+    TRY(c->alloc(&c->d_Mpart, nb * R));
+    TRY(c->alloc(&c->d_rowmax, R));
+    TRY(c->end_group());
+    place_acc(c);
     // poisson: a table of (W, log W), where it is a small part of the memory left
     // (25,680 rotations x 12,800 pixels: the expansion 1.38 -> 0.98 ms)
     const int64_t tab = expand_table_entries(c->cfg.side);
     if (c->cfg.interp == EMC_INTERP_NEAREST && !c->gauss &&
-        sizeof(uint2) * (size_t)tab <= avail_bytes(c, 0) / 8)
+        small_part(c, sizeof(uint2) * (size_t)tab, 0))
       TRY(c->alloc(&c->d_vtab, tab));
     return EMC_OK;
   }
@@ -783,6 +828,8 @@ static emc_status alloc_work(emc_context* c) {
   TRY(c->alloc(&c->d_lse, N));
   TRY(c->alloc(&c->d_plogp, N));
   TRY(c->alloc(&c->d_Tpart, ((N + 1023) / 1024) * R));
+  TRY(c->end_group());
+  place_acc(c);
   // Y (R x Npad FP32) and the dense compress operand P' (2 x Rpad x Npad
   // FP16) are the large buffers.  Where they do not fit the memory limit or
   // the free device memory, Y holds rotation chunks (half of what is left)
@@ -2845,7 +2892,10 @@ static emc_status run_proposed(emc_context* c, const ProposedPlan& pl, Select se
     TRY(c->alloc(&c->d_best, N));
     TRY(c->alloc(&c->d_bestp, N));
   }
-  if (!c->d_acc) TRY(alloc_acc(c, true));
+  if (!c->d_acc) {
+    TRY(alloc_acc(c, true));
+    place_acc(c);
+  }
   if (pairs > c->pairs_cap || c->cand_m != m) {
     int64_t cap = c->pairs_cap;
     TRY(grow(c, &c->d_cand, cap, pairs));
