@@ -205,6 +205,7 @@ struct emc_context {
   // then responsibilities).  i8_planes 0: the counts are not small integers,
   // or the memory is not there, and the CUDA-core contractions run
   int i8_planes = 0;
+  int64_t i8_rows = 0;  // rotations of one chunk
   int8_t *d_i8 = nullptr, *d_K8 = nullptr, *d_Kt8 = nullptr, *d_digits = nullptr;
   float* d_unit = nullptr;
   uint32_t* d_ktot = nullptr;  // photons at each pixel
@@ -1005,7 +1006,10 @@ emc_status emc_set_patterns(emc_context* c, const float* counts) {
 // The byte operands of an FP32 context whose largest count is `top` (every
 // count an integer): one digit plane up to 127, two above.  They are kept only
 // where they take less than half of the memory that is left, and the CUDA-core
-// contractions run without them.
+// contractions run without them.  The digit planes are those of as many rotations
+// as fit 2 GB: the contractions then run over one chunk of rotations after the
+// other (hundreds of tiles each), and a context does not take as much memory
+// again as its slices or responsibilities.
 static void i8_prepare(emc_context* c, float top, int64_t nonzero) {
   const int64_t N = c->N, R = c->R, npa = c->npa;
   const int planes = top <= (float)kI8MaxCount ? 1 : 2;
@@ -1013,7 +1017,11 @@ static void i8_prepare(emc_context* c, float top, int64_t nonzero) {
   const double most = std::min((double)top, (double)kI8MaxCount) * (double)std::max(N, npa);
   const int64_t ldK = round_up(npa, 16), ldT = round_up(N, 16);
   auto pad = [](size_t n) { return (n + 255) / 256 * 256; };
-  const size_t digits = pad((size_t)kI8Digits * (size_t)R * (size_t)std::max(ldK, ldT));
+  const int64_t row = kI8Digits * std::max(ldK, ldT);
+  const int64_t most_rows = std::max<int64_t>(((int64_t)2 << 30) / row / 128 * 128, 128);
+  const int64_t chunks = (R + most_rows - 1) / most_rows;
+  const int64_t rows = chunks == 1 ? R : round_up((R + chunks - 1) / chunks, 128);
+  const size_t digits = pad((size_t)(rows * row));
   const size_t k8 = pad((size_t)planes * (size_t)(N * ldK)), kt8 = pad((size_t)planes * (size_t)(npa * ldT));
   const size_t unit = pad(sizeof(float) * (size_t)R), ktot = pad(sizeof(uint32_t) * (size_t)npa);
   const size_t small = pad(sizeof(int32_t) * (size_t)(2 * R));
@@ -1021,7 +1029,7 @@ static void i8_prepare(emc_context* c, float top, int64_t nonzero) {
   const size_t rembits = pad(sizeof(uint32_t) * (size_t)(R * i8_bit_words(N)));
   const size_t bytes = k8 + kt8 + digits + unit + ktot + small + rembits + lists;
   const bool fits = top <= (float)kI8MaxCount2 && most <= kI8MaxTotal &&
-                    (double)R * kI8Digits < 2147483647.0 &&
+                    (double)rows * kI8Digits < 2147483647.0 &&
                     ((bytes <= ((size_t)64 << 20) && !c->mem_limit) ||
                      (c->i8_planes == planes && nonzero <= c->i8_nonzero) ||
                      bytes <= avail_bytes(c, c->size_of(c->d_i8)) / 2);
@@ -1037,6 +1045,7 @@ static void i8_prepare(emc_context* c, float top, int64_t nonzero) {
     return;
   }
   c->i8_planes = planes;
+  c->i8_rows = rows;
   c->d_K8 = c->d_i8;
   c->d_Kt8 = c->d_K8 + k8;
   c->d_digits = c->d_Kt8 + kt8;
@@ -1051,8 +1060,8 @@ static void i8_prepare(emc_context* c, float top, int64_t nonzero) {
   c->d_kidx = reinterpret_cast<int32_t*>(c->d_ktotal + 1);
   c->d_kval = reinterpret_cast<float*>(c->d_kidx + nonzero);
   c->i8_nonzero = nonzero;
-  bool ok = i8_encode(&c->tmXp, c->d_digits, npa, kI8Digits * R, ldK, false) &&
-            i8_encode(&c->tmXn, c->d_digits, N, kI8Digits * R, ldT, false);
+  bool ok = i8_encode(&c->tmXp, c->d_digits, npa, kI8Digits * rows, ldK, false) &&
+            i8_encode(&c->tmXn, c->d_digits, N, kI8Digits * rows, ldT, false);
   for (int k = 0; k < planes && ok; ++k)
     ok = i8_encode(&c->tmK8[k], c->d_K8 + (int64_t)k * N * ldK, npa, N, ldK, true) &&
          i8_encode(&c->tmKt8[k], c->d_Kt8 + (int64_t)k * npa * ldT, N, npa, ldT, true);
@@ -1758,24 +1767,28 @@ static emc_status i8_loglik(emc_context* c) {
     CK(c, launch_pattern_stats(c->d_S, nullptr, c->R, c->npa, c->npa, 1, c->d_rowstat, c->st));
     c->launches += 1;
   }
-  CK(c, launch_quant_rows(c->d_S, nullptr, c->d_rowmax, c->R, c->npa, round_up(c->npa, 16),
-                          c->d_digits, c->d_unit, nullptr, nullptr, nullptr, c->st));
-  I8LLArgs a{};
-  a.R = c->R;
-  a.N = c->N;
-  a.poisson = c->gauss ? 0 : 1;
-  a.unit = c->d_unit;
-  a.scaling = c->d_scaling_prev;
-  a.rowstat = c->d_rowstat;
-  a.patstat = c->d_patsq;
-  a.gauss_inv = gauss_inv(c);
-  a.LL = c->d_LL64;
-  for (int k = c->i8_planes - 1; k >= 0; --k) {
-    a.pass = c->i8_planes == 1 ? I8_ONLY : k ? I8_HIGH : I8_LOW;
-    a.mult = k ? 128.0 : 1.0;
-    CK(c, launch_i8_loglik(c->tmK8[k], c->tmXp, c->npa, a, c->d_status, c->num_sms, c->st));
+  for (int64_t r0 = 0; r0 < c->R; r0 += c->i8_rows) {
+    const int64_t rows = std::min(c->i8_rows, c->R - r0);
+    CK(c, launch_quant_rows(c->d_S + r0 * c->npa, nullptr, c->d_rowmax + r0, rows, c->npa,
+                            round_up(c->npa, 16), c->d_digits, c->d_unit + r0, nullptr, nullptr,
+                            nullptr, c->st));
+    I8LLArgs a{};
+    a.R = rows;
+    a.N = c->N;
+    a.poisson = c->gauss ? 0 : 1;
+    a.unit = c->d_unit + r0;
+    a.scaling = c->d_scaling_prev;
+    a.rowstat = c->d_rowstat + r0;
+    a.patstat = c->d_patsq;
+    a.gauss_inv = gauss_inv(c);
+    a.LL = c->d_LL64 + r0 * c->N;
+    for (int k = c->i8_planes - 1; k >= 0; --k) {
+      a.pass = c->i8_planes == 1 ? I8_ONLY : k ? I8_HIGH : I8_LOW;
+      a.mult = k ? 128.0 : 1.0;
+      CK(c, launch_i8_loglik(c->tmK8[k], c->tmXp, c->npa, a, c->d_status, c->num_sms, c->st));
+    }
+    c->launches += 1 + c->i8_planes;
   }
-  c->launches += 1 + c->i8_planes;
   return EMC_OK;
 }
 
@@ -1783,21 +1796,27 @@ static emc_status i8_loglik(emc_context* c) {
 // from the responsibility sweep), contracted with the counts by pixel.
 static emc_status i8_slicesums(emc_context* c) {
   TRY(current_maxima(c, c->d_LL, c->d_scaling, c->N));
-  CK(c, launch_quant_rows(c->d_LL, c->d_scaling, c->d_rowmax, c->R, c->N, round_up(c->N, 16),
-                          c->d_digits, c->d_unit, c->d_small, c->d_rembits,
-                          c->d_remcount, c->st));
-  I8UArgs a{};
-  a.R = c->R;
-  a.npa = c->npa;
-  a.unit = c->d_unit;
-  a.T = c->d_T;
-  a.U = c->d_S;  // the averaged slices replace the expanded ones (emc_atomic.cu:96)
-  a.ktot = c->d_ktot;
-  a.flag = c->d_small;
-  for (int k = c->i8_planes - 1; k >= 0; --k) {
-    a.pass = c->i8_planes == 1 ? I8_ONLY : k ? I8_HIGH : I8_LOW;
-    a.mult = k ? 128.0 : 1.0;
-    CK(c, launch_i8_slices(c->tmKt8[k], c->tmXn, c->N, a, c->d_status, c->num_sms, c->st));
+  const int64_t words = i8_bit_words(c->N);
+  for (int64_t r0 = 0; r0 < c->R; r0 += c->i8_rows) {
+    const int64_t rows = std::min(c->i8_rows, c->R - r0);
+    CK(c, launch_quant_rows(c->d_LL + r0 * c->N, c->d_scaling, c->d_rowmax + r0, rows, c->N,
+                            round_up(c->N, 16), c->d_digits, c->d_unit + r0, c->d_small + r0,
+                            c->d_rembits + r0 * words, c->d_remcount + r0, c->st));
+    I8UArgs a{};
+    a.R = rows;
+    a.npa = c->npa;
+    a.unit = c->d_unit + r0;
+    a.T = c->d_T + r0;
+    // the averaged slices replace the expanded ones (emc_atomic.cu:96)
+    a.U = c->d_S + r0 * c->npa;
+    a.ktot = c->d_ktot;
+    a.flag = c->d_small + r0;
+    for (int k = c->i8_planes - 1; k >= 0; --k) {
+      a.pass = c->i8_planes == 1 ? I8_ONLY : k ? I8_HIGH : I8_LOW;
+      a.mult = k ? 128.0 : 1.0;
+      CK(c, launch_i8_slices(c->tmKt8[k], c->tmXn, c->N, a, c->d_status, c->num_sms, c->st));
+    }
+    c->launches += 1 + c->i8_planes;
   }
   I8SmallArgs f{};
   f.R = c->R;
@@ -1817,7 +1836,7 @@ static emc_status i8_slicesums(emc_context* c) {
   f.kval = c->d_kval;
   f.U = c->d_S;
   CK(c, launch_small_terms(f, c->num_sms, c->st));
-  c->launches += 2 + c->i8_planes;
+  c->launches += 1;
   return EMC_OK;
 }
 
