@@ -152,7 +152,7 @@ template <class Epi>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + kEpiThreads, 1)
     i8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const int64_t m_tiles, const int64_t n_tiles, const int64_t k_blocks,
-                   const int64_t plane_rows, const int raster, const Epi epi, TcStatus* status) {
+                   const int64_t plane_rows, const Epi epi, TcStatus* status) {
   extern __shared__ uint8_t dyn_smem[];
   __shared__ __align__(8) uint64_t full_bar[kStages], empty_bar[kStages];
   __shared__ __align__(8) uint64_t tfull_bar, tempty_bar, drain_bar;
@@ -199,13 +199,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + kEpiThreads, 1)
   const int64_t num_tiles = m_tiles * n_tiles;
   const int64_t cid = blockIdx.x >> 1, ncl = gridDim.x >> 1;
 
-  // m fastest in bands of `raster` n tiles (as tc_pair_kernel)
+  // m fastest: the SMs in flight share the digit tiles (bands of n tiles: no change)
   auto tile_mn = [&](int64_t t, int64_t& m, int64_t& n) {
-    const int64_t span = (int64_t)raster * m_tiles, band = t / span, o0 = band * raster;
-    const int64_t g = n_tiles - o0 < raster ? n_tiles - o0 : raster;
-    const int64_t w = t - band * span;
-    n = o0 + w % g;
-    m = w / g;
+    n = t / m_tiles;
+    m = t - n * m_tiles;
   };
 
   if (warp == 0) {
@@ -378,7 +375,7 @@ cudaError_t run_i8(const CUtensorMap& tmA, const CUtensorMap& tmB, int64_t m, in
   const int64_t tiles = mt * nt, pairs = num_sms / 2;
   if (tiles == 0 || pairs == 0) return cudaErrorInvalidValue;
   kern<<<2 * (unsigned)(tiles < pairs ? tiles : pairs), 64 + kEpiThreads, dyn, st>>>(
-      tmA, tmB, mt, nt, (k + kStepK - 1) / kStepK, n, 1, epi, status);
+      tmA, tmB, mt, nt, (k + kStepK - 1) / kStepK, n, epi, status);
   return cudaGetLastError();
 }
 

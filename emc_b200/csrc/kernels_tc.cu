@@ -353,18 +353,17 @@ __global__ void __launch_bounds__(64 + 32 * Epi::kEpiWarps, 1)
 //   s_k = sum e^(LL-m_k),  d_k = sum e^(LL-m_k) X,  q_k = sum e^(LL-m_k) (LL-m_k)
 // with X the scaling denominator term (gaussian: C_rp, poisson: sum W_r).  The
 // combine kernel turns them into lse_p, the new scaling and sum P log P.
-// EW = 8 or 16: two or four warps per TMEM lane quarter, each with a share of
-// the 256 columns; at the end of a row the shares' running partials are merged
-// into the first's through shared memory.  Sixteen warps: with short K (small
-// detectors) and in the last wave the epilogue is what is waited for.  One SM
+// Sixteen warps, four per TMEM lane quarter, each with a share of the 256
+// columns; at the end of a row the shares' running partials are merged into the
+// first's through shared memory.  With short K (small detectors) and in the last
+// wave the epilogue is what is waited for.  One SM
 // with four / eight / sixteen warps: 256 patterns x 3,240 rotations at 32^2
 // 37.9 / 31.7 / 29.7 us, 10,000 x 10,860 at 32^2 gaussian 0.85 / 0.57 / 0.47 ms.
-template <int EW>
-struct EpiMaxT {
+struct EpiMax {
   static constexpr bool kListed = false;
   static constexpr int kSets = 1;
-  static constexpr int kEpiWarps = EW;
-  static constexpr int kShares = EW / 4;
+  static constexpr int kEpiWarps = 16;
+  static constexpr int kShares = kEpiWarps / 4;
   static constexpr int kSmemBytes = BN * 8 + (kShares - 1) * BM * 16;
   MaxEpiArgs a;
   int64_t n0, ntile, p;
@@ -383,8 +382,8 @@ struct EpiMaxT {
     ntile = nt;
     share = tid >> 7;
     sbuf = smem;
-    epi_bar(32 * EW);
-    for (int c = tid; c < BN; c += 32 * EW) {
+    epi_bar(32 * kEpiWarps);
+    for (int c = tid; c < BN; c += 32 * kEpiWarps) {
       const int64_t r = n0 + c;
       const double w = r < a.R ? a.rowstat[r] : 0.0;
       if (a.poisson) {
@@ -394,7 +393,7 @@ struct EpiMaxT {
         rs[c] = w * a.gauss_inv;
       }
     }
-    epi_bar(32 * EW);
+    epi_bar(32 * kEpiWarps);
     (void)mt;
   }
   __device__ void row_begin(int64_t p_) {
@@ -456,38 +455,35 @@ struct EpiMaxT {
     }
   }
   __device__ void row_end() {
-    if constexpr (kShares > 1) {
-      // merge the column shares' partials of this row (log-sum-exp relative to
-      // the larger maximum)
-      float4* other = reinterpret_cast<float4*>(sbuf + BN * 8);
-      const int lr = (int)(p % BM);
-      if (share > 0) other[(share - 1) * BM + lr] = make_float4(mx, sm, sd, sq);
-      epi_bar(32 * EW);
-      if (share > 0) return;
+    // merge the column shares' partials of this row (log-sum-exp relative to
+    // the larger maximum)
+    float4* other = reinterpret_cast<float4*>(sbuf + BN * 8);
+    const int lr = (int)(p % BM);
+    if (share > 0) other[(share - 1) * BM + lr] = make_float4(mx, sm, sd, sq);
+    epi_bar(32 * kEpiWarps);
+    if (share > 0) return;
 #pragma unroll
-      for (int k = 0; k < kShares - 1; ++k) {
-        const float4 o = other[k * BM + lr];
-        if (!(o.x > -FLT_MAX)) continue;
-        if (mx > -FLT_MAX) {
-          const float m = fmaxf(mx, o.x);
-          const float f1 = __expf(mx - m), f2 = __expf(o.x - m);
-          sq = f1 * (sq + (mx - m) * sm) + f2 * (o.w + (o.x - m) * o.y);
-          sm = f1 * sm + f2 * o.y;
-          sd = f1 * sd + f2 * o.z;
-          mx = m;
-        } else {
-          mx = o.x;
-          sm = o.y;
-          sd = o.z;
-          sq = o.w;
-        }
+    for (int k = 0; k < kShares - 1; ++k) {
+      const float4 o = other[k * BM + lr];
+      if (!(o.x > -FLT_MAX)) continue;
+      if (mx > -FLT_MAX) {
+        const float m = fmaxf(mx, o.x);
+        const float f1 = __expf(mx - m), f2 = __expf(o.x - m);
+        sq = f1 * (sq + (mx - m) * sm) + f2 * (o.w + (o.x - m) * o.y);
+        sm = f1 * sm + f2 * o.y;
+        sd = f1 * sd + f2 * o.z;
+        mx = m;
+      } else {
+        mx = o.x;
+        sm = o.y;
+        sd = o.z;
+        sq = o.w;
       }
     }
     if (pv) a.part[ntile * a.N + p] = make_float4(mx, sm, sd, sq);
   }
   __device__ void tile_end(int64_t, int64_t, int, uint8_t*) {}
 };
-using EpiMax = EpiMaxT<16>;
 
 // compress: row = rotation, column = active pixel; inserts into model/weight.
 // Sixteen epilogue warps (four per TMEM lane quarter, a quarter of the columns
