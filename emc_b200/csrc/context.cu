@@ -793,8 +793,14 @@ static emc_status alloc_work(emc_context* c) {
     // (25,680 rotations x 12,800 pixels: the expansion 1.38 -> 0.98 ms)
     const int64_t tab = expand_table_entries(c->cfg.side);
     if (c->cfg.interp == EMC_INTERP_NEAREST && !c->gauss &&
-        small_part(c, sizeof(uint2) * (size_t)tab, 0))
-      TRY(c->alloc(&c->d_vtab, tab));
+        small_part(c, sizeof(uint2) * (size_t)tab, 0)) {
+      const std::string err = c->err;
+      if (c->alloc(&c->d_vtab, tab) != EMC_OK) {  // not needed
+        cudaGetLastError();
+        c->d_vtab = nullptr;
+        c->err = err;
+      }
+    }
     return EMC_OK;
   }
   c->Npad = round_up(N, 128);
@@ -1406,6 +1412,7 @@ static emc_status list_capacity_or_less(emc_context* c, int64_t n) {
   return s;
 }
 
+// Scratch of the deterministic (rotation, pattern) sort of n entries.
 static emc_status sort_scratch(emc_context* c, int64_t n) {
   TRY(grow(c, &c->d_sort_rp, c->sort_cap, n + 1));
   TRY(grow(c, &c->d_sort_v, c->sort_cap2, n + 1));
