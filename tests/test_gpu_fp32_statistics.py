@@ -86,3 +86,33 @@ def test_statistics_of_broad_posteriors(lik, N, R):
     ref = (Q * (LL - lse)).sum()
     np.testing.assert_allclose(st["sum_plogp"], ref, rtol=tol, atol=tol * N)
     np.testing.assert_allclose(st["total_loglik"], lse.sum(), rtol=1e-6, atol=1e-5 * N)
+
+
+@pytest.mark.parametrize("lik", ["gauss", "poisson"])
+@pytest.mark.parametrize("N,R,top", [(15, 127, 128), (16, 128, 127), (257, 129, 300), (129, 640, 16383)])
+def test_scaling_at_tile_edges_and_with_two_count_planes(lik, N, R, top):
+    """num / sum_r P X with the context's own P, whatever their sharpness: the
+    gaussian cross term comes out of the byte contraction's log-likelihood."""
+    import emc_b200 as E
+    from oracle import oracle as O
+    rng = np.random.default_rng(N + R)
+    model = (0.5 + rng.random(SIDE ** 3)).astype(np.float32)
+    counts = rng.poisson(0.3, (N, SIDE * SIDE)).astype(np.float32)
+    counts[np.arange(N), rng.integers(SIDE * SIDE, size=N)] = top
+    scale = ((0.5 + rng.random(N)) * counts.sum(1) / SIDE ** 2).astype(np.float32)
+    x, y, z = E.detector_coordinates(SIDE, 1e-10, 1.0 / SIDE, 1.0)
+    qa, _ = E.generate_rotations(3)
+    pick = np.random.default_rng(9).permutation(len(qa))[:R]
+    cfg = O.make_config(SIDE, N, R, likelihood=O.LL_POISSON if lik == "poisson" else O.LL_GAUSS)
+    S = O.expand(cfg, model, qa[pick], x, y, z).astype(np.float64)
+    K = counts.astype(np.float64)
+    with _setup(N, R, lik, counts, model, scale) as ctx:
+        ctx.expand()
+        ctx.maximize()
+        P, phi = ctx.get_buffer(E.BUF_RESP).astype(np.float64), ctx.get_scaling()
+    if lik == "poisson":
+        num, X = K.sum(1), np.broadcast_to(S.sum(1)[:, None], P.shape)
+    else:
+        num, X = (K * K).sum(1), S @ K.T
+    # P's normalisation cancels in the sweep's own sums: divided out here too
+    np.testing.assert_allclose(phi, num * P.sum(0) / (P * X).sum(0), rtol=2 * (20 + 4) * 2.0 ** -24)
